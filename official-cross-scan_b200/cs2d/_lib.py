@@ -91,6 +91,23 @@ def lib():
     return _lib
 
 
+_native_mod = None
+
+
+def native():
+    """The native host path of the PyTorch operators (``csrc/cs2d_torch.cpp``), on the same library."""
+    global _native_mod
+    if _native_mod is None:
+        lib()   # reports a missing build in its own words
+        try:
+            from . import _native
+        except ImportError as e:
+            raise RuntimeError("cs2d: cs2d/_native.so is missing or does not fit this PyTorch - build it with "
+                               "official-cross-scan_b200/csrc/build.sh; there is no fallback for it") from e
+        _native_mod = _native
+    return _native_mod
+
+
 def last_error() -> str:
     return lib().cs2d_last_error().decode()
 

@@ -35,11 +35,7 @@ maps, much slower when batch x channel tiles cannot fill the GPU).
 """
 from __future__ import annotations
 
-import ctypes
-
-import torch
-
-from . import _lib, ops
+from . import _lib
 
 
 def _masks(K):
@@ -48,92 +44,33 @@ def _masks(K):
     return rows, cols
 
 
-def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+def _check_shapes(u, delta, A, B, w):
+    d, K = u.size(1), B.size(1)
+    if delta.size(1) != K * d or A.size(0) != K * d or tuple(w.shape) != (K, d):
+        raise RuntimeError("expected delta (b, K*D, h, w), A (K*D, n), w (K, D)")
 
 
 def _dir_forward(u, delta, A, B, C, w, D, delta_bias, delta_softplus, keep_state=True, A_decay=None,
                  deterministic=False):
     """One launch for all directions, merged in the kernel: returns y (b, d, h, w) fp32 and the saved state
     (``None`` when ``keep_state`` is false: the forward then only holds one rolling row of state)."""
-    L = _lib.lib()
-    K, dim = B.size(1), A.size(0)
-    p = ops._problem(u, delta, A, B, C, D, delta_bias, A_decay, delta_softplus, torch.float32, "cross_scan_fwd",
-                     shared_u_dim=dim)
-    rows, cols = _masks(K)
-    wf = w.detach().float().contiguous()
-    dirs = _lib.Dirs(rows, cols, 1, _lib.DIRS_SERIAL if deterministic else 0, wf.data_ptr(), None)
-    nbytes = (L.cs2d_saved_bytes if keep_state else L.cs2d_fwd_only_scratch_bytes)(ctypes.byref(p))
-    if nbytes == 0:
-        raise RuntimeError(f"cs2d forward: {_lib.last_error()}")
-    with torch.cuda.device(u.device):
-        # reproducible form, rows of at most 256 columns: the kernel writes the merged image; otherwise it adds onto it
-        alloc = torch.empty if deterministic and u.size(-1) <= 256 else torch.zeros
-        out = alloc(tuple(u.shape), dtype=torch.float32, device=u.device)
-        saved = torch.empty(nbytes // 4, dtype=torch.float32, device=u.device)
-        rc = (L.cs2d_fwd_dir if keep_state else L.cs2d_fwd_only)(
-            ctypes.byref(p), ctypes.byref(dirs), _ptr(out), out.stride(0), out.stride(1), out.stride(2), _ptr(saved),
-            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
-    ops._raise_on(rc, "forward")
-    return out, (saved if keep_state else None)
+    return _lib.native().cross_fwd(u, delta, A, B, C, w, D, delta_bias, bool(delta_softplus), keep_state, A_decay,
+                                   bool(deterministic))
 
 
 def _dir_backward(u, delta, A, B, C, w, D, delta_bias, dy, saved, delta_softplus, A_decay=None, deterministic=False):
     """dy: gradient of the merged image (b, d, h, w), input dtype or fp32, shared by the directions."""
-    L = _lib.lib()
-    K, dim, n = B.size(1), A.size(0), A.size(1)
-    dev = u.device
-    p = ops._problem(u, delta, A, B, C, D, delta_bias, A_decay, delta_softplus, dy.dtype, "cross_scan_bwd",
-                     shared_u_dim=dim)
-    rows, cols = _masks(K)
-    wf = w.detach().float().contiguous()
-    with torch.cuda.device(dev):
-        alloc = torch.empty if deterministic and u.size(-1) <= 256 else torch.zeros
-        du = alloc(tuple(u.shape), dtype=torch.float32, device=dev)
-        dw = torch.zeros(dim, dtype=torch.float32, device=dev)
-        ddelta = torch.empty(tuple(delta.shape), dtype=u.dtype, device=dev)
-        total, parts = ops.param_grad_layout(dim, n, D is not None, delta_bias is not None, A_decay is not None)
-        flat = torch.zeros(total, dtype=torch.float32, device=dev)
-        part = lambda name: flat[parts[name][0]:parts[name][0] + parts[name][1]] if name in parts else None
-        dB = torch.zeros(tuple(B.shape), dtype=torch.float32, device=dev)
-        dC = torch.zeros(tuple(C.shape), dtype=torch.float32, device=dev)
-        scratch = torch.empty(L.cs2d_bwd_scratch_bytes(ctypes.byref(p)) // 4, dtype=torch.float32, device=dev)
-        dirs = _lib.Dirs(rows, cols, 3, _lib.DIRS_SERIAL if deterministic else 0, wf.data_ptr(), dw.data_ptr())  # u, dy shared
-        rc = L.cs2d_bwd_dir(ctypes.byref(p), ctypes.byref(dirs), _ptr(dy), dy.stride(0), dy.stride(1), dy.stride(2),
-                            _ptr(saved), _ptr(scratch), _ptr(du), _ptr(ddelta), _ptr(part("dA")), _ptr(dB), _ptr(dC),
-                            _ptr(part("dD")), _ptr(part("ddelta_bias")), _ptr(part("dA_decay")),
-                            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
-    ops._raise_on(rc, "backward")
-    return (du.to(u.dtype), ddelta, part("dA").view(dim, n), dB.to(B.dtype), dC.to(C.dtype), dw.view(K, dim // K),
-            part("dD"), part("ddelta_bias"), part("dA_decay"))
+    return tuple(_lib.native().cross_bwd(u, delta, A, B, C, w, D, delta_bias, dy, saved, bool(delta_softplus), A_decay,
+                                         bool(deterministic)))
 
 
-class CrossScan2D(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, u, delta, A, B, C, w, D=None, delta_bias=None, delta_softplus=True, A_decay=None,
-                deterministic=False):
-        _check_shapes(u, delta, A, B, w)
-        ctx.delta_softplus, ctx.deterministic = delta_softplus, bool(deterministic)
-        u, delta = u.contiguous(), delta.contiguous()   # B, C may be strided views (innermost stride 1)
-        y, saved = _dir_forward(u, delta, A, B, C, w, D, delta_bias, delta_softplus, A_decay=A_decay,
-                                deterministic=ctx.deterministic)
-        ctx.save_for_backward(u, delta, A, B, C, D, delta_bias, w, saved, A_decay)
-        return y.to(u.dtype)
+class CrossScan2D:
+    """The operator as a function object: ``CrossScan2D.apply(u, delta, A, B, C, w, D, delta_bias, delta_softplus,
+    A_decay, deterministic)``.  The autograd node itself is native (``csrc/cs2d_torch.cpp``)."""
 
     @staticmethod
-    def backward(ctx, dy):
-        u, delta, A, B, C, D, delta_bias, w, saved, A_decay = ctx.saved_tensors
-        if dy.stride(-1) != 1:
-            dy = dy.contiguous()
-        du, ddelta, dA, dB, dC, dw, dD, dbias, ddecay = _dir_backward(u, delta, A, B, C, w, D, delta_bias, dy, saved,
-                                                                      ctx.delta_softplus, A_decay, ctx.deterministic)
-        return du, ddelta, dA, dB, dC, dw.to(w.dtype), dD, dbias, None, ddecay, None
-
-
-def _check_shapes(u, delta, A, B, w):
-    d, K = u.size(1), B.size(1)
-    if delta.size(1) != K * d or A.size(0) != K * d or tuple(w.shape) != (K, d):
-        raise RuntimeError("expected delta (b, K*D, h, w), A (K*D, n), w (K, D)")
+    def apply(u, delta, A, B, C, w, D=None, delta_bias=None, delta_softplus=True, A_decay=None, deterministic=False):
+        return _lib.native().cross(u, delta, A, B, C, w, D, delta_bias, bool(delta_softplus), A_decay, bool(deterministic))
 
 
 def cross_scan_2d(u, delta, A, B, C, w, D=None, delta_bias=None, delta_softplus=True, A_decay=None,
@@ -143,13 +80,4 @@ def cross_scan_2d(u, delta, A, B, C, w, D=None, delta_bias=None, delta_softplus=
     follows the reference's formula (the row-scan term is left out there).  ``deterministic`` (default:
     ``torch.are_deterministic_algorithms_enabled()``) selects the form of the merge whose ``y`` and ``du``
     come out with the same bits on every run (one CTA walks all directions); it is slower."""
-    if deterministic is None:
-        deterministic = torch.are_deterministic_algorithms_enabled()
-    needs_grad = torch.is_grad_enabled() and any(t is not None and t.requires_grad
-                                                 for t in (u, delta, A, B, C, w, D, delta_bias, A_decay))
-    if not needs_grad:  # evaluation: no saved state
-        _check_shapes(u, delta, A, B, w)
-        y, _ = _dir_forward(u.contiguous(), delta.contiguous(), A, B, C, w, D, delta_bias, delta_softplus,
-                            keep_state=False, A_decay=A_decay, deterministic=deterministic)
-        return y.to(u.dtype)
-    return CrossScan2D.apply(u, delta, A, B, C, w, D, delta_bias, delta_softplus, A_decay, bool(deterministic))
+    return _lib.native().cross(u, delta, A, B, C, w, D, delta_bias, bool(delta_softplus), A_decay, deterministic)

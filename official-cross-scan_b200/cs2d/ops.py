@@ -5,8 +5,10 @@ and return the same lists as the two pybind functions of the reference
 extension ``selective_nd_scan_cuda_oflex``
 (``kernels/selective_nd_scan/src/cusoflex/selective_scan_oflex.cpp:179-284``
 and ``:286-440``).  They allocate the outputs with torch and call the C-ABI
-library on the current CUDA stream; all arithmetic happens in the CUDA
-kernels, there is no PyTorch or CPU fallback.
+library on the current CUDA stream (in native code, ``csrc/cs2d_torch.cpp``); all
+arithmetic happens in the CUDA kernels, there is no PyTorch or CPU fallback.
+``_problem`` describes a problem to the C ABI for the callers that own their
+buffers (``cs2d.parallel``, ``cs2d.host``).
 
 Differences a caller can observe:
 * the three saved tensors ``x, x_v, x_sd`` returned by ``fwd`` are opaque in
@@ -100,22 +102,7 @@ def _raise_on(rc, what):
 
 def fwd(u, delta, A, B, C, D_=None, delta_bias_=None, delta_softplus=False, out_float=False, A_decay_=None):
     """Selective nd scan forward.  Returns ``[out, x, x_v, x_sd]``."""
-    L = _lib.lib()
-    out_dtype = torch.float32 if out_float else u.dtype
-    p = _problem(u, delta, A, B, C, D_, delta_bias_, A_decay_, delta_softplus, out_dtype, "selective_scan_fwd")
-    nbytes = L.cs2d_saved_bytes(ctypes.byref(p))
-    if nbytes == 0:
-        raise RuntimeError(f"cs2d forward: {_lib.last_error()}")
-    with torch.cuda.device(u.device):
-        out = torch.empty(tuple(u.shape), dtype=out_dtype, device=u.device)
-        x_v = torch.empty(nbytes // 4, dtype=torch.float32, device=u.device)
-        x = torch.empty(0, dtype=torch.float32, device=u.device)
-        x_sd = torch.empty(0, dtype=torch.float32, device=u.device)
-        stream = torch.cuda.current_stream(u.device).cuda_stream
-        rc = L.cs2d_fwd(ctypes.byref(p), _ptr(out), out.stride(0), out.stride(1), out.stride(2), _ptr(x_v),
-                        ctypes.c_void_p(stream))
-    _raise_on(rc, "forward")
-    return [out, x, x_v, x_sd]
+    return _lib.native().fwd(u, delta, A, B, C, D_, delta_bias_, bool(delta_softplus), bool(out_float), A_decay_)
 
 
 def fwd_only(u, delta, A, B, C, D_=None, delta_bias_=None, delta_softplus=False, out_float=False, A_decay_=None):
@@ -125,20 +112,7 @@ def fwd_only(u, delta, A, B, C, D_=None, delta_bias_=None, delta_softplus=False,
     rolling row per channel and state pair instead of the checkpoint buffer (a
     quarter of all h values), so evaluation needs a fraction of the memory.
     """
-    L = _lib.lib()
-    out_dtype = torch.float32 if out_float else u.dtype
-    p = _problem(u, delta, A, B, C, D_, delta_bias_, A_decay_, delta_softplus, out_dtype, "selective_scan_fwd")
-    nbytes = L.cs2d_fwd_only_scratch_bytes(ctypes.byref(p))
-    if nbytes == 0:
-        raise RuntimeError(f"cs2d forward: {_lib.last_error()}")
-    with torch.cuda.device(u.device):
-        out = torch.empty(tuple(u.shape), dtype=out_dtype, device=u.device)
-        scratch = torch.empty(nbytes // 4, dtype=torch.float32, device=u.device)
-        stream = torch.cuda.current_stream(u.device).cuda_stream
-        rc = L.cs2d_fwd_only(ctypes.byref(p), None, _ptr(out), out.stride(0), out.stride(1), out.stride(2),
-                             _ptr(scratch), ctypes.c_void_p(stream))
-    _raise_on(rc, "forward")
-    return out
+    return _lib.native().fwd_only(u, delta, A, B, C, D_, delta_bias_, bool(delta_softplus), bool(out_float), A_decay_)
 
 
 def param_grad_layout(dim, dstate, has_D, has_bias, has_decay):
@@ -174,64 +148,8 @@ def bwd(u, delta, A, B, C, D_, delta_bias_, dout, x_, x_v_, delta_softplus, A_de
     selects the backward without floating-point atomics (``cs2d_bwd_det``):
     bit-identical gradients from run to run, for rows of at most 256 columns.
     """
-    L = _lib.lib()
-    if deterministic is None:
-        deterministic = torch.are_deterministic_algorithms_enabled()
-    _check(dout.is_cuda, "dout must be a CUDA tensor")
-    _check(dout.dtype == u.dtype or dout.dtype == torch.float32, "dout must have the input dtype or float32")
-    _check(_inner_ok(dout), "dout must be contiguous in the last dimension")
-    _check(tuple(dout.shape) == tuple(u.shape), "dout must have shape (batch_size, dim, nrows, ncols)")
-    p = _problem(u, delta, A, B, C, D_, delta_bias_, A_decay_, delta_softplus, dout.dtype, "selective_scan_bwd")
-    _check(x_v_ is not None, "the saved state x_v returned by fwd is required")
-    nbytes = L.cs2d_saved_bytes(ctypes.byref(p))
-    if nbytes == 0:
-        raise RuntimeError(f"cs2d backward: {_lib.last_error()}")
-    _check(x_v_.is_cuda and x_v_.dtype == torch.float32 and x_v_.is_contiguous() and x_v_.numel() * 4 == nbytes,
-           "x_v is not the saved state fwd returned for these inputs")
-    batch, dim, nrows, ncols = u.shape
-    delta_dim = delta.size(1)
-    dev = u.device
-    with torch.cuda.device(dev):
-        du = torch.empty(tuple(u.shape), dtype=u.dtype, device=dev)
-        ddelta = torch.empty(tuple(u.shape), dtype=u.dtype, device=dev)
-        total, parts = param_grad_layout(dim, A.size(1), D_ is not None, delta_bias_ is not None,
-                                         A_decay_ is not None)
-        if param_grads is None:
-            param_grads = torch.zeros(total, dtype=torch.float32, device=dev)
-        _check(param_grads.is_cuda and param_grads.dtype == torch.float32 and param_grads.is_contiguous()
-               and param_grads.numel() == total, "param_grads must be a flat float32 CUDA tensor of the layout size")
-
-        def part(name):
-            if name not in parts:
-                return None
-            off, n = parts[name]
-            return param_grads[off:off + n]
-
-        dA = part("dA").view(dim, A.size(1))
-        dD, ddelta_bias, dA_decay = part("dD"), part("ddelta_bias"), part("dA_decay")
-        dB = torch.zeros(tuple(B.shape), dtype=torch.float32, device=dev)
-        dC = torch.zeros(tuple(C.shape), dtype=torch.float32, device=dev)
-        scratch = torch.empty(L.cs2d_bwd_scratch_bytes(ctypes.byref(p)) // 4, dtype=torch.float32, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        if deterministic:
-            nbytes_det = L.cs2d_bwd_det_scratch_bytes(ctypes.byref(p))
-            if nbytes_det == 0:
-                raise RuntimeError(f"cs2d backward has no deterministic implementation for this shape: {_lib.last_error()}")
-            det = torch.empty(nbytes_det // 4, dtype=torch.float32, device=dev)
-            rc = L.cs2d_bwd_det(ctypes.byref(p), None, _ptr(dout), dout.stride(0), dout.stride(1), dout.stride(2),
-                                _ptr(x_v_), _ptr(scratch), _ptr(det), _ptr(du), _ptr(ddelta), _ptr(dA), _ptr(dB), _ptr(dC),
-                                _ptr(dD), _ptr(ddelta_bias), _ptr(dA_decay), ctypes.c_void_p(stream))
-        else:
-            rc = L.cs2d_bwd(ctypes.byref(p), _ptr(dout), dout.stride(0), dout.stride(1), dout.stride(2), _ptr(x_v_),
-                            _ptr(scratch), _ptr(du), _ptr(ddelta), _ptr(dA), _ptr(dB), _ptr(dC), _ptr(dD),
-                            _ptr(ddelta_bias), _ptr(dA_decay), ctypes.c_void_p(stream))
-    _raise_on(rc, "backward")
-    if dim != delta_dim:
-        rep = dim // delta_dim
-        ddelta = ddelta.view(batch, delta_dim, rep, nrows, ncols).sum(2)
-        if ddelta_bias is not None:
-            ddelta_bias = ddelta_bias.view(delta_dim, rep).sum(1)
-    return [du, ddelta, dA, dB.to(B.dtype), dC.to(C.dtype), dD, ddelta_bias, dA_decay]
+    return _lib.native().bwd(u, delta, A, B, C, D_, delta_bias_, dout, x_v_, bool(delta_softplus), A_decay_, param_grads,
+                             deterministic)
 
 
 class SelectiveScan2D(torch.autograd.Function):
@@ -258,12 +176,9 @@ class SelectiveScan2D(torch.autograd.Function):
 
 def selective_scan_2d(u, delta, A, B, C, D=None, delta_bias=None, delta_softplus=False, out_float=False,
                       A_decay=None):
-    """Differentiable 2D-CrossScan selective scan (one scan orientation; see ``fwd``).
+    """Differentiable 2D-CrossScan selective scan (one scan orientation; see ``fwd``), through a native autograd node.
 
     When nothing can ask for a gradient (``torch.no_grad()`` or no input requires one) the
     forward keeps no saved state (``fwd_only``).
     """
-    if not (torch.is_grad_enabled() and any(t is not None and t.requires_grad
-                                            for t in (u, delta, A, B, C, D, delta_bias, A_decay))):
-        return fwd_only(u, delta, A, B, C, D, delta_bias, delta_softplus, out_float, A_decay)
-    return SelectiveScan2D.apply(u, delta, A, B, C, D, delta_bias, delta_softplus, out_float, A_decay)
+    return _lib.native().scan(u, delta, A, B, C, D, delta_bias, bool(delta_softplus), bool(out_float), A_decay)
