@@ -64,12 +64,13 @@ typedef struct {
 } cs2d_problem;
 
 /*
- * Bytes of the saved-state buffer the forward writes and the backward reads
- * (row checkpoints of the state h; for rows of at most 64 columns with more
- * than 8 states also the forward's regrouped fp32 copy of B and C, behind the
- * checkpoints).  It takes the place of the reference's
- * three side tensors x, x_v, x_sd (selective_scan_oflex.cpp:251-258); unlike
- * them it is NOT modified by the backward, so backward may run twice on it.
+ * Bytes of the saved-state buffer the forward writes and the backward reads:
+ * row checkpoints of the state h; for problems with more than two states and
+ * at least eight channels per group (the block-walk kernels) also h and the
+ * row scan at every eighth column and B and C regrouped.  It takes the place of
+ * the reference's three side tensors x, x_v, x_sd (selective_scan_oflex.cpp:251-258);
+ * unlike them it is NOT modified by the backward, so backward may run twice on it.
+ * A backward reads what the forward of the SAME problem, directions and flags wrote.
  * Returns 0 for an invalid problem.
  */
 size_t cs2d_saved_bytes(const cs2d_problem *p);

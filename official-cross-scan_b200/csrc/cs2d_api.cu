@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <initializer_list>
 
+#include "cs2d_blk.cuh"
 #include "cs2d_common.cuh"
 
 namespace cs2d {
@@ -17,6 +18,8 @@ cudaError_t launch_stream_fwd(const Dev &P, int L, int grid, cudaStream_t st);
 cudaError_t launch_stream_bwd(const Dev &P, int L, int grid, cudaStream_t st);
 int stream_pairs_per_cta(int L);
 cudaError_t launch_walk_fwd(const Dev &P, int grid, cudaStream_t st);
+cudaError_t launch_blk_fwd(const Blk &P, int NG, cudaStream_t st);
+cudaError_t launch_blk_bwd(const Blk &P, int NG, cudaStream_t st);
 void walk_geometry(int ncols, int *swd, int *lr);
 int walk_channels_per_cta(int lr);
 size_t walk_bc_bytes(int batch, int groups, int nrows, int ncols);
@@ -266,6 +269,13 @@ static int tile_view(const cs2d_problem *p, int t, bool backward, bool bulk_ok, 
 
 static bool walk_shape(const cs2d_problem *p) { return p->dstate > 8 && p->ncols <= 8 * STRIP; }
 
+static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o, bool backward);
+static size_t blk_row_bytes(const Blk &k, bool roll);
+static size_t blk_col_bytes(const Blk &k);
+static size_t blk_bc_bytes(const Blk &k, int NG);
+
+static bool blk_shape(const cs2d_problem *p) { return p->dstate > 2 && p->dim / p->n_groups >= 8; }
+
 static size_t edge_bytes(const cs2d_problem *p, int NPp) {
     return (size_t)p->batch * p->dim * NPp * p->nrows * sizeof(float4);
 }
@@ -273,7 +283,6 @@ static size_t edge_bytes(const cs2d_problem *p, int NPp) {
 // backward: adjoint rows; otherwise the forward's state rows - all checkpoints, or (rolling) one
 // row per channel and state pair for a forward that no backward follows
 static size_t layout_bytes(const cs2d_problem *p, bool backward, bool rolling = false) {
-    if (validate(p) != CS2D_OK) return 0;
     const int nt = n_tiles(p->ncols);
     size_t total = 0;
     int NPp = 1;
@@ -290,11 +299,24 @@ static size_t layout_bytes(const cs2d_problem *p, bool backward, bool rolling = 
     return total;
 }
 
-size_t cs2d_saved_bytes(const cs2d_problem *p) { return layout_bytes(p, false); }
+// Problems of the block-walk kernels: what those need, or the tile kernels, which the reproducible direction merge
+// uses - the size depends on the problem alone.
+static size_t state_bytes(const cs2d_problem *p, bool backward, bool rolling) {
+    if (validate(p) != CS2D_OK) return 0;
+    const size_t tile = layout_bytes(p, backward, rolling);
+    if (tile == 0 || !blk_shape(p)) return tile;
+    Blk k;
+    int NG;
+    blk_fill(k, NG, p, nullptr, backward);
+    const size_t need = backward ? blk_row_bytes(k, true) : blk_row_bytes(k, rolling) + (rolling ? blk_bc_bytes(k, NG) : 3 * blk_bc_bytes(k, NG) + blk_col_bytes(k));
+    return tile > need ? tile : need;
+}
 
-size_t cs2d_bwd_scratch_bytes(const cs2d_problem *p) { return layout_bytes(p, true); }
+size_t cs2d_saved_bytes(const cs2d_problem *p) { return state_bytes(p, false, false); }
 
-size_t cs2d_fwd_only_scratch_bytes(const cs2d_problem *p) { return layout_bytes(p, false, true); }
+size_t cs2d_bwd_scratch_bytes(const cs2d_problem *p) { return state_bytes(p, true, false); }
+
+size_t cs2d_fwd_only_scratch_bytes(const cs2d_problem *p) { return state_bytes(p, false, true); }
 
 // A group that walks the columns right-to-left sees the tile's scan columns at mirrored image
 // columns (Dev::cshift); 4-element accesses are only kept when that shift preserves 16-byte alignment.
@@ -356,8 +378,61 @@ static void stream_fill(Dev &d, const cs2d_problem *p, int *L, int *grid) {
 // exactly where the tile forward would, so the choice is invisible to the backward.
 static bool walk_fwd_ok(const cs2d_problem *p, const cs2d_dirs *o) { return walk_shape(p) && !has_dirs(o); }
 
+// ---- block-walk kernels (cs2d_blk_fwd.cu, cs2d_blk_bwd.cu) -------------------------------------------
+static bool blk_ok(const cs2d_problem *p, const cs2d_dirs *o) { return blk_shape(p) && !(o && o->merge_w && (o->flags & CS2D_DIRS_SERIAL)); }
+// the parts of the saved state (or of the forward-only scratch)
+static void blk_state(Blk &k, int NG, const void *saved, bool roll) {
+    char *q = const_cast<char *>(static_cast<const char *>(saved));
+    k.roll = roll;
+    k.row = reinterpret_cast<float4 *>(q);
+    k.bc = reinterpret_cast<float2 *>(q + blk_row_bytes(k, roll));
+    k.bc2 = reinterpret_cast<float4 *>(q + blk_row_bytes(k, roll) + blk_bc_bytes(k, NG));
+    k.col = reinterpret_cast<float4 *>(q + blk_row_bytes(k, roll) + 3 * blk_bc_bytes(k, NG));
+}
+static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o, bool backward) {
+    k = Blk{};
+    k.H = p->nrows; k.W = p->ncols; k.N = p->dstate; k.G = p->n_groups; k.dpg = p->dim / p->n_groups;
+    k.drep = p->dim / p->delta_dim;
+    k.io_dt = p->io_dtype; k.out_dt = p->out_dtype; k.softplus = p->delta_softplus;
+    k.u = p->u; k.delta = p->delta; k.B = p->B; k.C = p->C; k.A = p->A; k.D = p->D; k.bias = p->delta_bias; k.decay = p->A_decay;
+    k.u_bs = p->u_bs; k.u_ds = p->u_ds; k.u_hs = p->u_hs;
+    k.dl_bs = p->delta_bs; k.dl_ds = p->delta_ds; k.dl_hs = p->delta_hs;
+    k.A_ds = p->A_ds; k.A_ns = p->A_ns;
+    k.B_bs = p->B_bs; k.B_gs = p->B_gs; k.B_ns = p->B_ns; k.B_hs = p->B_hs;
+    k.C_bs = p->C_bs; k.C_gs = p->C_gs; k.C_ns = p->C_ns; k.C_hs = p->C_hs;
+    if (o) {
+        k.flip_h = o->flip_rows_mask; k.flip_w = o->flip_cols_mask; k.shared = o->shared_input;
+        k.mw = o->merge_w; k.dw = o->merge_dw;
+    }
+    k.nblk = (p->nrows + BK_R - 1) / BK_R; k.nstrip = (p->ncols + BK_S - 1) / BK_S;
+    NG = 8;
+    while (NG < p->dstate) NG <<= 1;
+    k.nsl = (k.dpg + 1) / 2;
+    k.NL = (int64_t)p->batch * k.G * k.nsl * NG;
+    const int spw = 32 / NG, ctas = !backward ? 4 : NG == 16 ? 3 : 2;   // slots per warp, CTAs per SM
+    k.ntile = (k.nsl + spw - 1) / spw; k.items = p->batch * k.G * k.ntile;
+    // Row workers: as few as fill the GPU; with short rows a worker waits for the others at the end of a row
+    const int64_t slots = (int64_t)kSMs * ctas * BK_WARPS;
+    double best = 1e300;
+    for (int rwl = 0; rwl < 3; ++rwl) {
+        const int rw = 1 << rwl;
+        if (rw > 1 && k.nblk < rw) break;
+        const int period = k.nstrip < BK_LAG * rw && rw > 1 ? BK_LAG * rw : k.nstrip;
+        const int64_t npass = (k.nblk + rw - 1) / rw, rounds = ((int64_t)k.items * rw + slots - 1) / slots;
+        // rounds of warps, each slower the more of them share an SM
+        const double cost = (double)rounds * (npass * period + BK_LAG * (rw - 1));
+        if (cost < best * 0.98) { best = cost; k.rwl = rwl; k.npass = (int)npass; k.period = period; }
+    }
+    const int64_t need = ((int64_t)k.items + (BK_WARPS >> k.rwl) - 1) / (BK_WARPS >> k.rwl);
+    const int64_t cap = ctas * kSMs;   // CTAs that fit at once
+    k.grid = (int)(need < cap ? need : cap);
+}
+static size_t blk_row_bytes(const Blk &k, bool roll) { return (size_t)(roll ? 1 : k.nblk) * k.nstrip * 4 * k.NL * sizeof(float4); }
+static size_t blk_bc_bytes(const Blk &k, int NG) { return (size_t)(k.items / k.ntile) * k.nblk * k.nstrip * BK_PX * NG * sizeof(float2); }
+static size_t blk_col_bytes(const Blk &k) { return (size_t)k.nblk * (k.nstrip - 1) * 4 * k.NL * sizeof(float4); }
+
 static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_t out_bs, int64_t out_ds,
-                    int64_t out_hs, void *saved, void *stream, bool rolling = false) {
+                    int64_t out_hs, void *saved, void *stream, bool rolling = false, bool tile = false) {
     int rc = validate(p);
     if (rc) return rc;
     if ((rc = check_dirs(p, o))) return rc;
@@ -382,6 +457,17 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
         cudaError_t e = launch_stream_fwd(d, L, grid, reinterpret_cast<cudaStream_t>(stream));
         if (e != cudaSuccess) return fail(CS2D_ERR_CUDA, "forward launch failed: %s", cudaGetErrorString(e));
         g_launches.fetch_add(1);
+        return CS2D_OK;
+    }
+    if (!tile && blk_ok(p, o)) {
+        Blk k;
+        int NG;
+        blk_fill(k, NG, p, o, false);
+        k.out = out; k.o_bs = out_bs; k.o_ds = out_ds; k.o_hs = out_hs;
+        blk_state(k, NG, saved, rolling);
+        cudaError_t e = launch_blk_fwd(k, NG, reinterpret_cast<cudaStream_t>(stream));
+        if (e != cudaSuccess) return fail(CS2D_ERR_CUDA, "forward launch failed: %s", cudaGetErrorString(e));
+        g_launches.fetch_add(2);   // the regrouping of B and C, then the scan
         return CS2D_OK;
     }
     if (walk_fwd_ok(p, o)) {
@@ -481,7 +567,7 @@ static cudaError_t launch_sum(float *out, const float *part, int64_t n, int coun
 }
 
 // layout of the deterministic backward's scratch, in floats
-struct DetLayout { int64_t nB, dB, dC, dA, dD, dbias, ddecay, total; int ntiles, grid, zero; };
+struct DetLayout { int64_t nB, dB, dC, dA, dD, dbias, ddecay, state, total; int ntiles, grid, zero; };
 static int det_layout(const cs2d_problem *p, DetLayout *l) {
     if (n_tiles(p->ncols) > 1)
         return fail(CS2D_ERR_UNSUPPORTED, "the deterministic backward covers ncols <= %d", kTileCols);
@@ -500,6 +586,8 @@ static int det_layout(const cs2d_problem *p, DetLayout *l) {
     l->dB = 0; l->dC = l->dB + l->ntiles * l->nB; l->dA = l->dC + l->ntiles * l->nB;
     l->dD = l->dA + (int64_t)p->batch * p->dim * p->dstate; l->dbias = l->dD + (int64_t)p->batch * p->dim;
     l->ddecay = l->dbias + (int64_t)p->batch * p->dim; l->total = l->ddecay + l->grid;
+    l->state = (l->total + 3) & ~int64_t(3);   // problems of the block-walk kernels: the tile kernels' checkpoints
+    if (blk_shape(p)) l->total = l->state + (int64_t)(layout_bytes(p, false) / 4);
     return CS2D_OK;
 }
 
@@ -522,6 +610,30 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
     if (dA_decay && !p->A_decay) return fail(CS2D_ERR_INVALID, "dA_decay requested without A_decay");
     int *status = status_ptr();
     if (!status) return fail(CS2D_ERR_CUDA, "cannot locate the device status word");
+    if (!det && blk_ok(p, o)) {
+        Blk k;
+        int NG;
+        blk_fill(k, NG, p, o, true);
+        blk_state(k, NG, saved, false);
+        k.out = const_cast<void *>(dout); k.o_bs = dout_bs; k.o_ds = dout_ds; k.o_hs = dout_hs;
+        k.adj = reinterpret_cast<float4 *>(scratch);
+        k.du = du; k.ddelta = ddelta; k.dA = dA; k.dB = dB; k.dC = dC; k.dD = dD; k.dbias = ddelta_bias; k.ddecay = dA_decay;
+        k.vec_dbc = vec_ok(dB, 4, p->ncols, {}) && vec_ok(dC, 4, p->ncols, {});
+        cudaError_t e = launch_blk_bwd(k, NG, reinterpret_cast<cudaStream_t>(stream));
+        if (e != cudaSuccess) return fail(CS2D_ERR_CUDA, "backward launch failed: %s", cudaGetErrorString(e));
+        g_launches.fetch_add(1);
+        return CS2D_OK;
+    }
+    if (det && blk_ok(p, o)) {
+        // The deterministic backward is the tile kernels'; their checkpoints are made again (y goes to du, which is
+        // written later).
+        cs2d_problem q = *p;
+        q.out_dtype = p->io_dtype;
+        void *st = det + dl.state;
+        if ((rc = fwd_impl(&q, o, du, (int64_t)p->dim * p->nrows * p->ncols, (int64_t)p->nrows * p->ncols, p->ncols, st, stream, false, true)))
+            return rc;
+        saved = st;
+    }
     const bool streamed = stream_ok(p, o);   // the forward of this problem ran on the streaming kernel
     if (streamed && !det) {
         Dev d;

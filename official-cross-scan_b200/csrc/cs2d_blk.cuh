@@ -1,0 +1,162 @@
+// Block-walk kernels (sm_100a): what the forward (cs2d_blk_fwd.cu) and the backward (cs2d_blk_bwd.cu) share.
+//
+// A thread owns the recurrences of two channels - the halves of packed fp32x2 registers - for one state, and walks
+// the image in blocks of 4 rows by 8 columns: along a block column by column, the four rows of a column one after the
+// other, then on to the next block of the row of blocks, then to the next row of blocks.  Nothing is exchanged
+// between threads to solve the recurrence: no scan over lanes, no second pass, no skew to fill and drain.  What
+// crosses a block goes through registers (along the row: h, q, s, a of the last column) or through one row of h per
+// row of blocks (down: written as float4, 512 consecutive bytes per warp, read back by the block below).
+//
+// A warp is self-contained: its lanes are the NG states of 32/NG slots (a slot is a channel pair), it loads, transforms
+// (softplus) and stages delta and u of its own slots in shared memory, sums over the states through shared memory and
+// writes the results.  Neighbouring lanes share delta and u (measured on B200: a 128-bit shared load takes 2 cycles of
+// the SM's load unit when neighbouring lanes share their address, 4 otherwise, whatever else is broadcast - and that unit,
+// not arithmetic, bounds these kernels).  No barriers; sixteen warps per SM hide each other's latencies.
+//
+// Images with few recurrences run with 2 or 4 row WORKERS per CTA of four warps: worker w takes every RW-th row of
+// blocks, LAG steps behind worker w-1, which has then left the row of h it needs; the CTA's warps then meet on its
+// barrier once per block.
+#pragma once
+
+#include "cs2d_common.cuh"
+
+namespace cs2d {
+
+constexpr int BK_R = 4, BK_S = 8, BK_PX = BK_R * BK_S;   // a block: rows, columns, pixels
+constexpr int BK_WARPS = 4;                               // warps per CTA
+constexpr int BK_LAG = 2;                                 // steps between neighbouring row workers
+static_assert(BK_R == RB, "row blocks and checkpoint cadence agree with the other kernels");
+
+struct Blk {
+    int H, W, N, G, dpg, drep, io_dt, out_dt, softplus;
+    int nblk, nstrip;       // rows of blocks, blocks per row
+    int period;             // steps per row of blocks: nstrip, or more when a worker has to wait for the others
+    int rwl;                // log2 of the row workers per CTA
+    int nsl;                // slots per group
+    int ntile, items;       // warps' worth of slots per group; work items = batch * G * ntile
+    int grid;
+    int npass;              // rows of blocks per worker: ceil(nblk / workers)
+    unsigned flip_h, flip_w;
+    int shared;             // bit 0: u has dpg channels shared by the groups, bit 1: dout
+    int roll;               // forward: one rolling row of h instead of the checkpoints
+    int64_t NL;             // threads' worth of recurrences: batch * G * nsl * state slots
+    const void *u, *delta, *B, *C;
+    const float *A, *D, *bias, *decay;
+    int64_t u_bs, u_ds, u_hs, dl_bs, dl_ds, dl_hs, A_ds, A_ns;
+    int64_t B_bs, B_gs, B_ns, B_hs, C_bs, C_gs, C_ns, C_hs;
+    void *out; int64_t o_bs, o_ds, o_hs;    // forward: out; backward: dout
+    const float *mw; float *dw;             // direction merge (see Dev)
+    // Checkpoints, threads innermost so that a warp moves whole lines:
+    //   row [nblk][nstrip][4][NL] float4 = h of the block's last row, two columns per float4 (rolling: nblk = 1)
+    //   col [nblk][nstrip-1][4][NL] float4 = (q, s) of the column left of block strip+1, one row per float4
+    float4 *row, *col;
+    float2 *bc;                             // B and C in walk order, and for a backward with every value twice (blk_bc_kernel)
+    float4 *bc2;
+    // backward
+    float4 *adj;                            // [nstrip][4][NL]: the adjoint row m between rows of blocks
+    void *du, *ddelta;
+    float *dA, *dB, *dC, *dD, *dbias, *ddecay;
+    int vec_dbc;                            // dB, dC: rows of whole aligned groups of four columns
+};
+
+// 16-byte asynchronous copies to shared memory, in groups
+__device__ __forceinline__ void bk_cp16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void bk_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void bk_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Position in a warp's stream of blocks: its items, passes of an item, blocks of a row.
+struct BkPos {
+    int item, pass, strip, bg, g, slot;   // batch * G + group, group, first slot of the item inside its group
+    __device__ __forceinline__ void decode(const Blk &P, int spw) {
+        bg = item / P.ntile;
+        g = bg % P.G;
+        slot = (item % P.ntile) * spw;
+    }
+    __device__ __forceinline__ void next(const Blk &P, int spw, int stride) {
+        if (++strip < P.period) return;
+        strip = 0;
+        if (++pass < P.npass) return;
+        pass = 0;
+        item += stride;
+        decode(P, spw);
+    }
+};
+
+__device__ __forceinline__ float rcp(float x) {   // of a value in [1, 4]: no range to guard
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// softplus(x) = max(x, 0) + log(1 + t), t = exp(-|x|) in (0, 1]; log(1 + t) = 2 atanh(s) with s = t / (2 + t) <= 1/3
+// from its power series (terms up to s^13: remainder below 1e-8 of the sum), two values at a time.  x above 20
+// passes through: the logarithm is then below half a unit in the last place.  SIG: `sig` = 1 / (1 + exp(-x)).
+// About 3e-7 relative.
+template <bool SIG>
+__device__ __forceinline__ float2 bk_softplus2(float2 x, float2 *sig) {
+    const float2 t = f2(ex2(-fabsf(x.x) * LOG2E), ex2(-fabsf(x.y) * LOG2E)), d = add2(t, bc(2.f));
+    const float2 s = mul2(t, f2(rcp(d.x), rcp(d.y))), z = mul2(s, s);
+    float2 q = fma2(z, bc(1.f / 13.f), bc(1.f / 11.f));
+    q = fma2(q, z, bc(1.f / 9.f)); q = fma2(q, z, bc(1.f / 7.f)); q = fma2(q, z, bc(0.2f)); q = fma2(q, z, bc(1.f / 3.f));
+    const float2 h = fma2(mul2(s, z), q, s);
+    if constexpr (SIG) {
+        const float2 e = add2(t, bc(1.f)), r = f2(rcp(e.x), rcp(e.y)), tr = mul2(t, r);
+        *sig = f2(x.x >= 0.f ? r.x : tr.x, x.y >= 0.f ? r.y : tr.y);
+    }
+    return fma2(h, bc(2.f), f2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+}
+
+// Elements of the input type.  bk_ldp: loaded only when `on` (else 0), as raw bits: the guard is a predicate on the
+// load, and nothing depends on the register until the value is used.
+template <int DT> struct bk_type { using t = uint16_t; };
+template <> struct bk_type<CS2D_F32> { using t = uint32_t; };
+template <int DT>
+__device__ __forceinline__ uint32_t bk_ldp(const typename bk_type<DT>::t *p, bool on) {
+    if constexpr (DT == CS2D_F32) {
+        uint32_t v;
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.nc.b32 %0, [%1];\n\t}" : "=r"(v) : "l"(p), "r"((int)on));
+        return v;
+    } else {
+        unsigned short v;
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b16 %0, 0;\n\t@p ld.global.nc.b16 %0, [%1];\n\t}" : "=h"(v) : "l"(p), "r"((int)on));
+        return v;
+    }
+}
+// 16 bytes: zeros unless `on`.  NC: through the read-only path (nothing in this kernel writes them).
+template <bool NC>
+__device__ __forceinline__ float4 bk_ld16(const float4 *p, bool on) {
+    float4 v;
+    if constexpr (NC)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@p ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];\n\t}"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "r"((int)on));
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@p ld.global.v4.f32 {%0,%1,%2,%3}, [%4];\n\t}"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "r"((int)on) : "memory");
+    return v;
+}
+__device__ __forceinline__ void bk_red16(float *p, float4 v, bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p red.global.add.v4.f32 [%0], {%1,%2,%3,%4};\n\t}" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"((int)on) : "memory");
+}
+__device__ __forceinline__ void bk_st16(float4 *p, float4 v, bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p st.global.v4.f32 [%0], {%1,%2,%3,%4};\n\t}" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"((int)on) : "memory");
+}
+template <int DT>
+__device__ __forceinline__ float bk_cvt(uint32_t raw) {
+    if constexpr (DT == CS2D_F32) return __uint_as_float(raw);
+    else if constexpr (DT == CS2D_BF16) return __uint_as_float(raw << 16);
+    else return __half2float(__ushort_as_half((unsigned short)raw));
+}
+// Results: fp32, the input type, or (merge) added onto an fp32 image.
+template <int DT, bool MERGE>
+__device__ __forceinline__ void bk_st(void *base, int64_t i, float v, bool on) {
+    if constexpr (MERGE) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p red.global.add.f32 [%0], %1;\n\t}" ::"l"(reinterpret_cast<float *>(base) + i), "f"(v), "r"((int)on) : "memory");
+    } else if constexpr (DT == CS2D_F32) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}" ::"l"(reinterpret_cast<float *>(base) + i), "f"(v), "r"((int)on) : "memory");
+    } else {
+        const unsigned short h = DT == CS2D_BF16 ? __bfloat16_as_ushort(__float2bfloat16(v)) : __half_as_ushort(__float2half(v));
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}" ::"l"(reinterpret_cast<uint16_t *>(base) + i), "h"(h), "r"((int)on) : "memory");
+    }
+}
+}  // namespace cs2d

@@ -1,0 +1,361 @@
+// Block-walk forward (sm_100a); the decomposition is described in cs2d_blk.cuh.
+//   q(r,c) = a*(q(r,c-1) + T),  T = h(r-1,c) - 0.5*(a(r-1,c) + a(r,c-1))*h(r-1,c-1)
+//   s(r,c) = a*s(r,c-1) + p,    h = q + s,    y = D*u + sum_n C*(q + p/4)
+// which is the reference's recurrence (include/cusoflex/selective_scan_fwd_kernel_oflex.cuh:214-338: h, the row scan
+// s, y = C*(h - s + p/4)) carried as q = h - s, so that the difference y needs is never formed by subtraction.
+#include "cs2d_blk.cuh"
+
+namespace cs2d {
+
+// B and C in the order the walk consumes them: [batch*G][nblk][nstrip][32 pixels, column by column][NG] (B, C), fp32, in
+// scan coordinates; pixels outside the image and states past dstate are zero.  One 16-byte asynchronous copy per lane then
+// fetches what two states of a pixel need, without address arithmetic or conversions in the walk.  For a backward, which
+// is short of registers and instructions rather than of shared-memory bandwidth, also with every value twice:
+// [32 pixels][(B, B, B', B'), (C, C, C', C')][8] of the states n and n + 8 (16 slots), [32][8] (B, B, C, C) (8 slots).
+template <int DT>
+__global__ void blk_bc_kernel(const __grid_constant__ Blk P, int NG) {
+    using T = typename bk_type<DT>::t;
+    const int nt = P.nblk * P.nstrip, tile = blockIdx.x % nt, bg = blockIdx.x / nt, g = bg % P.G, b = bg / P.G;
+    const int strip = tile % P.nstrip, blk = tile / P.nstrip;
+    const bool fh = (P.flip_h >> g) & 1u, fw = (P.flip_w >> g) & 1u;
+    const T *B = reinterpret_cast<const T *>(P.B) + (int64_t)b * P.B_bs + (int64_t)g * P.B_gs;
+    const T *C = reinterpret_cast<const T *>(P.C) + (int64_t)b * P.C_bs + (int64_t)g * P.C_gs;
+    float2 *dst = P.bc + ((int64_t)bg * P.nblk * P.nstrip + tile) * BK_PX * NG;
+    __shared__ float2 sm[16][BK_PX + 1];
+    for (int e = threadIdx.x; e < BK_PX * NG; e += blockDim.x) {   // read along rows
+        const int px = e % BK_PX, n = e / BK_PX, r = blk * BK_R + px / BK_S, c = strip * BK_S + px % BK_S;
+        const bool on = n < P.N && r < P.H && c < P.W;
+        const int64_t o = (int64_t)(fw ? P.W - 1 - c : c);
+        const int fr = fh ? P.H - 1 - r : r;
+        const uint32_t bv = bk_ldp<DT>(B + (int64_t)n * P.B_ns + (int64_t)fr * P.B_hs + o, on), cv = bk_ldp<DT>(C + (int64_t)n * P.C_ns + (int64_t)fr * P.C_hs + o, on);
+        sm[n][px] = f2(bk_cvt<DT>(bv), bk_cvt<DT>(cv));
+    }
+    __syncthreads();
+    if (!P.roll) {
+        float4 *dst2 = P.bc2 + ((int64_t)bg * P.nblk * P.nstrip + tile) * BK_PX * NG;
+        for (int e = threadIdx.x; e < BK_PX * NG; e += blockDim.x) {
+            const int n = e & 7, i = e / NG, px = (i % BK_R) * BK_S + i / BK_R;
+            const float2 v = sm[n][px], v8 = NG == 16 ? sm[n + 8][px] : v;
+            dst2[e] = NG == 8 ? make_float4(v.x, v.x, v.y, v.y) : (e & 8) ? make_float4(v.y, v.y, v8.y, v8.y) : make_float4(v.x, v.x, v8.x, v8.x);
+        }
+    }
+    for (int e = threadIdx.x; e < BK_PX * NG; e += blockDim.x) {   // write in walk order
+        const int n = e % NG, i = e / NG;
+        dst[e] = sm[NG == 16 ? (n >> 1) + (n & 1) * 8 : n][(i % BK_R) * BK_S + i / BK_R];   // (states n and n + 8 side by side)
+    }
+}
+
+template <int NG>
+struct BkFwd {   // a warp's shared memory
+    static constexpr int SPW = 32 / NG, YP = 34;                  // slots per warp; pitch of a pixel's sums
+    static constexpr int in = 0;                                  // float4 [SPW][33] (dl, dl', dlu, dlu') of the two channels, row by row
+    static constexpr int par = in + SPW * 33 * 16;                // float4 [SPW] (delta_bias, delta_bias', D, D')
+    static constexpr int y = par + SPW * 16;                      // float2 [16][YP] half a block's C*(q + p/4) of every lane
+    static constexpr int bc = y + 16 * YP * 8;                    // float2 [4][8][NG] B, C: ring of quarter blocks
+    static constexpr int y0 = bc + 4 * 8 * NG * 8;                // float2 [SPW][33] D*u
+    static constexpr int top = y0 + SPW * 33 * 8;                 // float2 [SPW][9]  dl of the row above
+    static constexpr int total = (top + SPW * 9 * 8 + 15) & ~15;
+};
+
+template <int NG, int DT, bool KEEP>
+__global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_constant__ Blk P) {
+    using S = BkFwd<NG>;
+    using T = typename bk_type<DT>::t;
+    constexpr int SPW = S::SPW, YP = S::YP, NCP = NG / 8 > 0 ? NG / 8 : 1;   // NCP: 16-byte copies per lane and quarter block
+    extern __shared__ __align__(16) unsigned char smem_[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char *sm = smem_ + warp * S::total;
+    float4 *sIn = reinterpret_cast<float4 *>(sm + S::in), *sPar = reinterpret_cast<float4 *>(sm + S::par);
+    float2 *sY = reinterpret_cast<float2 *>(sm + S::y), *sBC = reinterpret_cast<float2 *>(sm + S::bc);
+    float2 *sY0 = reinterpret_cast<float2 *>(sm + S::y0), *sTop = reinterpret_cast<float2 *>(sm + S::top);
+    const int rw = 1 << P.rwl, w = warp & (rw - 1), nsub = BK_WARPS >> P.rwl, stride = gridDim.x * nsub;
+    const int n = lane % NG, sl_ = lane / NG;              // this thread's state and slot of the warp
+    const int lr = lane >> 3, lc = lane & 7;               // its pixel when staging
+    const int first = blockIdx.x * nsub, lmax = (P.items - first + stride - 1) / stride * P.npass * P.period;
+    const int steps = lmax + BK_LAG * (rw - 1);
+    const bool softplus = P.softplus != 0, drep1 = P.drep == 1;
+    const bool chain = P.nstrip == 1 && rw == 1;           // the next block is always the one below
+    const float2 lgd = bc(P.decay ? log2f(__ldg(P.decay)) : 0.f);
+
+    BkPos pos;
+    pos.item = first + (warp >> P.rwl); pos.pass = pos.strip = 0;
+    pos.decode(P, SPW);
+    auto live = [&](const BkPos &q, int L) { return L >= 0 && L < lmax && q.item < P.items && q.strip < P.nstrip && q.pass * rw + w < P.nblk; };
+
+    // ---- loads of the next block: raw delta and u of the lane's pixel for every channel of the warp, delta of the row above ----
+    uint32_t vd[2 * SPW], vu[2 * SPW], vt[SPW / 2];
+    const T *pd = nullptr, *pu = nullptr, *pt = nullptr;   // at the first block of the row of blocks
+    auto load_raw = [&](const BkPos &q) {
+        const int r0 = (q.pass * rw + w) * BK_R, ch0 = q.slot * 2, cg = q.g * P.dpg + ch0;
+        const bool fw = (P.flip_w >> q.g) & 1u;
+        if (q.strip == 0) {
+            const bool fh = (P.flip_h >> q.g) & 1u;
+            const int b = q.bg / P.G, fr = fh ? P.H - 1 - (r0 + lr) : r0 + lr, fc = fw ? P.W - 1 - lc : lc;
+            const T *db = reinterpret_cast<const T *>(P.delta) + (int64_t)b * P.dl_bs + fc;
+            pd = db + (int64_t)fr * P.dl_hs + (int64_t)(cg / P.drep) * P.dl_ds;
+            pt = db + (int64_t)(fh ? P.H - r0 : r0 - 1) * P.dl_hs + (drep1 ? (int64_t)(cg + lr) * P.dl_ds : 0);
+            pu = reinterpret_cast<const T *>(P.u) + (int64_t)b * P.u_bs + (int64_t)((P.shared & 1) ? ch0 : cg) * P.u_ds + (int64_t)fr * P.u_hs + fc;
+        }
+        const int64_t cs = fw ? -q.strip * BK_S : q.strip * BK_S;
+        const bool okc = q.strip * BK_S + lc < P.W, pix = okc && r0 + lr < P.H;
+        const int nch = P.dpg - ch0;
+        const T *qd = pd + cs, *qu = pu + cs;
+        if (drep1) {
+#pragma unroll
+            for (int k = 0; k < 2 * SPW; ++k) {
+                vd[k] = bk_ldp<DT>(qd, pix && k < nch);
+                vu[k] = bk_ldp<DT>(qu, pix && k < nch);
+                qd += P.dl_ds; qu += P.u_ds;
+            }
+#pragma unroll
+            for (int i = 0; i < SPW / 2; ++i) vt[i] = bk_ldp<DT>(pt + cs + 4 * i * P.dl_ds, okc && r0 > 0 && lr + 4 * i < nch);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 2 * SPW; ++k) {
+                vd[k] = bk_ldp<DT>(qd + (int64_t)((cg + k) / P.drep - cg / P.drep) * P.dl_ds, pix && k < nch);
+                vu[k] = bk_ldp<DT>(qu, pix && k < nch);
+                qu += P.u_ds;
+            }
+#pragma unroll
+            for (int i = 0; i < SPW / 2; ++i)
+                vt[i] = bk_ldp<DT>(pt + cs + (int64_t)((cg + lr + 4 * i) / P.drep) * P.dl_ds, okc && r0 > 0 && lr + 4 * i < nch);
+        }
+    };
+    // quarter qt (two columns) of B and C of a block into its place in the ring
+    auto copy_bc = [&](const unsigned char *src, int qt, bool on) {
+        unsigned char *dst = reinterpret_cast<unsigned char *>(sBC + qt * 8 * NG) + lane * 16;
+        src += qt * 64 * NG + lane * 16;
+        if (on && (NG >= 8 || lane < 4 * NG)) {
+#pragma unroll
+            for (int i = 0; i < NCP; ++i) bk_cp16(dst + 512 * i, src + 512 * i);
+        }
+        bk_commit();
+    };
+
+    float2 A2 = bc(0.f), hcorner = bc(0.f);
+    float2 hl[BK_R], al[BK_R], ql[BK_R], sl[BK_R];         // column left of the block
+    float2 hup[BK_S];                                      // the row of h above the block; hcorner: its value left of the current column
+#pragma unroll
+    for (int c = 0; c < BK_S; ++c) hup[c] = bc(0.f);
+#pragma unroll
+    for (int r = 0; r < BK_R; ++r) { hl[r] = al[r] = ql[r] = sl[r] = bc(0.f); }
+    int64_t oo = 0;
+    // places of the block after the current one: B and C, the row of h it writes, the row of h above it, the column left of it
+    const unsigned char *nbc = nullptr;
+    float4 *nrow = nullptr, *ncol = nullptr;
+    const int64_t up = KEEP ? (int64_t)P.nstrip * 4 * P.NL : 0;   // from a block's row of h back to the one above it
+    auto place = [&](const BkPos &q) {   // at the start of a row of blocks
+        const int blk = q.pass * rw + w;
+        const int64_t lin = ((int64_t)q.bg * P.nsl + min(q.slot + sl_, P.nsl - 1)) * NG + n;
+        nbc = reinterpret_cast<const unsigned char *>(P.bc + ((int64_t)q.bg * P.nblk + blk) * P.nstrip * BK_PX * NG);
+        nrow = P.row + (int64_t)(KEEP ? blk : 0) * P.nstrip * 4 * P.NL + lin;
+        ncol = P.col + ((int64_t)blk * (P.nstrip - 1) - 1) * 4 * P.NL + lin;
+    };
+    // half k of the row of h above block `q`, whose row of h goes to nrow
+    auto fetch = [&](const BkPos &q, int k) {
+        const bool there = q.pass * rw + w > 0;
+        const float4 *src = nrow - up + 2 * k * P.NL;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float4 v = there ? src[i * P.NL] : make_float4(0.f, 0.f, 0.f, 0.f);
+            hup[4 * k + 2 * i] = f2(v.x, v.y); hup[4 * k + 2 * i + 1] = f2(v.z, v.w);
+        }
+    };
+    auto enter = [&](const BkPos &q) {   // the first block after a pause: everything its predecessor would have started
+        place(q);
+        load_raw(q);
+        copy_bc(nbc, 0, true); copy_bc(nbc, 1, true); copy_bc(nbc, 2, true);
+        if (!chain) { fetch(q, 0); fetch(q, 1); }
+    };
+    if (w == 0 && live(pos, 0)) enter(pos);
+    for (int g = 0; g < steps; ++g) {
+        const int L = g - BK_LAG * w;
+        BkPos nxt = pos;
+        if (L >= 0) nxt.next(P, SPW, stride);
+        const bool non = live(nxt, L + 1);
+        if (!live(pos, L)) {   // before the worker's first block, past its last row of blocks, or past its items
+            if (non) enter(nxt);
+            if (rw > 1) __syncthreads();
+            pos = nxt;
+            continue;
+        }
+        const int blk = pos.pass * rw + w, G0 = pos.g;
+        const unsigned char *tbc = nbc;
+        float4 *trow = nrow, *tcol = ncol;
+        if (nxt.strip == 0) { if (non) place(nxt); }
+        else { nbc += BK_PX * NG * 8; nrow += 4 * P.NL; ncol += 4 * P.NL; }
+        const bool mine = pos.slot + sl_ < P.nsl;
+        {
+            const int ch0 = pos.slot * 2, cg = G0 * P.dpg + ch0, nch = P.dpg - ch0, r0 = blk * BK_R;
+            const bool pix = r0 + lr < P.H && pos.strip * BK_S + lc < P.W;
+            if (pos.strip == 0) {
+                const bool fh = (P.flip_h >> G0) & 1u, fw = (P.flip_w >> G0) & 1u;
+                const int r = r0 + ((lane >> 2) & 3), c = lane & 3;
+                oo = (int64_t)(pos.bg / P.G) * P.o_bs + (int64_t)((P.mw ? ch0 : cg) + 2 * (lane >> 4)) * P.o_ds +
+                     (int64_t)(fh ? P.H - 1 - r : r) * P.o_hs + (fw ? P.W - 1 - c : c);
+                if (pos.pass == 0) {   // a new item
+                    const int c0 = min(2 * sl_, nch - 1), c1 = min(2 * sl_ + 1, nch - 1);
+                    const float *a = P.A + (int64_t)cg * P.A_ds + n * P.A_ns;
+                    A2 = n < P.N ? f2(__ldg(a + c0 * P.A_ds) * LOG2E, __ldg(a + c1 * P.A_ds) * LOG2E) : bc(0.f);
+                    if (lane < SPW) {
+                        const int k = 2 * lane;
+                        sPar[lane] = make_float4(P.bias && k < nch ? __ldg(P.bias + (cg + k) / P.drep) : 0.f, P.bias && k + 1 < nch ? __ldg(P.bias + (cg + k + 1) / P.drep) : 0.f,
+                                                 P.D && k < nch ? __ldg(P.D + cg + k) : 0.f, P.D && k + 1 < nch ? __ldg(P.D + cg + k + 1) : 0.f);
+                    }
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int r = 0; r < BK_R; ++r) { hl[r] = al[r] = ql[r] = sl[r] = bc(0.f); }
+                hcorner = bc(0.f);
+            } else if (KEEP) {   // q, s of the column left of the block
+#pragma unroll
+                for (int r = 0; r < BK_R; ++r) bk_st16(tcol + r * P.NL, make_float4(ql[r].x, ql[r].y, sl[r].x, sl[r].y), mine);
+            }
+            // ---- stage: pixels and channels outside the image get dl = 0 (a = 1 or the decay, p = 0) ----
+#pragma unroll
+            for (int i = 0; i < SPW; ++i) {
+                const float4 par = sPar[i];
+                const float2 uv = f2(bk_cvt<DT>(vu[2 * i]), bk_cvt<DT>(vu[2 * i + 1]));
+                float2 dl = f2(bk_cvt<DT>(vd[2 * i]) + par.x, bk_cvt<DT>(vd[2 * i + 1]) + par.y);
+                if (softplus) dl = bk_softplus2<false>(dl, nullptr);
+                dl = f2(pix && 2 * i < nch ? dl.x : 0.f, pix && 2 * i + 1 < nch ? dl.y : 0.f);
+                const float2 dlu = mul2(dl, uv);
+                sIn[i * 33 + lane] = make_float4(dl.x, dl.y, dlu.x, dlu.y);
+                sY0[i * 33 + lane] = mul2(uv, f2(par.z, par.w));
+            }
+#pragma unroll
+            for (int i = 0; i < SPW / 2; ++i) {
+                const int k = lr + 4 * i;
+                const float4 par = sPar[k >> 1];
+                float2 dl = bc(bk_cvt<DT>(vt[i]) + ((k & 1) ? par.y : par.x));
+                if (softplus) dl = bk_softplus2<false>(dl, nullptr);
+                reinterpret_cast<float *>(sTop)[((k >> 1) * 9 + lc) * 2 + (k & 1)] = dl.x;   // (columns outside the image meet h = 0)
+            }
+        }
+        __syncwarp();
+        if (non) load_raw(nxt);
+        // Software pipeline over the block's pixels (column by column): the shared-memory loads of a pixel are issued two
+        // pixels ahead, its exponential and products one ahead.
+        const float4 *tIn = sIn + sl_ * 33;
+        const float2 *tTop = sTop + sl_ * 9;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            float2 hb[4];
+#pragma unroll
+            for (int qt = 2 * k; qt < 2 * k + 2; ++qt) {
+                bk_wait<2>();
+                __syncwarp();   // this quarter's B and C are here, the quarter before it has been read by all lanes
+                copy_bc(qt == 0 ? tbc : nbc, (qt + 3) & 3, qt == 0 || non);
+                {
+                    const float2 *tBC = sBC + qt * 8 * NG + (NG == 16 ? (n & 7) * 2 + (n >> 3) : n);
+                    float4 rin[2];
+                    float2 rbc[2];
+                    float2 hd, hu, au;
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) { rin[x] = tIn[(x % 4) * BK_S + qt * 2 + x / 4]; rbc[x] = tBC[x * NG]; }
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) {
+                        const int c = qt * 2 + x / 4, r = x % 4, cc = c & 3;
+                        const float4 in = rin[x & 1];
+                        const float2 b = rbc[x & 1];
+                        if (x + 2 < 8) { rin[x & 1] = tIn[((x + 2) % 4) * BK_S + qt * 2 + (x + 2) / 4]; rbc[x & 1] = tBC[(x + 2) * NG]; }
+                        if (r == 0) { hd = hcorner; hu = hcorner = hup[c]; au = blk > 0 ? ex2_2(fma2(tTop[c], A2, lgd)) : bc(0.f); }
+                        const float2 a = ex2_2(fma2(f2(in.x, in.y), A2, lgd));
+                        const float2 p = mul2(bc(b.x), f2(in.z, in.w));
+                        const float2 t = mul2(add2(au, al[r]), hd);
+                        const float2 z = add2(ql[r], fma2(t, bc(-0.5f), hu));
+                        const float2 s = fma2(a, sl[r], p);
+                        const float2 q = mul2(a, z), h = fma2(a, z, s);
+                        sY[(r * 4 + cc) * YP + lane] = mul2(bc(b.y), fma2(p, bc(0.25f), q));
+                        hd = hl[r]; hu = h; au = a;
+                        hl[r] = h; al[r] = a; ql[r] = q; sl[r] = s;
+                        if (r == BK_R - 1) hb[cc] = h;
+                    }
+                }
+            }
+            if (blk + 1 < P.nblk) {   // the block's last row of h
+                bk_st16(trow + 2 * k * P.NL, make_float4(hb[0].x, hb[0].y, hb[1].x, hb[1].y), mine);
+                bk_st16(trow + (2 * k + 1) * P.NL, make_float4(hb[2].x, hb[2].y, hb[3].x, hb[3].y), mine);
+            }
+            // Half k of the row of h above the next block into the registers of half k of this one's, which are done with: the
+            // loads travel while the other half is computed.  What they read was written at least two steps ago.
+            if (chain) {   // the block below is next
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) hup[k * 4 + cc] = nxt.pass > 0 ? hb[cc] : bc(0.f);
+            } else if (non) {
+                fetch(nxt, k);
+            }
+            __syncwarp();
+            {   // sums over the states of half a block: a lane takes one pixel of every second slot
+                const bool fw = (P.flip_w >> G0) & 1u;
+                const int px = lane & 15, c0 = pos.strip * BK_S + k * 4, nch = P.dpg - pos.slot * 2 - 2 * (lane >> 4);
+                const bool okp = blk * BK_R + (px >> 2) < P.H && c0 + (px & 3) < P.W;
+                const int64_t o = oo + (fw ? -c0 : c0);
+#pragma unroll
+                for (int i = 0; i < SPW / 2; ++i) {
+                    const int s2 = (lane >> 4) + 2 * i;
+                    const float4 *yp = reinterpret_cast<const float4 *>(sY + px * YP + s2 * NG);
+                    float2 v = sY0[s2 * 33 + (px >> 2) * BK_S + k * 4 + (px & 3)], v2 = bc(0.f);
+#pragma unroll
+                    for (int m = 0; m < NG / 2; ++m) {
+                        const float4 t = yp[m];
+                        v = add2(v, f2(t.x, t.y)); v2 = add2(v2, f2(t.z, t.w));
+                    }
+                    v = add2(v, v2);
+                    const int64_t oi = o + (int64_t)(4 * i) * P.o_ds;
+                    const bool ok0 = okp && 4 * i < nch, ok1 = okp && 4 * i + 1 < nch;
+                    if (P.mw) {
+                        const float *m = P.mw + G0 * P.dpg + pos.slot * 2 + 2 * s2;
+                        bk_st<CS2D_F32, true>(P.out, oi, ok0 ? v.x * __ldg(m) : 0.f, ok0);
+                        bk_st<CS2D_F32, true>(P.out, oi + P.o_ds, ok1 ? v.y * __ldg(m + 1) : 0.f, ok1);
+                    } else if (P.out_dt == CS2D_F32) {
+                        bk_st<CS2D_F32, false>(P.out, oi, v.x, ok0);
+                        bk_st<CS2D_F32, false>(P.out, oi + P.o_ds, v.y, ok1);
+                    } else {
+                        bk_st<DT, false>(P.out, oi, v.x, ok0);
+                        bk_st<DT, false>(P.out, oi + P.o_ds, v.y, ok1);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (rw > 1) __syncthreads();   // the rows of h written in this step are there for the other workers
+        pos = nxt;
+    }
+    bk_wait<0>();
+}
+
+template <int NG, int DT, bool KEEP>
+static cudaError_t launch(const Blk &P, cudaStream_t st) {
+    auto kernel = blk_fwd_kernel<NG, DT, KEEP>;
+    constexpr int smem = BkFwd<NG>::total * BK_WARPS;
+    static bool attr_done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !attr_done[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) attr_done[dev] = true;
+    }
+    blk_bc_kernel<DT><<<P.nblk * P.nstrip * (P.items / P.ntile), 128, 0, st>>>(P, NG);
+    kernel<<<P.grid, BK_WARPS * 32, smem, st>>>(P);
+    return cudaGetLastError();
+}
+template <int NG>
+static cudaError_t launch_dt(const Blk &P, cudaStream_t st) {
+    switch (P.io_dt) {
+        case CS2D_F32: return P.roll ? launch<NG, CS2D_F32, false>(P, st) : launch<NG, CS2D_F32, true>(P, st);
+        case CS2D_F16: return P.roll ? launch<NG, CS2D_F16, false>(P, st) : launch<NG, CS2D_F16, true>(P, st);
+        default: return P.roll ? launch<NG, CS2D_BF16, false>(P, st) : launch<NG, CS2D_BF16, true>(P, st);
+    }
+}
+
+cudaError_t launch_blk_fwd(const Blk &P, int NG, cudaStream_t st) {
+    switch (NG) {
+        case 16: return launch_dt<16>(P, st);
+        case 8: return launch_dt<8>(P, st);
+    }
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace cs2d

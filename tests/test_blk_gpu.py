@@ -1,0 +1,101 @@
+"""The block-walk kernels (three or more states, at least eight channels per group) against the float64 oracle: images of
+one block and less, ragged in both directions, one to four row workers per CTA, odd channel counts (a slot with one live
+half), every number of state slots, delta shared by channels (the addresses of neighbouring channels coincide), fp32
+results of 16-bit inputs, rows that do and do not allow groups of four, state decay, and the deterministic
+backward, which makes the tile kernels' checkpoints again."""
+import pytest
+import torch
+
+from conftest import TOL, check_close
+import cs2d
+from cs2d.synthetic import make_inputs
+from oracle import cs2d_oracle as O
+
+pytestmark = pytest.mark.gpu
+NAMES = ("du", "ddelta", "dA", "dB", "dC", "dD", "ddelta_bias", "dA_decay")
+
+CASES = [
+    ((1, 1, 8, 3, 1, 1), torch.float32, {}),           # a single pixel
+    ((1, 2, 9, 16, 4, 8), torch.float32, {}),          # exactly one block; an odd number of channels
+    ((2, 1, 8, 8, 5, 9), torch.float32, {}),           # one row and one column more than a block
+    ((1, 1, 11, 9, 40, 7), torch.float32, {}),         # one block per row: the row of h stays in registers or waits for the workers
+    ((3, 1, 10, 16, 9, 33), torch.bfloat16, {}),       # 5 blocks per row, two row workers with a short last pass
+    ((1, 2, 12, 5, 27, 70), torch.float16, {}),        # 9 blocks per row, four row workers
+    ((1, 1, 16, 16, 16, 64), torch.float32, {"delta_dim": 4}),
+    ((2, 1, 8, 7, 13, 20), torch.float32, {"a_decay": 0.9, "with_bias": False}),
+    ((1, 4, 8, 16, 12, 300), torch.float32, {"with_D": False}),   # wider than a tile launch
+    ((40, 1, 34, 16, 6, 10), torch.float32, {}),       # more warps than the GPU holds at once
+]
+
+
+def _dev(inp):
+    return {k: (v.cuda() if v is not None else None) for k, v in inp.items()}
+
+
+def _oracle(inp, softplus=True):
+    f = {k: (v.float() if v is not None else None) for k, v in inp.items()}
+    a = (f["u"], f["delta"], f["A"], f["B"], f["C"], f["D"], f["delta_bias"])
+    return O.fwd(*a, softplus, f["A_decay"]), O.bwd(*a, f["dout"], softplus, f["A_decay"])
+
+
+@pytest.mark.parametrize("det", [False, True], ids=["atomic", "deterministic"])
+@pytest.mark.parametrize("shape,dtype,kw", CASES, ids=[f"{s}-{str(d)[6:]}" for s, d, _ in CASES])
+def test_block_walk_against_oracle(shape, dtype, kw, det):
+    if det and (shape[-1] > 256 or (shape[-1] > 64 and shape[3] <= 8)):
+        pytest.skip("no deterministic backward for these rows")
+    inp = make_inputs(*shape, dtype=dtype, seed=12, **kw)
+    d = _dev(inp)
+    args = (d["u"], d["delta"], d["A"], d["B"], d["C"], d["D"], d["delta_bias"])
+    out, x, xv, xsd = cs2d.fwd(*args, True, False, d["A_decay"])
+    g = cs2d.bwd(*args, d["dout"], x, xv, True, d["A_decay"], xsd, deterministic=det)
+    assert torch.equal(cs2d.fwd_only(*args, True, False, d["A_decay"]), out)
+    yo, go = _oracle(inp)
+    rtol, atol = TOL[str(dtype)[6:]]
+    check_close("out", out.float().cpu().numpy(), yo, rtol, atol)
+    for name, t in zip(NAMES, g):
+        ref = go["dA_decay_ref" if name == "dA_decay" else name]
+        if ref is None:
+            assert t is None, name
+            continue
+        check_close(name, t.float().cpu().numpy(), ref, rtol, atol)
+    assert cs2d.device_status() == 0
+
+
+def test_fp32_results_of_strided_16bit_inputs_without_softplus():
+    inp = make_inputs(2, 2, 10, 6, 11, 19, dtype=torch.bfloat16, seed=5, with_bias=False)
+    inp["delta"] = (inp["delta"].float().abs() * 0.1).to(torch.bfloat16)
+    d = _dev(inp)
+    big = torch.zeros(2, 30, 11, 24, dtype=torch.bfloat16, device="cuda")
+    big[:, 7:27, :, 3:22] = d["u"]
+    d["u"] = big[:, 7:27, :, 3:22]              # channels and columns of a larger tensor
+    d["B"] = d["B"].transpose(0, 1).contiguous().transpose(0, 1)
+    args = (d["u"], d["delta"], d["A"], d["B"], d["C"], d["D"], d["delta_bias"])
+    o = cs2d.fwd(*args, False, True, None)
+    assert o[0].dtype == torch.float32
+    g = cs2d.bwd(*args, d["dout"].float(), o[1], o[2], False, None, o[3])
+    yo, go = _oracle(inp, softplus=False)
+    check_close("out", o[0].cpu().numpy(), yo, 1e-4, 1e-5)   # fp32 output: arithmetic error only
+    for name, t in zip(NAMES, g):
+        if t is not None:
+            check_close(name, t.float().cpu().numpy(), go[name], 2e-2, 1e-3)
+
+
+@pytest.mark.parametrize("shape,dtype", [((1, 4, 9, 16, 10, 21), torch.float32), ((2, 4, 8, 4, 19, 44), torch.bfloat16)])
+def test_four_corner_merge(shape, dtype):
+    b, K, dd, n, h, w = shape
+    inp = make_inputs(b, K, dd, n, h, w, dtype=dtype, seed=2)
+    gen = torch.Generator().manual_seed(9)
+    host = dict(u=torch.randn(b, dd, h, w, generator=gen).to(dtype), delta=inp["delta"], A=inp["A"], B=inp["B"], C=inp["C"],
+                w=torch.rand(K, dd, generator=gen) - 0.3, D=inp["D"], delta_bias=inp["delta_bias"])
+    dy = torch.randn(b, dd, h, w, generator=gen).to(dtype)
+    dev = {k: v.cuda().requires_grad_(True) for k, v in host.items()}
+    y = cs2d.cross_scan_2d(*dev.values(), True)
+    y.backward(dy.cuda())
+    ref = {k: v.double().requires_grad_(True) for k, v in host.items()}
+    yo = O.cross_fwd_torch(*ref.values(), True)
+    yo.backward(dy.double())
+    rtol, atol = TOL[str(dtype)[6:]]
+    check_close("y", y.detach().float().cpu().numpy(), yo.detach().numpy(), rtol, atol)
+    for k in host:
+        check_close("d" + k, dev[k].grad.float().cpu().numpy(), ref[k].grad.numpy(), rtol, atol)
+    assert cs2d.device_status() == 0
