@@ -67,7 +67,9 @@ typedef struct {
  * Bytes of the saved-state buffer the forward writes and the backward reads:
  * row checkpoints of the state h; for problems with more than two states and
  * at least eight channels per group (the block-walk kernels) also h and the
- * row scan at every eighth column and B and C regrouped.  It takes the place of
+ * row scan at every eighth column and B and C regrouped; for those with a single
+ * state (the pair-walk kernels) the same with the transition in place of B and C.
+ * It takes the place of
  * the reference's three side tensors x, x_v, x_sd (selective_scan_oflex.cpp:251-258);
  * unlike them it is NOT modified by the backward, so backward may run twice on it.
  * A backward reads what the forward of the SAME problem, directions and flags wrote.

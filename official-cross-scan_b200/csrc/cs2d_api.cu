@@ -1,12 +1,14 @@
 // extern "C" boundary of the cs2d library: validation, launch geometry, errors.
 // Mirrors the checks of the reference host binding
 // (src/cusoflex/selective_scan_oflex.cpp:188-245 and :298-391) on raw pointers.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <initializer_list>
 
 #include "cs2d_blk.cuh"
+#include "cs2d_pair.cuh"
 #include "cs2d_common.cuh"
 
 namespace cs2d {
@@ -20,6 +22,8 @@ int stream_pairs_per_cta(int L);
 cudaError_t launch_walk_fwd(const Dev &P, int grid, cudaStream_t st);
 cudaError_t launch_blk_fwd(const Blk &P, int NG, cudaStream_t st);
 cudaError_t launch_blk_bwd(const Blk &P, int NG, cudaStream_t st);
+cudaError_t launch_pair_fwd(const Pw &P, bool keep, cudaStream_t st);
+cudaError_t launch_pair_bwd(const Pw &P, cudaStream_t st);
 void walk_geometry(int ncols, int *swd, int *lr);
 int walk_channels_per_cta(int lr);
 size_t walk_bc_bytes(int batch, int groups, int nrows, int ncols);
@@ -276,6 +280,16 @@ static size_t blk_bc_bytes(const Blk &k, int NG);
 
 static bool blk_shape(const cs2d_problem *p) { return p->dstate > 2 && p->dim / p->n_groups >= 8; }
 
+static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool backward, const void *img = nullptr, int64_t img_bs = 0,
+                      int64_t img_ds = 0, int64_t img_hs = 0);
+static size_t pair_row_bytes(const Pw &k, bool roll);
+static size_t pair_col_bytes(const Pw &k);
+
+// (a warp of the pair-walk kernels works on 64 channels: too few of them and it is idle)
+static bool pair_shape(const cs2d_problem *p) {
+    return p->dstate == 1 && p->dim / p->n_groups >= 8 && p->delta_softplus && !p->A_decay && p->delta_dim == p->dim;
+}
+
 static size_t edge_bytes(const cs2d_problem *p, int NPp) {
     return (size_t)p->batch * p->dim * NPp * p->nrows * sizeof(float4);
 }
@@ -299,12 +313,19 @@ static size_t layout_bytes(const cs2d_problem *p, bool backward, bool rolling = 
     return total;
 }
 
-// Problems of the block-walk kernels: what those need, or the tile kernels, which the reproducible direction merge
-// uses - the size depends on the problem alone.
+// Problems of the block-walk and the pair-walk kernels: what those need, or the tile kernels, which the reproducible
+// direction merge uses - the size depends on the problem alone.
 static size_t state_bytes(const cs2d_problem *p, bool backward, bool rolling) {
     if (validate(p) != CS2D_OK) return 0;
     const size_t tile = layout_bytes(p, backward, rolling);
-    if (tile == 0 || !blk_shape(p)) return tile;
+    if (tile == 0) return tile;
+    if (pair_shape(p)) {
+        Pw k;
+        pair_fill(k, p, nullptr, backward);
+        const size_t need = backward || rolling ? pair_row_bytes(k, true) : pair_row_bytes(k, false) + pair_col_bytes(k);
+        return tile > need ? tile : need;
+    }
+    if (!blk_shape(p)) return tile;
     Blk k;
     int NG;
     blk_fill(k, NG, p, nullptr, backward);
@@ -431,6 +452,99 @@ static size_t blk_row_bytes(const Blk &k, bool roll) { return (size_t)(roll ? 1 
 static size_t blk_bc_bytes(const Blk &k, int NG) { return (size_t)(k.items / k.ntile) * k.nblk * k.nstrip * BK_PX * NG * sizeof(float2); }
 static size_t blk_col_bytes(const Blk &k) { return (size_t)k.nblk * (k.nstrip - 1) * 4 * k.NL * sizeof(float4); }
 
+// ---- pair-walk kernels (cs2d_pair_fwd.cu, cs2d_pair_bwd.cu) -------------------------------------------
+// One scan orientation and rows of at most 128 columns also have the streaming kernels, which lose where they load a row
+// element by element or word by word (measured, training step with 6k to 200k channels, streaming / pair-walk us: 16-bit
+// 7 columns 494 / 178, 14: 395 / 281, 22: 338 / 265, 37: 1120 / 861, but 16: 260 / 258, 28: 259 / 340, 30: 357 / 415, 61: 733 / 843;
+// fp32 7 columns 513 / 192, 16: 637 / 424, 56: 738 / 785).  The alternative of directions and of wider rows are the tile
+// kernels (28x28 cross 2133 / 398, 150x150 scan 21944 / 4273), except where a few warps' worth of channels on a large map
+// would leave the GPU idle (8 items of 224x224: 4265 / 7178; of 56x56: 794 / 507).
+static bool pair_ok(const cs2d_problem *p, const cs2d_dirs *o) {
+    if (!pair_shape(p) || (o && o->merge_w && (o->flags & CS2D_DIRS_SERIAL))) return false;
+    const int W = p->ncols, dpg = p->dim / p->n_groups;
+    if (has_dirs(o) || W > 16 * STRIP)
+        return W <= 64 || (int64_t)p->batch * p->n_groups * ((dpg + PW_CH - 1) / PW_CH) >= 16;
+    if (p->io_dtype == CS2D_F32) return W <= 16;
+    return W < 16 || (W % 2 ? W <= 45 : W % 4 && W <= 24);
+}
+// Bytes that may be moved at once, 8 at most: a divisor of every size and stride (in bytes) and of the address
+static int move_bytes(const void *ptr, std::initializer_list<int64_t> sizes) {
+    uintptr_t x = reinterpret_cast<uintptr_t>(ptr) | 8;
+    for (int64_t s : sizes) x |= (uintptr_t)s;
+    return (int)(x & (~x + 1));
+}
+static int lanes_for(int pieces) {
+    int l = 8;
+    while (l < pieces) l <<= 1;
+    return l;
+}
+static void pair_state(Pw &k, const void *saved, bool roll) {
+    char *q = const_cast<char *>(static_cast<const char *>(saved));
+    k.row = reinterpret_cast<float4 *>(q);
+    q += pair_row_bytes(k, roll);
+    k.colq = reinterpret_cast<float4 *>(q);
+    k.cola = reinterpret_cast<float2 *>(q + pair_col_bytes(k) / 3 * 2);
+}
+static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool backward, const void *img, int64_t img_bs, int64_t img_ds, int64_t img_hs) {   // img: out or dout
+    k = Pw{};
+    const int es = esize(p->io_dtype);
+    k.H = p->nrows; k.W = p->ncols; k.G = p->n_groups; k.dpg = p->dim / p->n_groups; k.io_dt = p->io_dtype;
+    k.u = p->u; k.delta = p->delta; k.B = p->B; k.C = p->C; k.A = p->A; k.D = p->D; k.bias = p->delta_bias;
+    k.u_bs = p->u_bs; k.u_ds = p->u_ds; k.u_hs = p->u_hs;
+    k.dl_bs = p->delta_bs; k.dl_ds = p->delta_ds; k.dl_hs = p->delta_hs; k.A_ds = p->A_ds;
+    k.B_bs = p->B_bs; k.B_gs = p->B_gs; k.B_hs = p->B_hs;
+    k.C_bs = p->C_bs; k.C_gs = p->C_gs; k.C_hs = p->C_hs;
+    if (o) {
+        k.flip_h = o->flip_rows_mask; k.flip_w = o->flip_cols_mask; k.shared = o->shared_input;
+        k.mw = o->merge_w; k.dw = o->merge_dw;
+    }
+    k.f32 = p->io_dtype != CS2D_F32 && p->out_dtype == CS2D_F32;
+    k.nblk = (k.H + PW_R - 1) / PW_R; k.nsub = (k.W + 7) / 8; k.wp = (k.W + 1) & ~1;
+    k.ntile = (k.dpg + PW_CH - 1) / PW_CH; k.items = p->batch * k.G * k.ntile;
+    // How blocks are moved (see cs2d_pair.cuh): whole bands where every tensor's rows are contiguous and a band fits
+    struct In { const void *p; int64_t bs, ds, hs; } in[3] = {{p->u, p->u_bs, p->u_ds, p->u_hs}, {p->delta, p->delta_bs, p->delta_ds, p->delta_hs}, {img, img_bs, img_ds, img_hs}};
+    const int ni = backward && img && !k.f32 ? 3 : 2;
+    k.lin = PW_R * k.W * es + (k.W & 1 ? 2 : 0) <= 128;
+    for (int i = 0; i < ni; ++i) k.lin = k.lin && in[i].hs == k.W;
+    if (!backward && img && !k.mw && !k.f32) k.lin = k.lin && img_hs == k.W;
+    k.vin = 8;
+    for (int i = 0; i < ni; ++i)
+        k.vin = std::min(k.vin, k.lin ? move_bytes(in[i].p, {in[i].bs * es, in[i].ds * es, (int64_t)PW_R * k.W * es, (int64_t)k.H * k.W * es})
+                                      : move_bytes(in[i].p, {in[i].bs * es, in[i].ds * es, in[i].hs * es, (int64_t)k.W * es}));
+    if (k.W & 1) k.vin = std::min(k.vin, es);
+    k.el = k.vin < 2 * es;
+    if (k.vin < 4) k.vin = 4;
+    k.fs = k.el && es == 2 && !k.lin ? 8 : 32 / es;
+    k.nstrip = k.lin ? 1 : (k.W + k.fs - 1) / k.fs;
+    k.lpin = k.lin ? lanes_for((PW_R * k.W * es + (k.el && es == 2 ? 2 : 0) + k.vin - 1) / k.vin) : 4 * (k.el && es == 2 ? 8 : 32 / k.vin);
+    // Row workers: as few as fill the GPU; with short rows a worker waits for the others at the end of a band
+    const int ctas = backward ? 2 : 3;
+    const int64_t slots = (int64_t)kSMs * ctas * PW_WARPS;
+    double best = 1e300;
+    for (int rwl = 0; rwl < 3; ++rwl) {
+        const int rw = 1 << rwl;
+        if (rw > 1 && k.nblk < rw) break;
+        const int period = k.nstrip < rw ? rw : k.nstrip;
+        const int64_t npass = (k.nblk + rw - 1) / rw, rounds = ((int64_t)k.items * rw + slots - 1) / slots;
+        const double cost = (double)rounds * (npass * period + rw - 1);
+        if (cost < best * 0.9) { best = cost; k.rwl = rwl; k.npass = (int)npass; k.period = period; }
+    }
+    const int64_t need = ((int64_t)k.items + (PW_WARPS >> k.rwl) - 1) / (PW_WARPS >> k.rwl), cap = ctas * kSMs;
+    k.grid = (int)(need < cap ? need : cap);
+}
+static size_t pair_row_bytes(const Pw &k, bool roll) { return (size_t)k.items * (roll ? 1 : k.nblk - 1) * k.wp * 32 * sizeof(float4); }
+static size_t pair_col_bytes(const Pw &k) { return (size_t)k.items * k.nblk * (k.nsub - 1) * PW_R * 32 * 24; }
+// pieces of results that take the place of inputs in shared memory
+static int pair_vout(const Pw &k, const void *ptr, int es, int64_t bs, int64_t ds, int64_t hs) {
+    if (k.el && es == 2) return 2;
+    if (k.lin) return move_bytes(ptr, {bs * es, ds * es, (int64_t)PW_R * k.W * es, (int64_t)k.H * k.W * es});
+    return move_bytes(ptr, {bs * es, ds * es, hs * es, (int64_t)k.W * es});
+}
+static void pair_out(Pw &k, int es, int vout) {
+    k.vout = std::min(vout, k.vin);
+    k.lpout = k.lin ? lanes_for(PW_R * k.W * es / k.vout) : 4 * k.fs * es / k.vout;
+}
+
 static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_t out_bs, int64_t out_ds,
                     int64_t out_hs, void *saved, void *stream, bool rolling = false, bool tile = false) {
     int rc = validate(p);
@@ -443,6 +557,19 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
     if (reinterpret_cast<uintptr_t>(saved) & 15) return fail(CS2D_ERR_INVALID, "saved must be 16-byte aligned");
     int *status = status_ptr();
     if (!status) return fail(CS2D_ERR_CUDA, "cannot locate the device status word");
+    if (!tile && pair_ok(p, o)) {
+        Pw k;
+        pair_fill(k, p, o, false, out, out_bs, out_ds, out_hs);
+        k.out = out; k.o_bs = out_bs; k.o_ds = out_ds; k.o_hs = out_hs;
+        const int es = esize(p->io_dtype);
+        pair_out(k, es, pair_vout(k, out, es, out_bs, out_ds, out_hs));
+        k.v32 = move_bytes(out, {out_bs * 4, out_ds * 4, out_hs * 4, (int64_t)k.W * 4}) == 8;
+        pair_state(k, saved, rolling);
+        cudaError_t e = launch_pair_fwd(k, !rolling, reinterpret_cast<cudaStream_t>(stream));
+        if (e != cudaSuccess) return fail(CS2D_ERR_CUDA, "forward launch failed: %s", cudaGetErrorString(e));
+        g_launches.fetch_add(1);
+        return CS2D_OK;
+    }
     if (stream_ok(p, o)) {
         Dev d;
         int L, grid;
@@ -586,8 +713,8 @@ static int det_layout(const cs2d_problem *p, DetLayout *l) {
     l->dB = 0; l->dC = l->dB + l->ntiles * l->nB; l->dA = l->dC + l->ntiles * l->nB;
     l->dD = l->dA + (int64_t)p->batch * p->dim * p->dstate; l->dbias = l->dD + (int64_t)p->batch * p->dim;
     l->ddecay = l->dbias + (int64_t)p->batch * p->dim; l->total = l->ddecay + l->grid;
-    l->state = (l->total + 3) & ~int64_t(3);   // problems of the block-walk kernels: the tile kernels' checkpoints
-    if (blk_shape(p)) l->total = l->state + (int64_t)(layout_bytes(p, false) / 4);
+    l->state = (l->total + 3) & ~int64_t(3);   // problems of the block-walk and pair-walk kernels: other kernels' checkpoints
+    if (blk_shape(p) || pair_shape(p)) l->total = l->state + (int64_t)(layout_bytes(p, false) / 4);
     return CS2D_OK;
 }
 
@@ -610,6 +737,22 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
     if (dA_decay && !p->A_decay) return fail(CS2D_ERR_INVALID, "dA_decay requested without A_decay");
     int *status = status_ptr();
     if (!status) return fail(CS2D_ERR_CUDA, "cannot locate the device status word");
+    if (!det && pair_ok(p, o)) {
+        Pw k;
+        pair_fill(k, p, o, true, dout, dout_bs, dout_ds, dout_hs);
+        pair_state(k, saved, false);
+        k.out = const_cast<void *>(dout); k.o_bs = dout_bs; k.o_ds = dout_ds; k.o_hs = dout_hs;
+        const int es = esize(p->io_dtype);
+        const int64_t W = p->ncols, HW = W * p->nrows;
+        pair_out(k, es, std::min(pair_vout(k, du, es, HW, HW, W), pair_vout(k, ddelta, es, HW, HW, W)));
+        k.v32 = move_bytes(du, {HW * 4, W * 4}) == 8;
+        k.adj = reinterpret_cast<float4 *>(scratch);
+        k.du = du; k.ddelta = ddelta; k.dA = dA; k.dB = dB; k.dC = dC; k.dD = dD; k.dbias = ddelta_bias;
+        cudaError_t e = launch_pair_bwd(k, reinterpret_cast<cudaStream_t>(stream));
+        if (e != cudaSuccess) return fail(CS2D_ERR_CUDA, "backward launch failed: %s", cudaGetErrorString(e));
+        g_launches.fetch_add(1);
+        return CS2D_OK;
+    }
     if (!det && blk_ok(p, o)) {
         Blk k;
         int NG;
@@ -624,8 +767,8 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
         g_launches.fetch_add(1);
         return CS2D_OK;
     }
-    if (det && blk_ok(p, o)) {
-        // The deterministic backward is the tile kernels'; their checkpoints are made again (y goes to du, which is
+    if (det && (blk_ok(p, o) || pair_ok(p, o))) {
+        // The deterministic backward is the tile kernels'; the checkpoints it reads are made again (y goes to du, which is
         // written later).
         cs2d_problem q = *p;
         q.out_dtype = p->io_dtype;

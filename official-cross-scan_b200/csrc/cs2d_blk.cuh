@@ -59,6 +59,8 @@ struct Blk {
     int vec_dbc;                            // dB, dC: rows of whole aligned groups of four columns
 };
 
+// stores to tensor memory have been made
+__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // 16-byte asynchronous copies to shared memory, in groups
 __device__ __forceinline__ void bk_cp16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");

@@ -26,7 +26,6 @@ __device__ __forceinline__ void tm_st(uint32_t a, float2 x) {
 __device__ __forceinline__ void tm_ld(uint32_t a, float2 (&x)[2]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=f"(x[0].x), "=f"(x[0].y), "=f"(x[1].x), "=f"(x[1].y) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void tm_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // the loaded values pass through the wait, so that nothing uses them before it
 __device__ __forceinline__ void tm_wait_ld(float2 (&x)[2]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(x[0].x), "+f"(x[0].y), "+f"(x[1].x), "+f"(x[1].y)::"memory");
