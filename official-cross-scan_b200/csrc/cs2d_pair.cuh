@@ -175,11 +175,12 @@ struct PwView {
         }
     }
     // x[0], x[1]: scan columns c, c + 1 of scan row r; `o` is the offset of column c, `o1` that of column c + 1 (EL) or of the
-    // lower of the two in memory
-    __device__ __forceinline__ void load(int r, int k, int o, int o1, bool rev, float (&x)[2]) const {
+    // lower of the two in memory.  What is not there (on, on1: row r, column c + 1 exist) is zero; EL: in its place there are other
+    // elements, which share words or rows with the block.
+    __device__ __forceinline__ void load(int r, int k, int o, int o1, bool rev, bool on, bool on1, float (&x)[2]) const {
         if constexpr (EL) {
             const uint32_t p = a[r & 1][k];
-            x[0] = elem(p + o); x[1] = elem(p + o1);
+            x[0] = elem(p + o, on); x[1] = elem(p + o1, on && on1);
         } else {
             const uint32_t p = a[0][0] + k * PW_HALF + o1;
             uint32_t lo, hi;
@@ -212,14 +213,14 @@ struct PwView {
             }
         }
     }
-    static __device__ __forceinline__ float elem(uint32_t p) {
+    static __device__ __forceinline__ float elem(uint32_t p, bool on) {
         if constexpr (ES == 4) {
             uint32_t v;
-            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.shared.b32 %0, [%1];\n\t}" : "=r"(v) : "r"(p), "r"((int)on) : "memory");
             return __uint_as_float(v);
         } else {
             unsigned short v;
-            asm volatile("ld.shared.b16 %0, [%1];" : "=h"(v) : "r"(p) : "memory");
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b16 %0, 0;\n\t@p ld.shared.b16 %0, [%1];\n\t}" : "=h"(v) : "r"(p), "r"((int)on) : "memory");
             return bk_cvt<DT>(v);
         }
     }

@@ -171,13 +171,14 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
                     const float2 hu2[2] = {f2(up[0].x, up[0].y), f2(up[1].x, up[1].y)}, au2[2] = {f2(up[0].z, up[0].w), f2(up[1].z, up[1].w)};
                     if (c + 2 < c2) load_up(c + 2);
                     else load_back(c);
+                    const bool on1 = c + 1 < nc;
                     int o[PW_R], o1[PW_R];
                     pw_offsets<ES, EL>(P, c, fh, fw, o, o1);
                     float xd[PW_R][2][2], xu[PW_R][2][2];   // row, channel, column
 #pragma unroll
                     for (int r = 0; r < PW_R; ++r)
 #pragma unroll
-                        for (int k = 0; k < 2; ++k) { vd.load(r, k, o[r], o1[r], fw, xd[r][k]); vu.load(r, k, o[r], o1[r], fw, xu[r][k]); }
+                        for (int k = 0; k < 2; ++k) { vd.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xd[r][k]); vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]); }
                     const uint32_t tt = tm + (c - c1) * 32;
 #pragma unroll
                     for (int cc = 0; cc < 2; ++cc) {
@@ -223,13 +224,9 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
                             const bool on = r0 + r < P.H && 2 * lane + k < nch;
                             xg[r][k][0] = __uint_as_float(bk_ldp<CS2D_F32>(src + fc, on)); xg[r][k][1] = __uint_as_float(bk_ldp<CS2D_F32>(src + (fw ? fc - 1 : fc + 1), on && on1));
                         } else {
-                            vg.load(r, k, o[r], o1[r], fw, xg[r][k]);
-                            if constexpr (EL) {   // what is not there: other elements that share words or rows with the block
-                                const bool on = r0 + r < P.H;
-                                xg[r][k][0] = on ? xg[r][k][0] : 0.f; xg[r][k][1] = on && on1 ? xg[r][k][1] : 0.f;
-                            }
+                            vg.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xg[r][k]);
                         }
-                        vu.load(r, k, o[r], o1[r], fw, xu[r][k]);
+                        vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]);
                     }
                 const uint32_t tt = tm + (c - c1) * 32;
                 float2 rv[2][4];

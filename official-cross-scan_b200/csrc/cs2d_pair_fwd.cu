@@ -94,13 +94,14 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
                     P.cola[o + r * 32] = al[r];
                 }
             }
+            const bool on1 = c + 1 < nc;
             int o[PW_R], o1[PW_R];
             pw_offsets<ES, EL>(P, c, fh, fw, o, o1);
             float xd[PW_R][2][2], xu[PW_R][2][2];   // row, channel, column
 #pragma unroll
             for (int r = 0; r < PW_R; ++r)
 #pragma unroll
-                for (int k = 0; k < 2; ++k) { vd.load(r, k, o[r], o1[r], fw, xd[r][k]); vu.load(r, k, o[r], o1[r], fw, xu[r][k]); }
+                for (int k = 0; k < 2; ++k) { vd.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xd[r][k]); vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]); }
             const float2 hu2[2] = {f2(up[0].x, up[0].y), f2(up[1].x, up[1].y)}, au2[2] = {f2(up[0].z, up[0].w), f2(up[1].z, up[1].w)};
             if (c + 2 < nc) fetch_up(c + 2);
             float2 y[PW_R][2];
@@ -123,7 +124,6 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
                 }
                 if (blk + 1 < P.nblk) row[(c + cc) * 32] = make_float4(hl[PW_R - 1].x, hl[PW_R - 1].y, al[PW_R - 1].x, al[PW_R - 1].y);
             }
-            const bool on1 = c + 1 < nc;
             if (DIRS && (P.mw || P.f32)) {   // straight to the fp32 results (merge: onto the image)
                 const int fc = fw ? P.W - 1 - c0 - c : c0 + c;
 #pragma unroll

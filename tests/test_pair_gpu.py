@@ -87,7 +87,7 @@ def test_fp32_results_of_16_bit_views(w):
 @pytest.mark.parametrize("shape,dtype", [((1, 4, 9, 1, 6, 20), torch.float32), ((2, 4, 66, 1, 7, 7), torch.bfloat16),
                                          ((1, 4, 12, 1, 10, 14), torch.float16), ((3, 4, 8, 1, 28, 56), torch.bfloat16),
                                          ((4, 4, 10, 1, 11, 100), torch.float32), ((1, 4, 10, 1, 6, 21), torch.bfloat16),
-                                         ((1, 4, 10, 1, 9, 7), torch.float32)])
+                                         ((1, 4, 10, 1, 9, 7), torch.float32), ((4, 4, 14, 1, 9, 9), torch.bfloat16)])
 def test_corner_directions_and_merge(shape, dtype):
     b, K, d, n, h, w = shape
     inp = make_inputs(*shape, dtype=dtype, seed=2)
