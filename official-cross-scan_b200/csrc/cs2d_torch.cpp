@@ -8,7 +8,10 @@
 // binding (src/cusoflex/selective_scan_oflex.cpp:179-440).
 //
 // Buffers of one backward: the parameter gradients (dA | dD | ddelta_bias | dA_decay) are one zero-filled
-// fp32 buffer; the fp32 sums behind 16-bit dB and dC are another one (one fill instead of two).
+// fp32 buffer; the fp32 sums behind 16-bit dB and dC are another one (one fill instead of two).  Small
+// problems take one allocation and one fill for all of these and the scratch (see BwdBuffers).  The backward
+// runs on a thread of the autograd engine that has just been woken: every call of the tensor library costs
+// twice there what it costs in a warm loop (measured 45 us for what takes 22 us on the calling thread).
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -120,12 +123,14 @@ void raise_on(int rc, const char *what) {
 }
 Tensor f32(const Tensor &like, int64_t n) { return at::empty({n}, like.options().dtype(at::kFloat)); }
 cudaStream_t stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
-Tensor zeros_f32(const Tensor &like, int64_t n) {   // zero-filled with one asynchronous memset
+void zero(const Tensor &t, int64_t n) {   // the first n floats, with one asynchronous memset
+    if (n <= 0) return;
+    const cudaError_t e = cudaMemsetAsync(t.data_ptr(), 0, (size_t)n * 4, stream_of(t));
+    CS2D_CHECK(e == cudaSuccess, "cs2d: zero fill failed: ", cudaGetErrorString(e));
+}
+Tensor zeros_f32(const Tensor &like, int64_t n) {
     Tensor t = f32(like, n);
-    if (n > 0) {
-        const cudaError_t e = cudaMemsetAsync(t.data_ptr(), 0, (size_t)n * 4, stream_of(like));
-        CS2D_CHECK(e == cudaSuccess, "cs2d: zero fill failed: ", cudaGetErrorString(e));
-    }
+    zero(t, n);
     return t;
 }
 float *fp(const Tensor &t) { return given(t) ? t.data_ptr<float>() : nullptr; }
@@ -157,27 +162,66 @@ ParamLayout param_layout(int64_t dim, int64_t n, bool has_D, bool has_bias, bool
 
 struct Grads { Tensor du, ddelta, dA, dB, dC, dD, dbias, ddecay, dw; };
 
-// dB and dC as the kernels accumulate them (fp32, zero-filled; 16-bit inputs: one buffer, one fill) and as
-// the caller gets them: two tensors of the input type that share no storage
-struct BCGrads {
-    Tensor b, c;
-    BCGrads(const Tensor &B) {
-        const int64_t n = B.numel();
+// A contiguous tensor on part of another one's storage (no view in autograd's eyes, a fifth of the cost of narrow + view)
+Tensor part_of(const Tensor &t, int64_t offset, at::IntArrayRef sizes) {
+    c10::Storage st = t.storage();
+    Tensor r = at::detail::make_tensor<c10::TensorImpl>(std::move(st), t.key_set(), t.dtype());
+    r.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    r.unsafeGetTensorImpl()->set_storage_offset(t.storage_offset() + offset);
+    return r;
+}
+
+// Device buffers of a backward: `nparam` floats of parameter gradients and the fp32 sums of dB and dC, zero-filled, and
+// the scratch.  Up to 256 KB in all they are one allocation with one fill, and 16-bit dB and dC are rounded together:
+// what a caller keeps then keeps no more than that alive.  Larger ones are buffers of their own: two tensors dB and dC
+// that share no storage.
+struct BwdBuffers {
+    Tensor params, b, c, scratch;
+    int64_t half = 0, off = -1;   // off: where dB starts in a shared buffer; dC follows `half` elements later
+    float *dB, *dC;
+    void *scratch_ptr;
+    BwdBuffers(const Tensor &B, int64_t nparam, size_t scratch_bytes, bool share) {
+        const int64_t n = B.numel(), head = (nparam + 7) & ~int64_t(7), ns = (int64_t)(scratch_bytes / 4);
+        half = (n + 7) & ~int64_t(7);
+        if (share && head + 2 * half + ns <= (1 << 16)) {
+            off = head;
+            params = f32(B, head + 2 * half + ns);
+            zero(params, head + 2 * half);
+            float *p = params.data_ptr<float>();
+            dB = p + off; dC = dB + half; scratch_ptr = dC + half;
+            return;
+        }
+        if (nparam > 0) params = zeros_f32(B, nparam);
         if (B.scalar_type() == at::kFloat) {
             b = zeros_f32(B, n); c = zeros_f32(B, n);
         } else {
-            const int64_t half = (n + 3) & ~int64_t(3);
             const Tensor flat = zeros_f32(B, 2 * half);
-            b = flat.narrow(0, 0, n); c = flat.narrow(0, half, n);
+            b = part_of(flat, 0, {n}); c = part_of(flat, half, {n});
+        }
+        dB = b.data_ptr<float>(); dC = c.data_ptr<float>();
+        scratch = f32(B, ns);
+        scratch_ptr = scratch.data_ptr();
+    }
+    void result(const Tensor &B, Tensor &gB, Tensor &gC) {
+        const auto ty = B.scalar_type();
+        if (off >= 0) {
+            const bool cast = ty != at::kFloat;
+            const Tensor t = cast ? part_of(params, off, {2 * half}).to(ty) : params;
+            gB = part_of(t, cast ? 0 : off, B.sizes());
+            gC = part_of(t, (cast ? 0 : off) + half, B.sizes());
+        } else {
+            gB = (ty == at::kFloat ? b : b.to(ty)).view(B.sizes());
+            gC = (ty == at::kFloat ? c : c.to(ty)).view(B.sizes());
         }
     }
-    float *dB() { return b.data_ptr<float>(); }
-    float *dC() { return c.data_ptr<float>(); }
-    void result(const Tensor &B, Tensor &gB, Tensor &gC) {
-        gB = (B.scalar_type() == at::kFloat ? b : b.to(B.scalar_type())).view(B.sizes());
-        gC = (B.scalar_type() == at::kFloat ? c : c.to(B.scalar_type())).view(B.sizes());
-    }
 };
+
+void param_views(Grads &g, const Tensor &flat, const ParamLayout &l, int64_t dim, int64_t n) {
+    g.dA = part_of(flat, 0, {dim, n});
+    if (l.dD >= 0) g.dD = part_of(flat, l.dD, {dim});
+    if (l.dbias >= 0) g.dbias = part_of(flat, l.dbias, {dim});
+    if (l.ddecay >= 0) g.ddecay = part_of(flat, l.ddecay, {1});
+}
 
 Grads scan_backward(const Args &a, const Tensor &dout, const Tensor &state, const OptT &param_grads, bool deterministic) {
     CS2D_CHECK(dout.is_cuda(), "dout must be a CUDA tensor");
@@ -197,30 +241,25 @@ Grads scan_backward(const Args &a, const Tensor &dout, const Tensor &state, cons
     Grads g;
     g.du = at::empty(a.u.sizes(), a.u.options());
     g.ddelta = at::empty(a.u.sizes(), a.u.options());
-    Tensor flat;
-    if (param_grads.has_value()) {
+    const bool own = !param_grads.has_value();   // (a caller that brings its own buffer - the dispatcher operators - wants no shared storage)
+    BwdBuffers buf(a.B, own ? l.total : 0, cs2d_bwd_scratch_bytes(&p), own);
+    Tensor flat = buf.params;
+    if (!own) {
         flat = *param_grads;
         CS2D_CHECK(flat.is_cuda() && flat.scalar_type() == at::kFloat && flat.is_contiguous() && flat.numel() == l.total,
                    "param_grads must be a flat float32 CUDA tensor of the layout size");
-    } else {
-        flat = zeros_f32(a.u, l.total);
     }
-    g.dA = flat.narrow(0, 0, dim * n).view({dim, n});
-    if (l.dD >= 0) g.dD = flat.narrow(0, l.dD, dim);
-    if (l.dbias >= 0) g.dbias = flat.narrow(0, l.dbias, dim);
-    if (l.ddecay >= 0) g.ddecay = flat.narrow(0, l.ddecay, 1);
-    BCGrads bc(a.B);
-    const Tensor scratch = f32(a.u, (int64_t)(cs2d_bwd_scratch_bytes(&p) / 4));
+    param_views(g, flat, l, dim, n);
     if (deterministic) {
         const size_t ndet = cs2d_bwd_det_scratch_bytes(&p);
         CS2D_CHECK(ndet != 0, "cs2d backward has no deterministic implementation for this shape: ", cs2d_last_error());
         const Tensor det = f32(a.u, (int64_t)(ndet / 4));
         raise_on(cs2d_bwd_det(&p, nullptr, dout.const_data_ptr(), dout.stride(0), dout.stride(1), dout.stride(2), state.const_data_ptr(),
-                              scratch.data_ptr(), det.data_ptr(), g.du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), bc.dB(), bc.dC(),
+                              buf.scratch_ptr, det.data_ptr(), g.du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), buf.dB, buf.dC,
                               fp(g.dD), fp(g.dbias), fp(g.ddecay), st), "backward");
     } else {
         raise_on(cs2d_bwd(&p, dout.const_data_ptr(), dout.stride(0), dout.stride(1), dout.stride(2), state.const_data_ptr(),
-                          scratch.data_ptr(), g.du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), bc.dB(), bc.dC(), fp(g.dD), fp(g.dbias),
+                          buf.scratch_ptr, g.du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), buf.dB, buf.dC, fp(g.dD), fp(g.dbias),
                           fp(g.ddecay), st), "backward");
     }
     if (p.delta_dim != dim) {
@@ -228,7 +267,7 @@ Grads scan_backward(const Args &a, const Tensor &dout, const Tensor &state, cons
         g.ddelta = g.ddelta.view({a.u.size(0), p.delta_dim, rep, a.u.size(2), a.u.size(3)}).sum(2);
         if (given(g.dbias)) g.dbias = g.dbias.view({p.delta_dim, rep}).sum(1);
     }
-    bc.result(a.B, g.dB, g.dC);
+    buf.result(a.B, g.dB, g.dC);
     return g;
 }
 
@@ -275,22 +314,17 @@ Grads cross_backward(const Args &a, const Tensor &w, const Tensor &dy, const Ten
     const ParamLayout l = param_layout(dim, n, given(a.D), given(a.bias), given(a.decay));
     const c10::cuda::CUDAGuard guard(a.u.device());
     Grads g;
-    Tensor flat = zeros_f32(a.u, l.total + dim);   // the parameter gradients, then dw
-    g.dw = flat.narrow(0, l.total, dim).view(w.sizes());
-    g.dA = flat.narrow(0, 0, dim * n).view({dim, n});
-    if (l.dD >= 0) g.dD = flat.narrow(0, l.dD, dim);
-    if (l.dbias >= 0) g.dbias = flat.narrow(0, l.dbias, dim);
-    if (l.ddecay >= 0) g.ddecay = flat.narrow(0, l.ddecay, 1);
+    BwdBuffers buf(a.B, l.total + dim, cs2d_bwd_scratch_bytes(&p), true);   // the parameter gradients, then dw
+    g.dw = part_of(buf.params, l.total, w.sizes());
+    param_views(g, buf.params, l, dim, n);
     Tensor du = merged_image(a.u, serial);
     g.ddelta = at::empty(a.delta.sizes(), a.delta.options());
-    BCGrads bc(a.B);
-    const Tensor scratch = f32(a.u, (int64_t)(cs2d_bwd_scratch_bytes(&p) / 4));
     const cs2d_dirs o = make_dirs(p.n_groups, 3, serial, wf, fp(g.dw));   // u and dy are shared by the directions
-    raise_on(cs2d_bwd_dir(&p, &o, dy.const_data_ptr(), dy.stride(0), dy.stride(1), dy.stride(2), state.const_data_ptr(), scratch.data_ptr(),
-                          du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), bc.dB(), bc.dC(), fp(g.dD), fp(g.dbias), fp(g.ddecay),
+    raise_on(cs2d_bwd_dir(&p, &o, dy.const_data_ptr(), dy.stride(0), dy.stride(1), dy.stride(2), state.const_data_ptr(), buf.scratch_ptr,
+                          du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), buf.dB, buf.dC, fp(g.dD), fp(g.dbias), fp(g.ddecay),
                           stream_of(a.u)), "backward");
     g.du = du.scalar_type() == a.u.scalar_type() ? du : du.to(a.u.scalar_type());
-    bc.result(a.B, g.dB, g.dC);
+    buf.result(a.B, g.dB, g.dC);
     if (g.dw.scalar_type() != w.scalar_type()) g.dw = g.dw.to(w.scalar_type());
     return g;
 }
