@@ -329,7 +329,7 @@ static size_t state_bytes(const cs2d_problem *p, bool backward, bool rolling) {
     Blk k;
     int NG;
     blk_fill(k, NG, p, nullptr, backward);
-    const size_t need = backward ? blk_row_bytes(k, true) : blk_row_bytes(k, rolling) + (rolling ? blk_bc_bytes(k, NG) : 3 * blk_bc_bytes(k, NG) + blk_col_bytes(k));
+    const size_t need = backward ? blk_row_bytes(k, true) : blk_row_bytes(k, rolling) + blk_bc_bytes(k, NG) + (rolling ? 0 : blk_col_bytes(k));
     return tile > need ? tile : need;
 }
 
@@ -407,8 +407,7 @@ static void blk_state(Blk &k, int NG, const void *saved, bool roll) {
     k.roll = roll;
     k.row = reinterpret_cast<float4 *>(q);
     k.bc = reinterpret_cast<float2 *>(q + blk_row_bytes(k, roll));
-    k.bc2 = reinterpret_cast<float4 *>(q + blk_row_bytes(k, roll) + blk_bc_bytes(k, NG));
-    k.col = reinterpret_cast<float4 *>(q + blk_row_bytes(k, roll) + 3 * blk_bc_bytes(k, NG));
+    k.col = reinterpret_cast<float4 *>(q + blk_row_bytes(k, roll) + blk_bc_bytes(k, NG));
 }
 static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o, bool backward) {
     k = Blk{};

@@ -50,8 +50,7 @@ struct Blk {
     //   row [nblk][nstrip][4][NL] float4 = h of the block's last row, two columns per float4 (rolling: nblk = 1)
     //   col [nblk][nstrip-1][4][NL] float4 = (q, s) of the column left of block strip+1, one row per float4
     float4 *row, *col;
-    float2 *bc;                             // B and C in walk order, and for a backward with every value twice (blk_bc_kernel)
-    float4 *bc2;
+    float2 *bc;                             // B and C in walk order (blk_bc_kernel)
     // backward
     float4 *adj;                            // [nstrip][4][NL]: the adjoint row m between rows of blocks
     void *du, *ddelta;

@@ -9,9 +9,7 @@ namespace cs2d {
 
 // B and C in the order the walk consumes them: [batch*G][nblk][nstrip][32 pixels, column by column][NG] (B, C), fp32, in
 // scan coordinates; pixels outside the image and states past dstate are zero.  One 16-byte asynchronous copy per lane then
-// fetches what two states of a pixel need, without address arithmetic or conversions in the walk.  For a backward, which
-// is short of registers and instructions rather than of shared-memory bandwidth, also with every value twice:
-// [32 pixels][(B, B, B', B'), (C, C, C', C')][8] of the states n and n + 8 (16 slots), [32][8] (B, B, C, C) (8 slots).
+// fetches what two states of a pixel need, without address arithmetic or conversions in the walk.
 template <int DT>
 __global__ void blk_bc_kernel(const __grid_constant__ Blk P, int NG) {
     using T = typename bk_type<DT>::t;
@@ -31,14 +29,6 @@ __global__ void blk_bc_kernel(const __grid_constant__ Blk P, int NG) {
         sm[n][px] = f2(bk_cvt<DT>(bv), bk_cvt<DT>(cv));
     }
     __syncthreads();
-    if (!P.roll) {
-        float4 *dst2 = P.bc2 + ((int64_t)bg * P.nblk * P.nstrip + tile) * BK_PX * NG;
-        for (int e = threadIdx.x; e < BK_PX * NG; e += blockDim.x) {
-            const int n = e & 7, i = e / NG, px = (i % BK_R) * BK_S + i / BK_R;
-            const float2 v = sm[n][px], v8 = NG == 16 ? sm[n + 8][px] : v;
-            dst2[e] = NG == 8 ? make_float4(v.x, v.x, v.y, v.y) : (e & 8) ? make_float4(v.y, v.y, v8.y, v8.y) : make_float4(v.x, v.x, v8.x, v8.x);
-        }
-    }
     for (int e = threadIdx.x; e < BK_PX * NG; e += blockDim.x) {   // write in walk order
         const int n = e % NG, i = e / NG;
         dst[e] = sm[NG == 16 ? (n >> 1) + (n & 1) * 8 : n][(i % BK_R) * BK_S + i / BK_R];   // (states n and n + 8 side by side)
