@@ -65,7 +65,7 @@ typedef struct {
 
 /*
  * Bytes of the saved-state buffer the forward writes and the backward reads:
- * row checkpoints of the state h; for problems with more than two states and
+ * row checkpoints of the state h; for problems with more than one state and
  * at least eight channels per group (the block-walk kernels) also h and the
  * row scan at every eighth column and B and C regrouped; for those with a single
  * state (the pair-walk kernels) the same with the transition in place of B and C.

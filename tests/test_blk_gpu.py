@@ -1,4 +1,4 @@
-"""The block-walk kernels (three or more states, at least eight channels per group) against the float64 oracle: images of
+"""The block-walk kernels (two or more states, at least eight channels per group) against the float64 oracle: images of
 one block and less, ragged in both directions, one to four row workers per CTA, odd channel counts (a slot with one live
 half), every number of state slots, delta shared by channels (the addresses of neighbouring channels coincide), fp32
 results of 16-bit inputs, rows that do and do not allow groups of four, state decay, and the deterministic
@@ -18,6 +18,7 @@ CASES = [
     ((1, 1, 8, 3, 1, 1), torch.float32, {}),           # a single pixel
     ((1, 2, 9, 16, 4, 8), torch.float32, {}),          # exactly one block; an odd number of channels
     ((2, 1, 8, 8, 5, 9), torch.float32, {}),           # one row and one column more than a block
+    ((2, 2, 13, 2, 6, 12), torch.bfloat16, {}),         # two states; half a block at the end of a row
     ((1, 1, 11, 9, 40, 7), torch.float32, {}),         # one block per row: the row of h stays in registers or waits for the workers
     ((3, 1, 10, 16, 9, 33), torch.bfloat16, {}),       # 5 blocks per row, two row workers with a short last pass
     ((1, 2, 12, 5, 27, 70), torch.float16, {}),        # 9 blocks per row, four row workers
