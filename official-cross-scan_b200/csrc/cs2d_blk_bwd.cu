@@ -50,8 +50,9 @@ struct BkBwd {   // a warp's shared memory
     static constexpr int total = (mw + SPW * 8 + 15) & ~15;
 };
 
-// EXTRA: the direction merge's dw, or dA_decay, is wanted.
-template <int NG, int DT, bool EXTRA>
+// EXTRA: the direction merge's dw, or dA_decay, is wanted.  HALF: the last block of a row has its left half only, whose right
+// half is left out (a 28-wide map: an eighth of the work; kept out of the other instances, which have no register to spare).
+template <int NG, int DT, bool EXTRA, bool HALF>
 __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel(const __grid_constant__ Blk P) {
     using S = BkBwd<NG>;
     using T = typename bk_type<DT>::t;
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
         const int ch0 = pos.slot * 2, cg = G0 * P.dpg + ch0, nch = P.dpg - ch0, b = pos.bg / P.G;
         const bool fh = (P.flip_h >> G0) & 1u, fw = (P.flip_w >> G0) & 1u;
         const bool mine = pos.slot + sl_ < P.nsl;
+        const int nhalf = !HALF || c0 + 4 < P.W ? 2 : 1;   // halves of the block that the image has
         if (pos.pass == 0 && pos.strip == 0) {   // a new item
             const int k0 = min(2 * sl_, nch - 1), k1 = min(2 * sl_ + 1, nch - 1);
             const float *a = P.A + (int64_t)cg * P.A_ds + n * P.A_ns;
@@ -288,9 +290,9 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
 #pragma unroll
             for (int i = 0; i < 2; ++i) { rin[i] = tIn[i * BK_S]; rb[i] = tBC[i * NG]; }
 #pragma unroll 1
-            for (int k = 0; k < 2; ++k) {
+            for (int k = 0; k < nhalf; ++k) {
                 const float2 up[4] = {f2(rowv[0].x, rowv[0].y), f2(rowv[0].z, rowv[0].w), f2(rowv[1].x, rowv[1].y), f2(rowv[1].z, rowv[1].w)};
-                fetch_row(1);
+                if (nhalf == 2) fetch_row(1);
                 const float4 *kIn = tIn + 4 * k;
                 const float2 *kBC = tBC + 16 * k * NG;
                 const uint32_t tk = tm + 64 * k;
@@ -324,7 +326,8 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
             adjv[0] = bk_ld16<false>(arow + 2 * k * P.NL, there);
             adjv[1] = bk_ld16<false>(arow + (2 * k + 1) * P.NL, there);
         };
-        fetch_adj(1);
+        fetch_adj(nhalf - 1);
+        if (non && nhalf == 1) copy_bc(nxt, 1);
         const float2 *tG = reinterpret_cast<const float2 *>(sm + S::g) + sl_ * NP;
         float2 dAt = bc(0.f);
         const int64_t HW = (int64_t)P.H * P.W;
@@ -339,9 +342,9 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
             rg[o] = tG[r * BK_S + 4 * k + cc];
             tm_ld(tm + 64 * k + 4 * j, rhq[o]);
         };
-        load(1, 15);
+        load(nhalf - 1, 15);
 #pragma unroll 1
-        for (int k = 1; k >= 0; --k) {
+        for (int k = nhalf - 1; k >= 0; --k) {
             const float2 up[4] = {f2(rowv[0].x, rowv[0].y), f2(rowv[0].z, rowv[0].w), f2(rowv[1].x, rowv[1].y), f2(rowv[1].z, rowv[1].w)};
             const float2 dn[4] = {f2(adjv[0].x, adjv[0].y), f2(adjv[0].z, adjv[0].w), f2(adjv[1].x, adjv[1].y), f2(adjv[1].z, adjv[1].w)};
             if (k) { fetch_row(0); fetch_adj(0); }
@@ -451,8 +454,8 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
                 const float2 u2 = f2(us.x, us.y), S1 = f2(S.x, S.y);
                 const float2 du = fma2(f2(par.z, par.w), gv, mul2(f2(in.x, in.y), S1));
                 const float2 dd = mul2(fma2(u2, S1, mul2(f2(S.z, S.w), bc(0.6931471805599453f))), f2(us.z, us.w));
-                accD[s] = fma2(gr, u2, accD[s]); accB[s] = add2(accB[s], dd);
                 const bool k0 = pix && 2 * s < nch, k1 = pix && 2 * s + 1 < nch;
+                accD[s] = fma2(gr, u2, accD[s]); accB[s] = add2(accB[s], HALF ? f2(pix ? dd.x : 0.f, pix ? dd.y : 0.f) : dd);   // (no sums where a half was left out)
                 const int64_t ch = (int64_t)(2 * s) * HW;
                 if (P.mw) {
                     bk_st<CS2D_F32, true>(P.du, odu + ch, du.x, k0);
@@ -517,9 +520,9 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(128));
 }
 
-template <int NG, int DT, bool EXTRA>
+template <int NG, int DT, bool EXTRA, bool HALF>
 static cudaError_t launch(const Blk &P, cudaStream_t st) {
-    auto kernel = blk_bwd_kernel<NG, DT, EXTRA>;
+    auto kernel = blk_bwd_kernel<NG, DT, EXTRA, HALF>;
     constexpr int smem = BkBwd<NG>::total * BK_WARPS;
     static bool attr_done[64] = {};
     int dev = 0;
@@ -534,7 +537,9 @@ static cudaError_t launch(const Blk &P, cudaStream_t st) {
 }
 template <int NG, int DT>
 static cudaError_t launch_ex(const Blk &P, cudaStream_t st) {
-    return P.mw || P.ddecay ? launch<NG, DT, true>(P, st) : launch<NG, DT, false>(P, st);
+    const bool half = ((P.W - 1) & 7) < 4;   // columns in the last block: at most 4
+    if (P.mw || P.ddecay) return half ? launch<NG, DT, true, true>(P, st) : launch<NG, DT, true, false>(P, st);
+    return half ? launch<NG, DT, false, true>(P, st) : launch<NG, DT, false, false>(P, st);
 }
 template <int NG>
 static cudaError_t launch_dt(const Blk &P, cudaStream_t st) {

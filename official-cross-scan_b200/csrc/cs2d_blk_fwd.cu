@@ -47,7 +47,8 @@ struct BkFwd {   // a warp's shared memory
     static constexpr int total = (top + SPW * 9 * 8 + 15) & ~15;
 };
 
-template <int NG, int DT, bool KEEP>
+// HALF: the last block of a row has its left half only, whose right half is left out
+template <int NG, int DT, bool KEEP, bool HALF>
 __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_constant__ Blk P) {
     using S = BkFwd<NG>;
     using T = typename bk_type<DT>::t;
@@ -230,13 +231,15 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
         const float2 *tTop = sTop + sl_ * 9;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
+            const bool there = !HALF || k == 0 || pos.strip * BK_S + 4 < P.W;   // the image has this half of the block
             float2 hb[4];
+            if constexpr (HALF) hb[0] = hb[1] = hb[2] = hb[3] = bc(0.f);
 #pragma unroll
             for (int qt = 2 * k; qt < 2 * k + 2; ++qt) {
                 bk_wait<2>();
                 __syncwarp();   // this quarter's B and C are here, the quarter before it has been read by all lanes
                 copy_bc(qt == 0 ? tbc : nbc, (qt + 3) & 3, qt == 0 || non);
-                {
+                if (there) {
                     const float2 *tBC = sBC + qt * 8 * NG + (NG == 16 ? (n & 7) * 2 + (n >> 3) : n);
                     float4 rin[2];
                     float2 rbc[2];
@@ -263,7 +266,7 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
                     }
                 }
             }
-            if (blk + 1 < P.nblk) {   // the block's last row of h
+            if (blk + 1 < P.nblk && there) {   // the block's last row of h
                 bk_st16(trow + 2 * k * P.NL, make_float4(hb[0].x, hb[0].y, hb[1].x, hb[1].y), mine);
                 bk_st16(trow + (2 * k + 1) * P.NL, make_float4(hb[2].x, hb[2].y, hb[3].x, hb[3].y), mine);
             }
@@ -276,7 +279,7 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
                 fetch(nxt, k);
             }
             __syncwarp();
-            {   // sums over the states of half a block: a lane takes one pixel of every second slot
+            if (there) {   // sums over the states of half a block: a lane takes one pixel of every second slot
                 const bool fw = (P.flip_w >> G0) & 1u;
                 const int px = lane & 15, c0 = pos.strip * BK_S + k * 4, nch = P.dpg - pos.slot * 2 - 2 * (lane >> 4);
                 const bool okp = blk * BK_R + (px >> 2) < P.H && c0 + (px & 3) < P.W;
@@ -315,9 +318,9 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
     bk_wait<0>();
 }
 
-template <int NG, int DT, bool KEEP>
+template <int NG, int DT, bool KEEP, bool HALF>
 static cudaError_t launch(const Blk &P, cudaStream_t st) {
-    auto kernel = blk_fwd_kernel<NG, DT, KEEP>;
+    auto kernel = blk_fwd_kernel<NG, DT, KEEP, HALF>;
     constexpr int smem = BkFwd<NG>::total * BK_WARPS;
     static bool attr_done[64] = {};
     int dev = 0;
@@ -331,12 +334,18 @@ static cudaError_t launch(const Blk &P, cudaStream_t st) {
     kernel<<<P.grid, BK_WARPS * 32, smem, st>>>(P);
     return cudaGetLastError();
 }
+template <int NG, int DT>
+static cudaError_t launch_half(const Blk &P, cudaStream_t st) {
+    const bool half = ((P.W - 1) & 7) < 4;   // columns in the last block: at most 4
+    if (P.roll) return half ? launch<NG, DT, false, true>(P, st) : launch<NG, DT, false, false>(P, st);
+    return half ? launch<NG, DT, true, true>(P, st) : launch<NG, DT, true, false>(P, st);
+}
 template <int NG>
 static cudaError_t launch_dt(const Blk &P, cudaStream_t st) {
     switch (P.io_dt) {
-        case CS2D_F32: return P.roll ? launch<NG, CS2D_F32, false>(P, st) : launch<NG, CS2D_F32, true>(P, st);
-        case CS2D_F16: return P.roll ? launch<NG, CS2D_F16, false>(P, st) : launch<NG, CS2D_F16, true>(P, st);
-        default: return P.roll ? launch<NG, CS2D_BF16, false>(P, st) : launch<NG, CS2D_BF16, true>(P, st);
+        case CS2D_F32: return launch_half<NG, CS2D_F32>(P, st);
+        case CS2D_F16: return launch_half<NG, CS2D_F16>(P, st);
+        default: return launch_half<NG, CS2D_BF16>(P, st);
     }
 }
 
