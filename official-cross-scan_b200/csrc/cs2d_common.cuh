@@ -138,6 +138,14 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 __device__ __forceinline__ float2 ex2_2(float2 x) { return make_float2(ex2(x.x), ex2(x.y)); }
+// log(1 + t) / t for t in [0, 1]: the polynomial of least relative error of degree 8 (3e-8; fitted by iteratively
+// reweighted least squares), 1.6e-7 when evaluated in fp32.
+__device__ __forceinline__ float2 log1p_over(float2 t) {
+    float2 q = fma2(t, bc(0.00523269462f), bc(-0.0295052433f));
+    q = fma2(q, t, bc(0.0782259651f)); q = fma2(q, t, bc(-0.136632475f)); q = fma2(q, t, bc(0.19106008f));
+    q = fma2(q, t, bc(-0.248429827f)); q = fma2(q, t, bc(0.333190969f)); q = fma2(q, t, bc(-0.499994931f));
+    return fma2(q, t, bc(0.99999997f));
+}
 
 template <int WIDTH>
 __device__ __forceinline__ float2 shfl_up2(float2 v, int off) {

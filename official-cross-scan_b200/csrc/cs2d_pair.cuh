@@ -270,14 +270,6 @@ template <int DT> struct PwBC {
     }
 };
 
-// log(1 + t) / t for t in [0, 1]: the polynomial of least relative error of degree 8 (3e-8; fitted by iteratively
-// reweighted least squares), 1.6e-7 when evaluated in fp32.
-__device__ __forceinline__ float2 pw_log1p_over(float2 t) {
-    float2 q = fma2(t, bc(0.00523269462f), bc(-0.0295052433f));
-    q = fma2(q, t, bc(0.0782259651f)); q = fma2(q, t, bc(-0.136632475f)); q = fma2(q, t, bc(0.19106008f));
-    q = fma2(q, t, bc(-0.248429827f)); q = fma2(q, t, bc(0.333190969f)); q = fma2(q, t, bc(-0.499994931f));
-    return fma2(q, t, bc(0.99999997f));
-}
 // softplus, and (SIG) its derivative
 template <bool SIG>
 __device__ __forceinline__ float2 pw_softplus2(float2 x, float2 *sig) {
@@ -286,7 +278,7 @@ __device__ __forceinline__ float2 pw_softplus2(float2 x, float2 *sig) {
         const float2 e = add2(t, bc(1.f)), r = f2(rcp(e.x), rcp(e.y)), tr = mul2(t, r);
         *sig = f2(x.x >= 0.f ? r.x : tr.x, x.y >= 0.f ? r.y : tr.y);
     }
-    return fma2(pw_log1p_over(t), t, f2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+    return fma2(log1p_over(t), t, f2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
 }
 
 // Writes the scan columns c, c + 1 of a row of fp32 results (image column fc, and the one on its right, or left when rev), or adds them

@@ -265,8 +265,10 @@ __device__ __forceinline__ float rcp(float x) {
 // threshold: above 20 the result is x itself (fwd kernel :221-224, bwd kernel :785-806).  softplus(x) >
 // x always and log(1 + e^20) < 20 + 1e-8, so max(log(1 + e^min(x,20)), x) is that rule without a
 // select, and e^20 / (1 + e^20) rounds to 1.  16-bit I/O (FAST) evaluates exp and log with the
-// special-function unit directly (absolute error ~1e-7, far inside the 16-bit tolerance); fp32 I/O
-// keeps log1pf.
+// special-function unit directly (absolute error ~1e-7, far inside the 16-bit tolerance).  fp32 I/O takes
+// max(x, 0) + log(1 + e^-|x|), about 2e-7 relative everywhere, two values at a time (log1pf was a third of the
+// kernels' time: 100x100 training step of 8x768 channels 1899 -> 1275 us); above 20 the logarithm is below half a unit
+// in the last place.
 template <bool FAST, bool WITH_SIG>
 __device__ __forceinline__ void softplus2(float2 x, float2 &dl, float2 &sig) {
     const float2 xc = f2(fminf(x.x, 20.f), fminf(x.y, 20.f));
@@ -277,9 +279,12 @@ __device__ __forceinline__ void softplus2(float2 x, float2 &dl, float2 &sig) {
         l = mul2(f2(lg2(u.x), lg2(u.y)), bc(LN2));
         if (WITH_SIG) sig = mul2(t, f2(rcp(u.x), rcp(u.y)));
     } else {
-        t = f2(__expf(xc.x), __expf(xc.y));
-        l = f2(log1pf(t.x), log1pf(t.y));
-        if (WITH_SIG) sig = f2(__fdividef(t.x, 1.f + t.x), __fdividef(t.y, 1.f + t.y));
+        t = f2(ex2(-fabsf(x.x) * LOG2E), ex2(-fabsf(x.y) * LOG2E));
+        l = fma2(log1p_over(t), t, f2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+        if (WITH_SIG) {
+            const float2 u = add2(t, bc(1.f)), r = f2(rcp(u.x), rcp(u.y)), tr = mul2(t, r);
+            sig = f2(x.x >= 0.f ? r.x : tr.x, x.y >= 0.f ? r.y : tr.y);
+        }
     }
     dl = f2(fmaxf(l.x, x.x), fmaxf(l.y, x.y));
 }
