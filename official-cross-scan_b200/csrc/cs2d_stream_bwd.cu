@@ -82,9 +82,14 @@ __device__ __forceinline__ void add_dbc_rows(float (&v)[16], float *rowB, float 
     }
 }
 
-// Thread-private rows parked in shared memory: row `k` of thread `tid` is four float4 (8 float2) at
-// [(k*4 + q) * STHREADS + tid], so that a warp's accesses are consecutive 16-byte words.
+// Thread-private rows.  16-bit inputs park them in shared memory: row `k` of thread `tid` is four float4 (8 float2) at
+// [(k*4 + q) * STHREADS + tid], so that a warp's accesses are consecutive 16-byte words.  fp32 inputs, whose staging takes
+// 98 KB, park them in TENSOR MEMORY, 16 columns of the thread's lane per row: with 57 KB of parked rows beside it a second
+// CTA per SM did not fit (8x768x56x56 training step 563 -> 484 us, 64x1536x20x20 803 -> 698; 16-bit 128x768x56x56 2329 ->
+// 2391, so those stay).
 constexpr int SB_ROWS = SRB + 3;   // h above the block, h of the block's rows, adjoint row m, its a
+constexpr int SB_COLS = 128;       // tensor memory columns of a CTA: a power of two that holds the rows
+static_assert(SB_ROWS * 16 <= SB_COLS, "the parked rows fit");
 constexpr int SB_PARK = SB_ROWS * 4 * STHREADS * 16;
 // Staging ring: every row the thread is going to need - the row above a block (delta and the h
 // checkpoint), the block's rows for the recompute (u, delta, B), the same rows bottom-up for the
@@ -96,7 +101,7 @@ constexpr int BW_DEPTH = 3;
 template <int DT, int GT>
 __host__ __device__ constexpr int bw_slot_words() { return 6 * slot_words<DT>() + 2 * slot_words<GT>(); }
 template <int DT, int GT>
-__host__ __device__ constexpr int bw_smem() { return SB_PARK + BW_DEPTH * bw_slot_words<DT, GT>() * STHREADS * 16; }
+__host__ __device__ constexpr int bw_smem() { return (DT == CS2D_F32 ? 0 : SB_PARK) + BW_DEPTH * bw_slot_words<DT, GT>() * STHREADS * 16; }
 __device__ __forceinline__ void park(float4 *sm, int k, const float2 (&v)[STRIP]) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) sm[(k * 4 + q) * STHREADS] = make_float4(v[2 * q].x, v[2 * q].y, v[2 * q + 1].x, v[2 * q + 1].y);
@@ -108,21 +113,55 @@ __device__ __forceinline__ void fetch(const float4 *sm, int k, float2 (&v)[STRIP
         v[2 * q] = f2(t.x, t.y); v[2 * q + 1] = f2(t.z, t.w);
     }
 }
+__device__ __forceinline__ void park(uint32_t tm, int k, const float2 (&v)[STRIP]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(tm + 16 * k),
+                 "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y),
+                 "f"(v[4].x), "f"(v[4].y), "f"(v[5].x), "f"(v[5].y), "f"(v[6].x), "f"(v[6].y), "f"(v[7].x), "f"(v[7].y) : "memory");
+}
+// fetch asks for a row; fetched: it is there (the values pass through the wait, so that nothing uses them before it)
+__device__ __forceinline__ void fetch(uint32_t tm, int k, float2 (&v)[STRIP]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y), "=f"(v[3].x), "=f"(v[3].y),
+                   "=f"(v[4].x), "=f"(v[4].y), "=f"(v[5].x), "=f"(v[5].y), "=f"(v[6].x), "=f"(v[6].y), "=f"(v[7].x), "=f"(v[7].y) : "r"(tm + 16 * k) : "memory");
+}
+__device__ __forceinline__ void fetched(float2 (&v)[STRIP]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[1].x), "+f"(v[1].y), "+f"(v[2].x), "+f"(v[2].y), "+f"(v[3].x), "+f"(v[3].y),
+                   "+f"(v[4].x), "+f"(v[4].y), "+f"(v[5].x), "+f"(v[5].y), "+f"(v[6].x), "+f"(v[6].y), "+f"(v[7].x), "+f"(v[7].y)::"memory");
+}
+__device__ __forceinline__ void parked() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // DT: type of u, delta, B, C, du, ddelta; G32: dout is fp32 (always with fp32 inputs; with 16-bit
 // inputs when the forward returned fp32).
 template <int L, int DT, bool G32>
-__global__ void __launch_bounds__(STHREADS, DT == CS2D_F32 ? 1 : 2) sbwd_kernel(const Dev P) {
+__global__ void __launch_bounds__(STHREADS, 2) sbwd_kernel(const Dev P) {
     static_assert(G32 || DT != CS2D_F32, "fp32 inputs come with an fp32 dout");
     extern __shared__ __align__(16) float4 sm_all[];
-    float4 *sm = sm_all + threadIdx.x;
+    constexpr bool TM = DT == CS2D_F32;
+    __shared__ uint32_t tm_base;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    if (TM && warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tm_base)), "r"(SB_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    auto place = [&]() {   // where this thread parks its rows
+        if constexpr (TM) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncthreads();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            return __shfl_sync(0xffffffffu, tm_base, 0) + ((uint32_t)warp << 21);   // this warp's lane quadrant
+        } else {
+            return sm_all + threadIdx.x;
+        }
+    };
+    const auto tm = place();
     constexpr int K_TOP = 0, K_ROW = 1, K_M = SRB + 1, K_A = SRB + 2;
     constexpr int GT = G32 ? CS2D_F32 : DT;
     constexpr int SW = slot_words<DT>(), GW = slot_words<GT>(), SLOTW = bw_slot_words<DT, GT>();
     constexpr int O_U0 = 0, O_U1 = SW, O_X0 = 2 * SW, O_X1 = 3 * SW, O_B = 4 * SW, O_C = 5 * SW, O_G0 = 6 * SW,
                   O_G1 = 6 * SW + GW, O_CK = 4 * SW;
     static_assert(O_CK + 4 <= SLOTW, "the checkpoint row fits behind the two delta strips");
-    uint4 *ring = reinterpret_cast<uint4 *>(sm_all + SB_ROWS * 4 * STHREADS) + threadIdx.x;
+    uint4 *ring = reinterpret_cast<uint4 *>(sm_all + (TM ? 0 : SB_ROWS * 4 * STHREADS)) + threadIdx.x;
     constexpr bool FAST = DT != CS2D_F32;
     const Who<L> w(P);
     constexpr int Wp = Who<L>::Wp;
@@ -153,7 +192,7 @@ __global__ void __launch_bounds__(STHREADS, DT == CS2D_F32 ? 1 : 2) sbwd_kernel(
         float2 z[STRIP];
 #pragma unroll
         for (int i = 0; i < STRIP; ++i) z[i] = bc(0.f);
-        park(sm, K_M, z); park(sm, K_A, z);   // below the image: no adjoint
+        park(tm, K_M, z); park(tm, K_A, z);   // below the image: no adjoint
     }
     float2 dA2 = bc(0.f), dD2 = bc(0.f), db2 = bc(0.f);
 
@@ -240,7 +279,7 @@ __global__ void __launch_bounds__(STHREADS, DT == CS2D_F32 ? 1 : 2) sbwd_kernel(
 #pragma unroll
                 for (int i = 0; i < STRIP; ++i) a_up[i] = ex2_2(mul2(dl[i], A2));
             }
-            park(sm, K_TOP, hprev);
+            park(tm, K_TOP, hprev);
             // ---- recompute h of the block's rows ----
             for (int rr = 0; rr < nr; ++rr) {   // not unrolled: the rows live in shared memory, the code stays small
                 float u0[STRIP], u1[STRIP], Bf[STRIP];
@@ -261,7 +300,7 @@ __global__ void __launch_bounds__(STHREADS, DT == CS2D_F32 ? 1 : 2) sbwd_kernel(
                     p[i] = mul2(bc(Bf[i]), mul2(dl[i], f2(u0[i], u1[i])));
                 }
                 srow_fwd<L, false>(j, a, p, hprev, a_up, h, sdummy);
-                park(sm, K_ROW + rr, h);
+                park(tm, K_ROW + rr, h);
 #pragma unroll
                 for (int i = 0; i < STRIP; ++i) { a_up[i] = a[i]; hprev[i] = h[i]; }
             }
@@ -299,7 +338,9 @@ __global__ void __launch_bounds__(STHREADS, DT == CS2D_F32 ? 1 : 2) sbwd_kernel(
             float2 a_r7 = bc(0.f);  // next lane's first column
             {
                 float2 m_dn[STRIP], a_dn[STRIP], bt[STRIP], mdr7 = bc(0.f);
-                fetch(sm, K_M, m_dn); fetch(sm, K_A, a_dn);
+                if constexpr (TM) parked();
+                fetch(tm, K_M, m_dn); fetch(tm, K_A, a_dn);
+                if constexpr (TM) { fetched(m_dn); fetched(a_dn); }
                 if constexpr (L > 1) {
                     a_r7 = shfl_down2<L>(a[0], 1);
                     mdr7 = shfl_down2<L>(m_dn[0], 1);
@@ -346,7 +387,8 @@ __global__ void __launch_bounds__(STHREADS, DT == CS2D_F32 ? 1 : 2) sbwd_kernel(
             float2 m[STRIP], m_dn[STRIP], hrow[STRIP], hup[STRIP];
 #pragma unroll
             for (int i = 0; i < STRIP; ++i) m[i] = mul2(a[i], dh[i]);
-            fetch(sm, K_M, m_dn); fetch(sm, K_ROW + rr, hrow); fetch(sm, K_ROW + rr - 1, hup);   // K_ROW - 1 == K_TOP
+            fetch(tm, K_M, m_dn); fetch(tm, K_ROW + rr, hrow); fetch(tm, K_ROW + rr - 1, hup);   // K_ROW - 1 == K_TOP
+            if constexpr (TM) { fetched(m_dn); fetched(hrow); fetched(hup); }
             float2 m_r7 = bc(0.f), h_l0 = bc(0.f);
             if constexpr (L > 1) {
                 m_r7 = shfl_down2<L>(m[0], 1);
@@ -354,7 +396,7 @@ __global__ void __launch_bounds__(STHREADS, DT == CS2D_F32 ? 1 : 2) sbwd_kernel(
                 m_r7.x = j == L - 1 ? 0.f : m_r7.x; m_r7.y = j == L - 1 ? 0.f : m_r7.y;
                 h_l0.x = j == 0 ? 0.f : h_l0.x; h_l0.y = j == 0 ? 0.f : h_l0.y;
             }
-            park(sm, K_M, m); park(sm, K_A, a);   // the adjoint row for the row above
+            park(tm, K_M, m); park(tm, K_A, a);   // the adjoint row for the row above
             float v[16], du0[STRIP], du1[STRIP], dd0[STRIP], dd1[STRIP];
 #pragma unroll
             for (int i = 0; i < STRIP; ++i) {
@@ -410,6 +452,12 @@ __global__ void __launch_bounds__(STHREADS, DT == CS2D_F32 ? 1 : 2) sbwd_kernel(
             if (P.dD) atomicAdd(P.dD + w.d1, dD2.y);
             if (P.dbias) atomicAdd(P.dbias + w.d1, db2.y);
         }
+    }
+    if constexpr (TM) {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(SB_COLS));
     }
 }
 
