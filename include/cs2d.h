@@ -79,7 +79,8 @@ size_t cs2d_saved_bytes(const cs2d_problem *p);
 
 /*
  * Bytes of the scratch buffer the backward needs (one adjoint row per channel
- * and state pair, carried between row blocks).  Contents are undefined before
+ * and state pair, carried between row blocks, or one per warp that is on the GPU
+ * at a time, whichever is more).  Contents are undefined before
  * and after a call.  The reference keeps the equivalent state in the x / x_sd
  * tensors it overwrites (selective_scan_bwd_kernel_oflex.cuh:490,726).
  * Returns 0 for an invalid or unsupported problem.
@@ -199,7 +200,8 @@ int cs2d_bwd_det(const cs2d_problem *p, const cs2d_dirs *dirs, const void *dout,
  * cs2d_fwd / cs2d_fwd_dir (dirs may be NULL), but instead of the saved-state
  * buffer it takes a scratch buffer of cs2d_fwd_only_scratch_bytes(p) bytes
  * (16-byte aligned, contents undefined before and after): one rolling row of h
- * per channel and state pair instead of one per four image rows.  The reference
+ * per channel and state pair (or per warp that is on the GPU at a time) instead
+ * of one per four image rows.  The reference
  * always writes its three side tensors (selective_scan_oflex.cpp:251-258,
  * selective_scan_fwd_kernel_oflex.cuh:289-295); it has no such mode.
  */
@@ -217,8 +219,10 @@ int cs2d_fwd_only(const cs2d_problem *p, const cs2d_dirs *dirs, void *out, int64
  * This entry point has no counterpart in the reference (whose host binding
  * allocates with torch).
  *   - inputs, saved state and ALL outputs are still passed by the caller;
- *   - problems whose cs2d_bwd_scratch_bytes() exceeds CS2D_NOALLOC_SCRATCH_BYTES
- *     are rejected with CS2D_ERR_UNSUPPORTED and a message (split the batch);
+ *   - problems whose adjoint rows (8 bytes per channel, state pair - a power of two
+ *     of them - and column, a row of up to 256 columns counting as 8, 16, 32 .. 256)
+ *     exceed CS2D_NOALLOC_SCRATCH_BYTES are rejected with CS2D_ERR_UNSUPPORTED and a
+ *     message (split the batch); kernels that keep rows per warp run fewer of them;
  *   - the first call on a device looks up the array's device address (a host
  *     call, no allocation); make that first call before starting a stream capture;
  *   - nothing needs clearing between calls, but the array is shared: calls that

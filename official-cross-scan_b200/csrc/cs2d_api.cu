@@ -274,7 +274,8 @@ static int tile_view(const cs2d_problem *p, int t, bool backward, bool bulk_ok, 
 static bool walk_shape(const cs2d_problem *p) { return p->dstate > 8 && p->ncols <= 8 * STRIP; }
 
 static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o, bool backward);
-static size_t blk_row_bytes(const Blk &k, bool roll);
+static size_t blk_row_bytes(const Blk &k);
+static size_t blk_team_bytes(const Blk &k, bool backward, int NG);
 static size_t blk_col_bytes(const Blk &k);
 static size_t blk_bc_bytes(const Blk &k, int NG);
 
@@ -284,7 +285,8 @@ static bool blk_shape(const cs2d_problem *p) { return p->dstate > 1 && p->dim / 
 
 static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool backward, const void *img = nullptr, int64_t img_bs = 0,
                       int64_t img_ds = 0, int64_t img_hs = 0);
-static size_t pair_row_bytes(const Pw &k, bool roll);
+static size_t pair_row_bytes(const Pw &k);
+static size_t pair_team_bytes(const Pw &k, bool backward);
 static size_t pair_col_bytes(const Pw &k);
 
 // (a warp of the pair-walk kernels works on 64 channels: too few of them and it is idle)
@@ -324,14 +326,14 @@ static size_t state_bytes(const cs2d_problem *p, bool backward, bool rolling) {
     if (pair_shape(p)) {
         Pw k;
         pair_fill(k, p, nullptr, backward);
-        const size_t need = backward || rolling ? pair_row_bytes(k, true) : pair_row_bytes(k, false) + pair_col_bytes(k);
+        const size_t need = backward || rolling ? pair_team_bytes(k, backward) : pair_row_bytes(k) + pair_col_bytes(k);
         return tile > need ? tile : need;
     }
     if (!blk_shape(p)) return tile;
     Blk k;
     int NG;
     blk_fill(k, NG, p, nullptr, backward);
-    const size_t need = backward ? blk_row_bytes(k, true) : blk_row_bytes(k, rolling) + blk_bc_bytes(k, NG) + (rolling ? 0 : blk_col_bytes(k));
+    const size_t need = backward ? blk_team_bytes(k, true, NG) : blk_bc_bytes(k, NG) + (rolling ? blk_team_bytes(k, false, NG) : blk_row_bytes(k) + blk_col_bytes(k));
     return tile > need ? tile : need;
 }
 
@@ -407,10 +409,12 @@ static bool blk_ok(const cs2d_problem *p, const cs2d_dirs *o) { return blk_shape
 static void blk_state(Blk &k, int NG, const void *saved, bool roll) {
     char *q = const_cast<char *>(static_cast<const char *>(saved));
     k.roll = roll;
+    k.bc = reinterpret_cast<float2 *>(q);
+    q += blk_bc_bytes(k, NG);
     k.row = reinterpret_cast<float4 *>(q);
-    k.bc = reinterpret_cast<float2 *>(q + blk_row_bytes(k, roll));
-    k.col = reinterpret_cast<float4 *>(q + blk_row_bytes(k, roll) + blk_bc_bytes(k, NG));
+    k.col = reinterpret_cast<float4 *>(q + blk_row_bytes(k));
 }
+static int blk_ctas(bool backward, int NG) { return !backward ? 4 : NG == 16 ? 3 : 2; }   // CTAs per SM
 static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o, bool backward) {
     k = Blk{};
     k.H = p->nrows; k.W = p->ncols; k.N = p->dstate; k.G = p->n_groups; k.dpg = p->dim / p->n_groups;
@@ -431,7 +435,7 @@ static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o,
     while (NG < p->dstate) NG <<= 1;
     k.nsl = (k.dpg + 1) / 2;
     k.NL = (int64_t)p->batch * k.G * k.nsl * NG;
-    const int spw = 32 / NG, ctas = !backward ? 4 : NG == 16 ? 3 : 2;   // slots per warp, CTAs per SM
+    const int spw = 32 / NG, ctas = blk_ctas(backward, NG);   // slots per warp, CTAs per SM
     k.ntile = (k.nsl + spw - 1) / spw; k.items = p->batch * k.G * k.ntile;
     // Row workers: as few as fill the GPU; with short rows a worker waits for the others at the end of a row
     const int64_t slots = (int64_t)kSMs * ctas * BK_WARPS;
@@ -449,7 +453,13 @@ static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o,
     const int64_t cap = ctas * kSMs;   // CTAs that fit at once
     k.grid = (int)(need < cap ? need : cap);
 }
-static size_t blk_row_bytes(const Blk &k, bool roll) { return (size_t)(roll ? 1 : k.nblk) * k.nstrip * 4 * k.NL * sizeof(float4); }
+static size_t blk_row_bytes(const Blk &k) { return (size_t)k.nblk * k.nstrip * 4 * k.NL * sizeof(float4); }
+// One row (the forward's rolling h, the backward's adjoint) per warp, or team of row workers, that is on the GPU at a time: a
+// team is done with it before its next item.  The bound does not depend on how the items are split, and so grows with the batch only.
+static int64_t resident(int64_t items, int ctas, int warps) { return std::min(items, (int64_t)ctas * kSMs * warps); }
+static size_t blk_team_bytes(const Blk &k, bool backward, int NG) {
+    return (size_t)resident(k.items, blk_ctas(backward, NG), BK_WARPS) * k.nstrip * 4 * 32 * sizeof(float4);
+}
 static size_t blk_bc_bytes(const Blk &k, int NG) { return (size_t)(k.items / k.ntile) * k.nblk * k.nstrip * BK_PX * NG * sizeof(float2); }
 static size_t blk_col_bytes(const Blk &k) { return (size_t)k.nblk * (k.nstrip - 1) * 4 * k.NL * sizeof(float4); }
 
@@ -474,15 +484,16 @@ static int move_bytes(const void *ptr, std::initializer_list<int64_t> sizes) {
     for (int64_t s : sizes) x |= (uintptr_t)s;
     return (int)(x & (~x + 1));
 }
+static int pair_ctas(bool backward) { return backward ? 2 : 3; }   // CTAs per SM
 static int lanes_for(int pieces) {
     int l = 8;
     while (l < pieces) l <<= 1;
     return l;
 }
-static void pair_state(Pw &k, const void *saved, bool roll) {
+static void pair_state(Pw &k, const void *saved) {
     char *q = const_cast<char *>(static_cast<const char *>(saved));
     k.row = reinterpret_cast<float4 *>(q);
-    q += pair_row_bytes(k, roll);
+    q += pair_row_bytes(k);
     k.colq = reinterpret_cast<float4 *>(q);
     k.cola = reinterpret_cast<float2 *>(q + pair_col_bytes(k) / 3 * 2);
 }
@@ -519,7 +530,7 @@ static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool bac
     k.nstrip = k.lin ? 1 : (k.W + k.fs - 1) / k.fs;
     k.lpin = k.lin ? lanes_for((PW_R * k.W * es + (k.el && es == 2 ? 2 : 0) + k.vin - 1) / k.vin) : 4 * (k.el && es == 2 ? 8 : 32 / k.vin);
     // Row workers: as few as fill the GPU; with short rows a worker waits for the others at the end of a band
-    const int ctas = backward ? 2 : 3;
+    const int ctas = pair_ctas(backward);
     const int64_t slots = (int64_t)kSMs * ctas * PW_WARPS;
     double best = 1e300;
     for (int rwl = 0; rwl < 3; ++rwl) {
@@ -533,7 +544,8 @@ static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool bac
     const int64_t need = ((int64_t)k.items + (PW_WARPS >> k.rwl) - 1) / (PW_WARPS >> k.rwl), cap = ctas * kSMs;
     k.grid = (int)(need < cap ? need : cap);
 }
-static size_t pair_row_bytes(const Pw &k, bool roll) { return (size_t)k.items * (roll ? 1 : k.nblk - 1) * k.wp * 32 * sizeof(float4); }
+static size_t pair_row_bytes(const Pw &k) { return (size_t)k.items * (k.nblk - 1) * k.wp * 32 * sizeof(float4); }
+static size_t pair_team_bytes(const Pw &k, bool backward) { return (size_t)resident(k.items, pair_ctas(backward), PW_WARPS) * k.wp * 32 * sizeof(float4); }
 static size_t pair_col_bytes(const Pw &k) { return (size_t)k.items * k.nblk * (k.nsub - 1) * PW_R * 32 * 24; }
 // pieces of results that take the place of inputs in shared memory
 static int pair_vout(const Pw &k, const void *ptr, int es, int64_t bs, int64_t ds, int64_t hs) {
@@ -565,7 +577,7 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
         const int es = esize(p->io_dtype);
         pair_out(k, es, pair_vout(k, out, es, out_bs, out_ds, out_hs));
         k.v32 = move_bytes(out, {out_bs * 4, out_ds * 4, out_hs * 4, (int64_t)k.W * 4}) == 8;
-        pair_state(k, saved, rolling);
+        pair_state(k, saved);
         cudaError_t e = launch_pair_fwd(k, !rolling, reinterpret_cast<cudaStream_t>(stream));
         if (e != cudaSuccess) return fail(CS2D_ERR_CUDA, "forward launch failed: %s", cudaGetErrorString(e));
         g_launches.fetch_add(1);
@@ -719,9 +731,20 @@ static int det_layout(const cs2d_problem *p, DetLayout *l) {
     return CS2D_OK;
 }
 
+// Fewer CTAs where the scratch is given and holds the rows of fewer teams (cs2d_bwd_noalloc).
+static bool fit_grid(int *grid, int64_t items, int teams_per_cta, size_t row, size_t limit) {
+    const int64_t teams = (int64_t)(limit / row);
+    if (std::min(items, (int64_t)*grid * teams_per_cta) <= teams) return true;
+    *grid = (int)(teams / teams_per_cta);
+    if (*grid > 0) return true;
+    fail(CS2D_ERR_UNSUPPORTED, "one row of the backward scratch is larger than the built-in buffer");
+    return false;
+}
+
 static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout, int64_t dout_bs, int64_t dout_ds,
                     int64_t dout_hs, const void *saved, void *scratch, void *du, void *ddelta, float *dA, float *dB,
-                    float *dC, float *dD, float *ddelta_bias, float *dA_decay, void *stream, float *det = nullptr) {
+                    float *dC, float *dD, float *ddelta_bias, float *dA_decay, void *stream, float *det = nullptr,
+                    size_t scratch_limit = SIZE_MAX) {
     int rc = validate(p);
     if (rc) return rc;
     if ((rc = check_dirs(p, o))) return rc;
@@ -741,12 +764,13 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
     if (!det && pair_ok(p, o)) {
         Pw k;
         pair_fill(k, p, o, true, dout, dout_bs, dout_ds, dout_hs);
-        pair_state(k, saved, false);
+        pair_state(k, saved);
         k.out = const_cast<void *>(dout); k.o_bs = dout_bs; k.o_ds = dout_ds; k.o_hs = dout_hs;
         const int es = esize(p->io_dtype);
         const int64_t W = p->ncols, HW = W * p->nrows;
         pair_out(k, es, std::min(pair_vout(k, du, es, HW, HW, W), pair_vout(k, ddelta, es, HW, HW, W)));
         k.v32 = move_bytes(du, {HW * 4, W * 4}) == 8;
+        if (!fit_grid(&k.grid, k.items, PW_WARPS >> k.rwl, (size_t)k.wp * 32 * sizeof(float4), scratch_limit)) return CS2D_ERR_UNSUPPORTED;
         k.adj = reinterpret_cast<float4 *>(scratch);
         k.du = du; k.ddelta = ddelta; k.dA = dA; k.dB = dB; k.dC = dC; k.dD = dD; k.dbias = ddelta_bias;
         cudaError_t e = launch_pair_bwd(k, reinterpret_cast<cudaStream_t>(stream));
@@ -763,6 +787,7 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
         k.adj = reinterpret_cast<float4 *>(scratch);
         k.du = du; k.ddelta = ddelta; k.dA = dA; k.dB = dB; k.dC = dC; k.dD = dD; k.dbias = ddelta_bias; k.ddecay = dA_decay;
         k.vec_dbc = vec_ok(dB, 4, p->ncols, {}) && vec_ok(dC, 4, p->ncols, {});
+        if (!fit_grid(&k.grid, k.items, BK_WARPS >> k.rwl, (size_t)k.nstrip * 4 * 32 * sizeof(float4), scratch_limit)) return CS2D_ERR_UNSUPPORTED;
         cudaError_t e = launch_blk_bwd(k, NG, reinterpret_cast<cudaStream_t>(stream));
         if (e != cudaSuccess) return fail(CS2D_ERR_CUDA, "backward launch failed: %s", cudaGetErrorString(e));
         g_launches.fetch_add(1);
@@ -948,7 +973,9 @@ int cs2d_bwd_noalloc(const cs2d_problem *p, const void *dout, int64_t dout_bs, i
                      float *ddelta_bias, float *dA_decay, void *stream) {
     int rc = validate(p);
     if (rc) return rc;
-    const size_t need = cs2d_bwd_scratch_bytes(p);
+    // The limit is on the tile kernels' rows, one per channel and state pair: the other families take as many CTAs as the array
+    // has rows for.
+    const size_t need = layout_bytes(p, true);
     if (need == 0) return CS2D_ERR_UNSUPPORTED;  // message already set by the planner
     if (need > (size_t)CS2D_NOALLOC_SCRATCH_BYTES)
         return fail(CS2D_ERR_UNSUPPORTED,
@@ -957,8 +984,8 @@ int cs2d_bwd_noalloc(const cs2d_problem *p, const void *dout, int64_t dout_bs, i
                     need, (size_t)CS2D_NOALLOC_SCRATCH_BYTES);
     void *scratch = noalloc_scratch_ptr();
     if (!scratch) return CS2D_ERR_CUDA;
-    return cs2d_bwd(p, dout, dout_bs, dout_ds, dout_hs, saved, scratch, du, ddelta, dA, dB, dC, dD, ddelta_bias,
-                    dA_decay, stream);
+    return bwd_impl(p, nullptr, dout, dout_bs, dout_ds, dout_hs, saved, scratch, du, ddelta, dA, dB, dC, dD, ddelta_bias,
+                    dA_decay, stream, nullptr, CS2D_NOALLOC_SCRATCH_BYTES);
 }
 
 int cs2d_device_status(void) {

@@ -47,12 +47,13 @@ struct Blk {
     void *out; int64_t o_bs, o_ds, o_hs;    // forward: out; backward: dout
     const float *mw; float *dw;             // direction merge (see Dev)
     // Checkpoints, threads innermost so that a warp moves whole lines:
-    //   row [nblk][nstrip][4][NL] float4 = h of the block's last row, two columns per float4 (rolling: nblk = 1)
+    //   row [nblk][nstrip][4][NL] float4 = h of the block's last row, two columns per float4
+    //       (rolling: [teams][nstrip][4][32], one row per warp, or per team of row workers, that is on the GPU at a time)
     //   col [nblk][nstrip-1][4][NL] float4 = (q, s) of the column left of block strip+1, one row per float4
     float4 *row, *col;
     float2 *bc;                             // B and C in walk order (blk_bc_kernel)
     // backward
-    float4 *adj;                            // [nstrip][4][NL]: the adjoint row m between rows of blocks
+    float4 *adj;                            // [teams][nstrip][4][32]: the adjoint row m between rows of blocks
     void *du, *ddelta;
     float *dA, *dB, *dC, *dD, *dbias, *ddecay;
     int vec_dbc;                            // dB, dC: rows of whole aligned groups of four columns

@@ -179,9 +179,9 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
             const int64_t lin = ((int64_t)q.bg * P.nsl + min(q.slot + sl_, P.nsl - 1)) * NG + n;
             row = P.row + ((int64_t)((blk - 1) * P.nstrip + strip) * 4) * P.NL + lin;
             col = P.col + ((int64_t)blk * (P.nstrip - 1) + strip - 1) * 4 * P.NL + lin;
-            arow = P.adj + (int64_t)strip * 4 * P.NL + lin;
+            arow = P.adj + ((int64_t)(first + (warp >> P.rwl)) * P.nstrip + strip) * 4 * 32 + lane;
         } else {
-            row -= 4 * P.NL; col -= 4 * P.NL; arow -= 4 * P.NL;
+            row -= 4 * P.NL; col -= 4 * P.NL; arow -= 4 * 32;
         }
         row_on = blk > 0;
         fetch_row(0);
@@ -323,8 +323,8 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
         float4 adjv[2];
         auto fetch_adj = [&](int k) {
             const bool there = blk + 1 < P.nblk;
-            adjv[0] = bk_ld16<false>(arow + 2 * k * P.NL, there);
-            adjv[1] = bk_ld16<false>(arow + (2 * k + 1) * P.NL, there);
+            adjv[0] = bk_ld16<false>(arow + 2 * k * 32, there);
+            adjv[1] = bk_ld16<false>(arow + (2 * k + 1) * 32, there);
         };
         fetch_adj(nhalf - 1);
         if (non && nhalf == 1) copy_bc(nxt, 1);
@@ -416,8 +416,8 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
                 __syncwarp();
             }
             if (blk > 0) {   // m of the block's first row
-                bk_st16(arow + 2 * k * P.NL, make_float4(mb[0].x, mb[0].y, mb[1].x, mb[1].y), mine);
-                bk_st16(arow + (2 * k + 1) * P.NL, make_float4(mb[2].x, mb[2].y, mb[3].x, mb[3].y), mine);
+                bk_st16(arow + 2 * k * 32, make_float4(mb[0].x, mb[0].y, mb[1].x, mb[1].y), mine);
+                bk_st16(arow + (2 * k + 1) * 32, make_float4(mb[2].x, mb[2].y, mb[3].x, mb[3].y), mine);
             }
             if (non) copy_bc(nxt, k);
             // half a block's dB and dC onto the results: four columns at a time where the rows allow it, else one

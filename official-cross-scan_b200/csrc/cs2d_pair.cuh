@@ -19,7 +19,8 @@
 // number of pieces.
 //
 // What crosses a band or 8 columns goes through global memory, threads innermost (512 bytes per warp and access):
-//   row  [item][band][column][32] float4 (h, h', a, a') of a band's last row (rolling: one band)
+//   row  [item][band][column][32] float4 (h, h', a, a') of a band's last row (rolling: one row per warp, or team of row
+//        workers, that is on the GPU at a time, whatever its item)
 //   colq [item][band][column / 8 - 1][4 rows][32] float4 (q, q', s, s') of the column left of a group of 8
 //   cola the same, float2 (a, a')
 // (q = h - s; an item is a warp's 64 channels of one image and group.)
@@ -54,7 +55,7 @@ struct Pw {
     void *out; int64_t o_bs, o_ds, o_hs;    // forward: out; backward: dout
     const float *mw; float *dw;             // direction merge (see Dev)
     float4 *row, *colq; float2 *cola;
-    float4 *adj;                            // backward, [item][column][32]: (m, m', a, a') of the row below a band
+    float4 *adj;                            // backward, [team][column][32]: (m, m', a, a') of the row below a band
     void *du, *ddelta;
     float *dA, *dB, *dC, *dD, *dbias;
 };

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
         const bool fh = DIRS && ((P.flip_h >> pos.g) & 1u), fw = DIRS && ((P.flip_w >> pos.g) & 1u);
         const int nc = min(P.fs, P.W - c0);
         const float4 *above = P.row + (((int64_t)pos.item * (P.nblk - 1) + blk - 1) * P.wp + c0) * 32 + lane;
-        float4 *arow = P.adj + ((int64_t)pos.item * P.wp + c0) * 32 + lane;
+        float4 *arow = P.adj + ((int64_t)(first + (warp >> P.rwl)) * P.wp + c0) * 32 + lane;
         if (pos.strip == 0) {
             if (pos.pass == 0) {   // a new item
                 const int k0 = min(2 * lane, nch - 1), k1 = min(2 * lane + 1, nch - 1);

@@ -58,8 +58,8 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
         const int blk = pos.pass * rw + w, r0 = blk * PW_R, c0 = pos.strip * P.fs, ch0 = pos.tile * PW_CH, cg = pos.g * P.dpg + ch0, nch = P.dpg - ch0, b = pos.bg / P.G;
         const bool fh = DIRS && ((P.flip_h >> pos.g) & 1u), fw = DIRS && ((P.flip_w >> pos.g) & 1u);
         const int nc = min(P.fs, P.W - c0);
-        // row of the band above (rolling: the same row), row of this band
-        float4 *row = P.row + (((int64_t)pos.item * (KEEP ? P.nblk - 1 : 1) + (KEEP ? blk : 0)) * P.wp + c0) * 32 + lane;
+        // row of the band above (rolling: the same row), row of this band (rolling: the team's)
+        float4 *row = P.row + ((KEEP ? (int64_t)pos.item * (P.nblk - 1) + blk : first + (warp >> P.rwl)) * P.wp + c0) * 32 + lane;
         const float4 *above = KEEP ? row - (int64_t)P.wp * 32 : row;
         float4 up[2];
         auto fetch_up = [&](int c) {
