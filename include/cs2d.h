@@ -73,7 +73,7 @@ typedef struct {
  * the reference's three side tensors x, x_v, x_sd (selective_scan_oflex.cpp:251-258);
  * unlike them it is NOT modified by the backward, so backward may run twice on it.
  * A backward reads what the forward of the SAME problem, directions and flags wrote.
- * Returns 0 for an invalid problem.
+ * Covers every set of directions (see cs2d_saved_bytes_dir).  Returns 0 for an invalid problem.
  */
 size_t cs2d_saved_bytes(const cs2d_problem *p);
 
@@ -176,6 +176,15 @@ int cs2d_bwd_dir(const cs2d_problem *p, const cs2d_dirs *dirs, const void *dout,
                  int64_t dout_ds, int64_t dout_hs, const void *saved, void *scratch, void *du, void *ddelta,
                  float *dA, float *dB, float *dC, float *dD, float *ddelta_bias, float *dA_decay,
                  void *stream);
+
+/*
+ * Sizes for one set of directions and flags (dirs may be NULL): what the kernels that run for it use, where
+ * cs2d_saved_bytes, cs2d_bwd_scratch_bytes and cs2d_fwd_only_scratch_bytes cover every set.  The scratch is that
+ * of cs2d_bwd_dir (and of cs2d_bwd, for NULL); cs2d_bwd_det takes the covering size.
+ */
+size_t cs2d_saved_bytes_dir(const cs2d_problem *p, const cs2d_dirs *dirs);
+size_t cs2d_bwd_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *dirs);
+size_t cs2d_fwd_only_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *dirs);
 
 /*
  * Deterministic backward: bit-identical results from run to run.  cs2d_bwd (like

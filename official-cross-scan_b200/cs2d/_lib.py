@@ -67,6 +67,8 @@ def lib():
         L.cs2d_bwd.restype = ctypes.c_int
         L.cs2d_bwd.argtypes = [ctypes.POINTER(Problem), vp, i64, i64, i64, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
         dp = ctypes.POINTER(Dirs)
+        for f in (L.cs2d_saved_bytes_dir, L.cs2d_bwd_scratch_bytes_dir, L.cs2d_fwd_only_scratch_bytes_dir):
+            f.restype, f.argtypes = ctypes.c_size_t, [ctypes.POINTER(Problem), dp]
         L.cs2d_fwd_dir.restype = ctypes.c_int
         L.cs2d_fwd_dir.argtypes = [ctypes.POINTER(Problem), dp, vp, i64, i64, i64, vp, vp]
         L.cs2d_fwd_only.restype = ctypes.c_int

@@ -48,6 +48,17 @@ def _auto_chunk(host, batch):
     return -(-batch // chunks)
 
 
+def _sizes(p, dirs, batch, chunk):
+    """Bytes of the saved state and of the backward scratch that serve a full chunk and the last one (which other kernels
+    may run, having fewer samples); 0 where a chunk has no kernel."""
+    L, o = _lib.lib(), ctypes.byref(dirs) if dirs is not None else None
+    sizes = []
+    for n in {min(chunk, batch), batch % chunk or chunk}:
+        p.batch = n
+        sizes.append((L.cs2d_saved_bytes_dir(ctypes.byref(p), o), L.cs2d_bwd_scratch_bytes_dir(ctypes.byref(p), o)))
+    return (0, 0) if any(0 in s for s in sizes) else tuple(max(s) for s in zip(*sizes))
+
+
 class HostPipeline:
     """Preallocated three-stream pipeline for one problem shape; see the module docstring."""
 
@@ -77,12 +88,10 @@ class HostPipeline:
                     s.update(dB=mk(B), dC=mk(B))
                 s["free"], s["loaded"], s["done"] = torch.cuda.Event(), torch.cuda.Event(), torch.cuda.Event()
                 self.slots.append(s)
-            # saved state and backward scratch are sized for a full chunk
             s0 = self.slots[0]
             p = ops._problem(s0["u"], s0["delta"], self.A, s0["B"], s0["C"], self.D, self.bias, None, delta_softplus, odt,
                              "host pipeline")
-            L = _lib.lib()
-            nsaved, nscr = L.cs2d_saved_bytes(ctypes.byref(p)), L.cs2d_bwd_scratch_bytes(ctypes.byref(p))
+            nsaved, nscr = _sizes(p, None, self.batch, c)
             if nsaved == 0 or nscr == 0:
                 raise RuntimeError(f"cs2d host pipeline: {_lib.last_error()}")
             for s in self.slots:
@@ -241,8 +250,8 @@ class CrossHostPipeline:
             s0 = self.slots[0]
             p = ops._problem(s0["u"], s0["delta"], self.A, s0["B"], s0["C"], self.D, self.bias, None, delta_softplus,
                              torch.float32, "host pipeline", shared_u_dim=dim)
-            L = _lib.lib()
-            nsaved, nscr = L.cs2d_saved_bytes(ctypes.byref(p)), L.cs2d_bwd_scratch_bytes(ctypes.byref(p))
+            dirs = _lib.Dirs(self.rows, self.cols, 3, 0, self.wf.data_ptr(), None)
+            nsaved, nscr = _sizes(p, dirs, self.batch, c)
             if nsaved == 0 or nscr == 0:
                 raise RuntimeError(f"cs2d host pipeline: {_lib.last_error()}")
             for s in self.slots:

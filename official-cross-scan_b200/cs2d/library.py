@@ -31,7 +31,7 @@ from . import _lib, ops
 _DT = ops._DT
 
 
-def _saved_numel(u, A, B, delta, out_float):
+def _saved_numel(u, A, B, delta, delta_softplus, out_float, A_decay):
     """Size of the saved-state buffer from shapes alone (no device pointers needed)."""
     p = _lib.Problem()
     p.batch, p.dim, p.nrows, p.ncols = (int(s) for s in u.shape)
@@ -41,7 +41,8 @@ def _saved_numel(u, A, B, delta, out_float):
     # the size query validates that the tensors are present but never dereferences them:
     # fake tensors have no storage, so it gets placeholder addresses
     p.u = p.delta = p.A = p.B = p.C = 256
-    nbytes = _lib.lib().cs2d_saved_bytes(ctypes.byref(p))
+    p.delta_softplus, p.A_decay = int(bool(delta_softplus)), None if A_decay is None else 256
+    nbytes = _lib.lib().cs2d_saved_bytes_dir(ctypes.byref(p), None)
     if nbytes == 0:
         raise RuntimeError(f"cs2d forward: {_lib.last_error()}")
     return nbytes // 4
@@ -58,7 +59,7 @@ def scan_fwd(u: Tensor, delta: Tensor, A: Tensor, B: Tensor, C: Tensor, D: Optio
 @scan_fwd.register_fake
 def _scan_fwd_fake(u, delta, A, B, C, D, delta_bias, delta_softplus, out_float, A_decay):
     out = u.new_empty(tuple(u.shape), dtype=torch.float32 if out_float else u.dtype)
-    return out, u.new_empty((_saved_numel(u, A, B, delta, out_float),), dtype=torch.float32)
+    return out, u.new_empty((_saved_numel(u, A, B, delta, delta_softplus, out_float, A_decay),), dtype=torch.float32)
 
 
 @torch.library.custom_op("cs2d::scan_bwd", mutates_args=(), device_types="cuda")

@@ -98,7 +98,7 @@ class ResidentStep:
         L = _lib.lib()
         p = ops._problem(u, t["delta"], t["A"], B, t["C"], t.get("D"), t.get("delta_bias"), None, delta_softplus, u.dtype,
                          "resident step")
-        nsaved, nscr = L.cs2d_saved_bytes(ctypes.byref(p)), L.cs2d_bwd_scratch_bytes(ctypes.byref(p))
+        nsaved, nscr = L.cs2d_saved_bytes_dir(ctypes.byref(p), None), L.cs2d_bwd_scratch_bytes_dir(ctypes.byref(p), None)
         if nsaved == 0 or nscr == 0:
             raise RuntimeError(f"cs2d resident step: {_lib.last_error()}")
         with torch.cuda.device(dev):

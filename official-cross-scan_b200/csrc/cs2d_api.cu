@@ -273,6 +273,14 @@ static int tile_view(const cs2d_problem *p, int t, bool backward, bool bulk_ok, 
 
 static bool walk_shape(const cs2d_problem *p) { return p->dstate > 8 && p->ncols <= 8 * STRIP; }
 
+// Which kernels run (the row-walk forward goes with the tile kernels: it writes the same checkpoints)
+enum Family { PAIR, STREAM, BLK, TILE };
+static Family family(const cs2d_problem *p, const cs2d_dirs *o);
+static bool walk_fwd_ok(const cs2d_problem *p, const cs2d_dirs *o);
+static bool pair_one(const cs2d_problem *p);
+static bool pair_dirs(const cs2d_problem *p);
+static int check_dirs(const cs2d_problem *p, const cs2d_dirs *o);
+static size_t stream_state_bytes(const cs2d_problem *p);
 static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o, bool backward);
 static size_t blk_row_bytes(const Blk &k);
 static size_t blk_team_bytes(const Blk &k, bool backward, int NG);
@@ -298,50 +306,69 @@ static size_t edge_bytes(const cs2d_problem *p, int NPp) {
     return (size_t)p->batch * p->dim * NPp * p->nrows * sizeof(float4);
 }
 
-// backward: adjoint rows; otherwise the forward's state rows - all checkpoints, or (rolling) one
-// row per channel and state pair for a forward that no backward follows
-static size_t layout_bytes(const cs2d_problem *p, bool backward, bool rolling = false) {
+// What a buffer holds: the forward's saved state, the rolling rows of a forward that no backward follows, the backward's scratch
+enum Buffer { SAVED, ROLLING, SCRATCH };
+
+// The tile kernels' layout: adjoint rows, or the forward's state rows - all checkpoints, or (rolling) one
+// row per channel and state pair
+static size_t layout_bytes(const cs2d_problem *p, Buffer what, bool walk) {
     const int nt = n_tiles(p->ncols);
     size_t total = 0;
     int NPp = 1;
     for (int t = 0; t < nt; ++t) {
         TileView tv;
-        if (tile_view(p, t, backward, false, &tv) != CS2D_OK) return 0;
-        total += backward || rolling ? tv.adj_bytes : tv.saved_bytes;
+        if (tile_view(p, t, what == SCRATCH, false, &tv) != CS2D_OK) return 0;
+        total += what == SAVED ? tv.saved_bytes : tv.adj_bytes;
         NPp = tv.g.NPp;
     }
     total += (size_t)(nt - 1) * edge_bytes(p, NPp);
-    // the row-walk forward keeps B and C, regrouped, behind the checkpoints (whatever the scan directions
-    // turn out to be: the size depends on the problem alone)
-    if (!backward && walk_shape(p)) total += walk_bc_bytes(p->batch, p->n_groups, p->nrows, p->ncols);
+    // the row-walk forward keeps B and C, regrouped, behind the checkpoints
+    if (what != SCRATCH && walk) total += walk_bc_bytes(p->batch, p->n_groups, p->nrows, p->ncols);
     return total;
 }
 
-// Problems of the block-walk and the pair-walk kernels: what those need, or the tile kernels, which the reproducible
-// direction merge uses - the size depends on the problem alone.
-static size_t state_bytes(const cs2d_problem *p, bool backward, bool rolling) {
-    if (validate(p) != CS2D_OK) return 0;
-    const size_t tile = layout_bytes(p, backward, rolling);
-    if (tile == 0) return tile;
-    if (pair_shape(p)) {
-        Pw k;
-        pair_fill(k, p, nullptr, backward);
-        const size_t need = backward || rolling ? pair_team_bytes(k, backward) : pair_row_bytes(k) + pair_col_bytes(k);
-        return tile > need ? tile : need;
-    }
-    if (!blk_shape(p)) return tile;
+static size_t blk_bytes(const cs2d_problem *p, Buffer what) {
     Blk k;
     int NG;
-    blk_fill(k, NG, p, nullptr, backward);
-    const size_t need = backward ? blk_team_bytes(k, true, NG) : blk_bc_bytes(k, NG) + (rolling ? blk_team_bytes(k, false, NG) : blk_row_bytes(k) + blk_col_bytes(k));
-    return tile > need ? tile : need;
+    blk_fill(k, NG, p, nullptr, what == SCRATCH);
+    if (what == SCRATCH) return blk_team_bytes(k, true, NG);
+    return blk_bc_bytes(k, NG) + (what == ROLLING ? blk_team_bytes(k, false, NG) : blk_row_bytes(k) + blk_col_bytes(k));
+}
+static size_t pair_bytes(const cs2d_problem *p, Buffer what) {
+    Pw k;
+    pair_fill(k, p, nullptr, what == SCRATCH);
+    return what == SAVED ? pair_row_bytes(k) + pair_col_bytes(k) : pair_team_bytes(k, what == SCRATCH);
 }
 
-size_t cs2d_saved_bytes(const cs2d_problem *p) { return state_bytes(p, false, false); }
+// Whatever the directions and flags
+static size_t any_bytes(const cs2d_problem *p, Buffer what) {
+    if (validate(p) != CS2D_OK) return 0;
+    const size_t tile = layout_bytes(p, what, walk_shape(p));
+    if (tile == 0) return 0;
+    const size_t need = pair_shape(p) && (pair_one(p) || pair_dirs(p)) ? pair_bytes(p, what) : blk_shape(p) ? blk_bytes(p, what) : 0;
+    return std::max(tile, need);
+}
 
-size_t cs2d_bwd_scratch_bytes(const cs2d_problem *p) { return state_bytes(p, true, false); }
+size_t cs2d_saved_bytes(const cs2d_problem *p) { return any_bytes(p, SAVED); }
 
-size_t cs2d_fwd_only_scratch_bytes(const cs2d_problem *p) { return state_bytes(p, false, true); }
+size_t cs2d_bwd_scratch_bytes(const cs2d_problem *p) { return any_bytes(p, SCRATCH); }
+
+size_t cs2d_fwd_only_scratch_bytes(const cs2d_problem *p) { return any_bytes(p, ROLLING); }
+
+// The same for one set of directions and flags: what the kernels that will run use
+static size_t exact_bytes(const cs2d_problem *p, const cs2d_dirs *o, Buffer what) {
+    if (validate(p) != CS2D_OK || check_dirs(p, o) != CS2D_OK || layout_bytes(p, what, false) == 0) return 0;
+    const Family f = family(p, o);
+    size_t n = 16;   // (no buffer is empty)
+    if (f == PAIR) n = pair_bytes(p, what);
+    else if (f == STREAM && what == SAVED) n = stream_state_bytes(p);
+    else if (f == BLK) n = blk_bytes(p, what);
+    else if (f == TILE) n = layout_bytes(p, what, walk_fwd_ok(p, o));
+    return std::max<size_t>(n, 16);
+}
+size_t cs2d_saved_bytes_dir(const cs2d_problem *p, const cs2d_dirs *o) { return exact_bytes(p, o, SAVED); }
+size_t cs2d_bwd_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *o) { return exact_bytes(p, o, SCRATCH); }
+size_t cs2d_fwd_only_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *o) { return exact_bytes(p, o, ROLLING); }
 
 // A group that walks the columns right-to-left sees the tile's scan columns at mirrored image
 // columns (Dev::cshift); 4-element accesses are only kept when that shift preserves 16-byte alignment.
@@ -360,12 +387,12 @@ static int check_dirs(const cs2d_problem *p, const cs2d_dirs *o) {
 // ---- streaming kernels (cs2d_stream.cu) -------------------------------------------------------
 // A problem with a single state per channel, one scan orientation, no A_decay and rows of at most
 // 128 columns (16 lanes of 8) runs on the streaming kernels: no shared-memory tiles, no backward scratch, and
-// checkpoints that pack two channels per value (half the bytes of the tile kernels' layout, which
-// is what cs2d_saved_bytes reports and therefore always large enough).  The choice depends on
+// checkpoints that pack two channels per value (half the bytes of the tile kernels' layout).  The choice depends on
 // nothing but these properties, so the forward and the backward of a problem always agree.
 static bool has_dirs(const cs2d_dirs *o) {
     return o && (o->flip_rows_mask || o->flip_cols_mask || o->shared_input || o->merge_w);
 }
+static bool dirs_serial(const cs2d_dirs *o) { return o && o->merge_w && (o->flags & CS2D_DIRS_SERIAL); }   // one CTA walks all directions
 static bool stream_ok(const cs2d_problem *p, const cs2d_dirs *o) {
     return p->dstate == 1 && !has_dirs(o) && !p->A_decay && p->ncols <= 16 * STRIP;
 }
@@ -374,6 +401,10 @@ static int stream_lanes(const cs2d_problem *p) {
     int L = 1;
     while (L < strips) L <<= 1;
     return L;
+}
+static size_t stream_state_bytes(const cs2d_problem *p) {
+    const size_t pairs = (size_t)p->batch * p->n_groups * ((p->dim / p->n_groups + 1) / 2);
+    return pairs * ((p->nrows + STREAM_RB - 1) / STREAM_RB) * (stream_lanes(p) * STRIP) * sizeof(float2);
 }
 // Geometry shared by both streaming launches: lanes per row, CTAs per (batch, group), grid.
 static void stream_fill(Dev &d, const cs2d_problem *p, int *L, int *grid) {
@@ -404,7 +435,7 @@ static void stream_fill(Dev &d, const cs2d_problem *p, int *L, int *grid) {
 static bool walk_fwd_ok(const cs2d_problem *p, const cs2d_dirs *o) { return walk_shape(p) && !has_dirs(o); }
 
 // ---- block-walk kernels (cs2d_blk_fwd.cu, cs2d_blk_bwd.cu) -------------------------------------------
-static bool blk_ok(const cs2d_problem *p, const cs2d_dirs *o) { return blk_shape(p) && !(o && o->merge_w && (o->flags & CS2D_DIRS_SERIAL)); }
+static bool blk_ok(const cs2d_problem *p, const cs2d_dirs *o) { return blk_shape(p) && !dirs_serial(o); }
 // the parts of the saved state (or of the forward-only scratch)
 static void blk_state(Blk &k, int NG, const void *saved, bool roll) {
     char *q = const_cast<char *>(static_cast<const char *>(saved));
@@ -434,7 +465,8 @@ static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o,
     NG = 8;
     while (NG < p->dstate) NG <<= 1;
     k.nsl = (k.dpg + 1) / 2;
-    k.NL = (int64_t)p->batch * k.G * k.nsl * NG;
+    k.NS = k.N <= 4 ? k.N + 1 : NG;
+    k.NL = (int64_t)p->batch * k.G * k.nsl * k.NS;
     const int spw = 32 / NG, ctas = blk_ctas(backward, NG);   // slots per warp, CTAs per SM
     k.ntile = (k.nsl + spw - 1) / spw; k.items = p->batch * k.G * k.ntile;
     // Row workers: as few as fill the GPU; with short rows a worker waits for the others at the end of a row
@@ -453,7 +485,7 @@ static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o,
     const int64_t cap = ctas * kSMs;   // CTAs that fit at once
     k.grid = (int)(need < cap ? need : cap);
 }
-static size_t blk_row_bytes(const Blk &k) { return (size_t)k.nblk * k.nstrip * 4 * k.NL * sizeof(float4); }
+static size_t blk_row_bytes(const Blk &k) { return (size_t)(k.nblk - 1) * k.nstrip * 4 * k.NL * sizeof(float4); }
 // One row (the forward's rolling h, the backward's adjoint) per warp, or team of row workers, that is on the GPU at a time: a
 // team is done with it before its next item.  The bound does not depend on how the items are split, and so grows with the batch only.
 static int64_t resident(int64_t items, int ctas, int warps) { return std::min(items, (int64_t)ctas * kSMs * warps); }
@@ -470,13 +502,20 @@ static size_t blk_col_bytes(const Blk &k) { return (size_t)k.nblk * (k.nstrip - 
 // fp32 7 columns 513 / 192, 16: 637 / 424, 56: 738 / 785).  The alternative of directions and of wider rows are the tile
 // kernels (28x28 cross 2133 / 398, 150x150 scan 21944 / 4273), except where a few warps' worth of channels on a large map
 // would leave the GPU idle (8 items of 224x224: 4265 / 7178; of 56x56: 794 / 507).
-static bool pair_ok(const cs2d_problem *p, const cs2d_dirs *o) {
-    if (!pair_shape(p) || (o && o->merge_w && (o->flags & CS2D_DIRS_SERIAL))) return false;
-    const int W = p->ncols, dpg = p->dim / p->n_groups;
-    if (has_dirs(o) || W > 16 * STRIP)
-        return W <= 64 || (int64_t)p->batch * p->n_groups * ((dpg + PW_CH - 1) / PW_CH) >= 16;
+static bool pair_dirs(const cs2d_problem *p) {   // the alternative: tile kernels
+    return p->ncols <= 64 || (int64_t)p->batch * p->n_groups * ((p->dim / p->n_groups + PW_CH - 1) / PW_CH) >= 16;
+}
+static bool pair_one(const cs2d_problem *p) {    // streaming kernels
+    const int W = p->ncols;
     if (p->io_dtype == CS2D_F32) return W <= 16;
     return W < 16 || (W % 2 ? W <= 45 : W % 4 && W <= 24);
+}
+static bool pair_ok(const cs2d_problem *p, const cs2d_dirs *o) {
+    if (!pair_shape(p) || dirs_serial(o)) return false;
+    return has_dirs(o) || p->ncols > 16 * STRIP ? pair_dirs(p) : pair_one(p);
+}
+static Family family(const cs2d_problem *p, const cs2d_dirs *o) {
+    return pair_ok(p, o) ? PAIR : stream_ok(p, o) ? STREAM : blk_ok(p, o) ? BLK : TILE;
 }
 // Bytes that may be moved at once, 8 at most: a divisor of every size and stride (in bytes) and of the address
 static int move_bytes(const void *ptr, std::initializer_list<int64_t> sizes) {
@@ -512,6 +551,7 @@ static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool bac
     }
     k.f32 = p->io_dtype != CS2D_F32 && p->out_dtype == CS2D_F32;
     k.nblk = (k.H + PW_R - 1) / PW_R; k.nsub = (k.W + 7) / 8; k.wp = (k.W + 1) & ~1;
+    k.np = (k.dpg + 1) / 2;
     k.ntile = (k.dpg + PW_CH - 1) / PW_CH; k.items = p->batch * k.G * k.ntile;
     // How blocks are moved (see cs2d_pair.cuh): whole bands where every tensor's rows are contiguous and a band fits
     struct In { const void *p; int64_t bs, ds, hs; } in[3] = {{p->u, p->u_bs, p->u_ds, p->u_hs}, {p->delta, p->delta_bs, p->delta_ds, p->delta_hs}, {img, img_bs, img_ds, img_hs}};
@@ -544,9 +584,9 @@ static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool bac
     const int64_t need = ((int64_t)k.items + (PW_WARPS >> k.rwl) - 1) / (PW_WARPS >> k.rwl), cap = ctas * kSMs;
     k.grid = (int)(need < cap ? need : cap);
 }
-static size_t pair_row_bytes(const Pw &k) { return (size_t)k.items * (k.nblk - 1) * k.wp * 32 * sizeof(float4); }
+static size_t pair_row_bytes(const Pw &k) { return (size_t)(k.items / k.ntile) * (k.nblk - 1) * k.wp * k.np * sizeof(float4); }
 static size_t pair_team_bytes(const Pw &k, bool backward) { return (size_t)resident(k.items, pair_ctas(backward), PW_WARPS) * k.wp * 32 * sizeof(float4); }
-static size_t pair_col_bytes(const Pw &k) { return (size_t)k.items * k.nblk * (k.nsub - 1) * PW_R * 32 * 24; }
+static size_t pair_col_bytes(const Pw &k) { return (size_t)(k.items / k.ntile) * k.nblk * (k.nsub - 1) * PW_R * k.np * 24; }
 // pieces of results that take the place of inputs in shared memory
 static int pair_vout(const Pw &k, const void *ptr, int es, int64_t bs, int64_t ds, int64_t hs) {
     if (k.el && es == 2) return 2;
@@ -644,7 +684,7 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
         TileView tv;
         const bool bulk = nt == 1 && !dirs && bulk_ok1(p->u, es, p->ncols, p->u_bs, p->u_ds, p->u_hs) &&
                           bulk_ok1(p->delta, es, p->ncols, p->delta_bs, p->delta_ds, p->delta_hs);
-        const bool serial = o && o->merge_w && (o->flags & CS2D_DIRS_SERIAL);   // a CTA walks all directions of its channel tile
+        const bool serial = dirs_serial(o);   // a CTA walks all directions of its channel tile
         if ((rc = tile_view(p, t, false, bulk, &tv, serial))) return rc;
         Dev d;
         fill(d, &tv.q, tv.g);
@@ -727,7 +767,7 @@ static int det_layout(const cs2d_problem *p, DetLayout *l) {
     l->dD = l->dA + (int64_t)p->batch * p->dim * p->dstate; l->dbias = l->dD + (int64_t)p->batch * p->dim;
     l->ddecay = l->dbias + (int64_t)p->batch * p->dim; l->total = l->ddecay + l->grid;
     l->state = (l->total + 3) & ~int64_t(3);   // problems of the block-walk and pair-walk kernels: other kernels' checkpoints
-    if (blk_shape(p) || pair_shape(p)) l->total = l->state + (int64_t)(layout_bytes(p, false) / 4);
+    if (blk_shape(p) || pair_shape(p)) l->total = l->state + (int64_t)(layout_bytes(p, SAVED, walk_shape(p)) / 4);
     return CS2D_OK;
 }
 
@@ -750,7 +790,7 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
     if ((rc = check_dirs(p, o))) return rc;
     DetLayout dl = {};
     if (det && (rc = det_layout(p, &dl))) return rc;
-    const bool dirs = o && (o->flip_rows_mask || o->flip_cols_mask || o->shared_input || o->merge_w);
+    const bool dirs = has_dirs(o);
     if (o && o->merge_w && (det || !(o->shared_input & 2)))
         return fail(CS2D_ERR_INVALID, "the direction merge needs the shared gradient image (shared_input bit 1) "
                                       "and is not combined with the deterministic backward");
@@ -846,7 +886,7 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
         const bool bulk = nt == 1 && !dirs && bulk_ok1(p->u, es, p->ncols, p->u_bs, p->u_ds, p->u_hs) &&
                           bulk_ok1(p->delta, es, p->ncols, p->delta_bs, p->delta_ds, p->delta_hs) &&
                           bulk_ok1(dout, eso, p->ncols, dout_bs, dout_ds, dout_hs);
-        const bool serial = o && o->merge_w && (o->flags & CS2D_DIRS_SERIAL);   // a CTA walks all directions of its channel tile
+        const bool serial = dirs_serial(o);   // a CTA walks all directions of its channel tile
         if ((rc = tile_view(p, t, true, bulk, &tv, serial))) return rc;
         Dev d;
         fill(d, &tv.q, tv.g);
@@ -975,7 +1015,7 @@ int cs2d_bwd_noalloc(const cs2d_problem *p, const void *dout, int64_t dout_bs, i
     if (rc) return rc;
     // The limit is on the tile kernels' rows, one per channel and state pair: the other families take as many CTAs as the array
     // has rows for.
-    const size_t need = layout_bytes(p, true);
+    const size_t need = layout_bytes(p, SCRATCH, false);
     if (need == 0) return CS2D_ERR_UNSUPPORTED;  // message already set by the planner
     if (need > (size_t)CS2D_NOALLOC_SCRATCH_BYTES)
         return fail(CS2D_ERR_UNSUPPORTED,

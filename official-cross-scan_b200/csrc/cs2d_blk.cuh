@@ -39,15 +39,17 @@ struct Blk {
     unsigned flip_h, flip_w;
     int shared;             // bit 0: u has dpg channels shared by the groups, bit 1: dout
     int roll;               // forward: one rolling row of h instead of the checkpoints
-    int64_t NL;             // threads' worth of recurrences: batch * G * nsl * state slots
+    int NS;                 // places of a slot in the checkpoints (see below)
+    int64_t NL;             // batch * G * nsl * NS
     const void *u, *delta, *B, *C;
     const float *A, *D, *bias, *decay;
     int64_t u_bs, u_ds, u_hs, dl_bs, dl_ds, dl_hs, A_ds, A_ns;
     int64_t B_bs, B_gs, B_ns, B_hs, C_bs, C_gs, C_ns, C_hs;
     void *out; int64_t o_bs, o_ds, o_hs;    // forward: out; backward: dout
     const float *mw; float *dw;             // direction merge (see Dev)
-    // Checkpoints, threads innermost so that a warp moves whole lines:
-    //   row [nblk][nstrip][4][NL] float4 = h of the block's last row, two columns per float4
+    // Checkpoints, threads innermost so that a warp moves whole lines.  A slot has NS places: of up to four states one each
+    // and one for all lanes past them, which hold the same values (B = C = 0); 8 or 16 otherwise.  Lane n uses place min(n, NS - 1).
+    //   row [nblk-1][nstrip][4][NL] float4 = h of the block's last row, two columns per float4
     //       (rolling: [teams][nstrip][4][32], one row per warp, or per team of row workers, that is on the GPU at a time)
     //   col [nblk][nstrip-1][4][NL] float4 = (q, s) of the column left of block strip+1, one row per float4
     float4 *row, *col;

@@ -173,15 +173,17 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
         rowv[0] = bk_ld16<true>(row + 2 * k * P.NL, row_on);
         rowv[1] = bk_ld16<true>(row + (2 * k + 1) * P.NL, row_on);
     };
+    auto adj_at = [&](int strip) { return P.adj + ((int64_t)(first + (warp >> P.rwl)) * P.nstrip + strip) * 4 * 32 + lane; };
     auto fetch = [&](const BkPos &q) {
         const int blk = blk_of(q), strip = P.nstrip - 1 - q.strip;
         if (q.strip == 0) {
-            const int64_t lin = ((int64_t)q.bg * P.nsl + min(q.slot + sl_, P.nsl - 1)) * NG + n;
+            const int64_t lin = ((int64_t)q.bg * P.nsl + min(q.slot + sl_, P.nsl - 1)) * P.NS + min(n, P.NS - 1);
             row = P.row + ((int64_t)((blk - 1) * P.nstrip + strip) * 4) * P.NL + lin;
             col = P.col + ((int64_t)blk * (P.nstrip - 1) + strip - 1) * 4 * P.NL + lin;
-            arow = P.adj + ((int64_t)(first + (warp >> P.rwl)) * P.nstrip + strip) * 4 * 32 + lane;
+            if (NG == 8) arow = adj_at(strip);
         } else {
-            row -= 4 * P.NL; col -= 4 * P.NL; arow -= 4 * 32;
+            row -= 4 * P.NL; col -= 4 * P.NL;
+            if (NG == 8) arow -= 4 * 32;
         }
         row_on = blk > 0;
         fetch_row(0);
@@ -320,6 +322,7 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
         }
         tm_wait_st();
         // ---- walk back with the adjoint, half a block per iteration ----
+        if (NG == 16) arow = adj_at(strip);   // (three CTAs per SM have no register to keep it; 32x4x192x16x56x56 fp32 3850 -> 3760 us)
         float4 adjv[2];
         auto fetch_adj = [&](int k) {
             const bool there = blk + 1 < P.nblk;

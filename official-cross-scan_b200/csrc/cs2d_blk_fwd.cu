@@ -134,11 +134,11 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
     // places of the block after the current one: B and C, the row of h it writes, the row of h above it, the column left of it
     const unsigned char *nbc = nullptr;
     float4 *nrow = nullptr, *ncol = nullptr;
-    const int64_t RL = KEEP ? P.NL : 32;                          // between the four parts of a block's row of h
+    auto RL = [&]() -> int64_t { return KEEP ? P.NL : 32; };      // between the four parts of a block's row of h
     const int64_t up = KEEP ? (int64_t)P.nstrip * 4 * P.NL : 0;   // from a block's row of h back to the one above it
     auto place = [&](const BkPos &q) {   // at the start of a row of blocks
         const int blk = q.pass * rw + w;
-        const int64_t lin = ((int64_t)q.bg * P.nsl + min(q.slot + sl_, P.nsl - 1)) * NG + n;
+        const int64_t lin = ((int64_t)q.bg * P.nsl + min(q.slot + sl_, P.nsl - 1)) * P.NS + min(n, P.NS - 1);
         nbc = reinterpret_cast<const unsigned char *>(P.bc + ((int64_t)q.bg * P.nblk + blk) * P.nstrip * BK_PX * NG);
         if constexpr (KEEP) nrow = P.row + (int64_t)blk * P.nstrip * 4 * P.NL + lin;
         else nrow = P.row + (int64_t)(first + (warp >> P.rwl)) * P.nstrip * 4 * 32 + lane;   // (an item's first row of blocks reads nothing)
@@ -147,10 +147,12 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
     // half k of the row of h above block `q`, whose row of h goes to nrow
     auto fetch = [&](const BkPos &q, int k) {
         const bool there = q.pass * rw + w > 0;
-        const float4 *src = nrow - up + 2 * k * RL;
+        const float4 *src = nrow - up + 2 * k * RL();
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const float4 v = there ? src[i * RL] : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if constexpr (NG == 16 || !KEEP) v = bk_ld16<false>(src + i * RL(), there);   // (8 slots, KEEP: 2 to 10 % slower than the branch)
+            else if (there) v = src[i * RL()];
             hup[4 * k + 2 * i] = f2(v.x, v.y); hup[4 * k + 2 * i + 1] = f2(v.z, v.w);
         }
     };
@@ -176,7 +178,7 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
         const unsigned char *tbc = nbc;
         float4 *trow = nrow, *tcol = ncol;
         if (nxt.strip == 0) { if (non) place(nxt); }
-        else { nbc += BK_PX * NG * 8; nrow += 4 * RL; ncol += 4 * P.NL; }
+        else { nbc += BK_PX * NG * 8; nrow += 4 * RL(); ncol += 4 * P.NL; }
         const bool mine = pos.slot + sl_ < P.nsl;
         {
             const int ch0 = pos.slot * 2, cg = G0 * P.dpg + ch0, nch = P.dpg - ch0, r0 = blk * BK_R;
@@ -269,8 +271,8 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
                 }
             }
             if (blk + 1 < P.nblk && there) {   // the block's last row of h
-                bk_st16(trow + 2 * k * RL, make_float4(hb[0].x, hb[0].y, hb[1].x, hb[1].y), mine);
-                bk_st16(trow + (2 * k + 1) * RL, make_float4(hb[2].x, hb[2].y, hb[3].x, hb[3].y), mine);
+                bk_st16(trow + 2 * k * RL(), make_float4(hb[0].x, hb[0].y, hb[1].x, hb[1].y), mine);
+                bk_st16(trow + (2 * k + 1) * RL(), make_float4(hb[2].x, hb[2].y, hb[3].x, hb[3].y), mine);
             }
             // Half k of the row of h above the next block into the registers of half k of this one's, which are done with: the
             // loads travel while the other half is computed.  What they read was written at least two steps ago.

@@ -19,11 +19,11 @@
 // number of pieces.
 //
 // What crosses a band or 8 columns goes through global memory, threads innermost (512 bytes per warp and access):
-//   row  [item][band][column][32] float4 (h, h', a, a') of a band's last row (rolling: one row per warp, or team of row
-//        workers, that is on the GPU at a time, whatever its item)
-//   colq [item][band][column / 8 - 1][4 rows][32] float4 (q, q', s, s') of the column left of a group of 8
+//   row  [item][band][column][nl] float4 (h, h', a, a') of a band's last row (rolling: [team][column][32], one row
+//        per warp, or team of row workers, that is on the GPU at a time)
+//   colq [item][band][column / 8 - 1][4 rows][nl] float4 (q, q', s, s') of the column left of a group of 8
 //   cola the same, float2 (a, a')
-// (q = h - s; an item is a warp's 64 channels of one image and group.)
+// (q = h - s; an item is a warp's 64 channels of one image and group; nl: its pairs of channels, 32 but for a group's last.)
 //
 // Few items run with 2 or 4 row WORKERS per CTA of four warps: worker w takes every RW-th band, one step behind worker
 // w - 1; the CTA's warps then meet on its barrier once per step.
@@ -41,6 +41,7 @@ struct Pw {
     int nblk, nstrip, nsub, wp;   // bands; fetched blocks per band; groups of 8 columns; columns, even
     int period, rwl, npass;       // steps per band, log2 of the row workers, bands per worker
     int ntile, items, grid;       // warps' worth of channels per group; batch * G * ntile
+    int np;                       // pairs of channels per group
     unsigned flip_h, flip_w;
     int shared;                   // bit 0: u has dpg channels shared by the groups, bit 1: dout
     int fs, lin, el;              // columns of a fetched block; whole bands; element by element
@@ -64,6 +65,13 @@ template <int DT> struct pw_io {
     static constexpr int ES = DT == CS2D_F32 ? 4 : 2, FS = 32 / ES;   // FS: most columns of a fetched block
 };
 
+// 8 bytes that nothing in the kernel writes: zeros unless `on`
+__device__ __forceinline__ float2 pw_ld8(const void *p, bool on) {
+    float2 v;
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t@p ld.global.nc.v2.f32 {%0,%1}, [%2];\n\t}" : "=f"(v.x), "=f"(v.y) : "l"(p), "r"((int)on));
+    return v;
+}
+
 struct PwPos {   // position in a warp's stream of blocks
     int item, pass, strip, bg, g, tile;
     __device__ __forceinline__ void decode(const Pw &P) {
@@ -71,6 +79,8 @@ struct PwPos {   // position in a warp's stream of blocks
         g = bg % P.G;
         tile = item % P.ntile;
     }
+    __device__ __forceinline__ int pairs(const Pw &P) const { return min(32, P.np - 32 * tile); }
+    __device__ __forceinline__ int64_t first(const Pw &P) const { return (int64_t)bg * P.np + 32 * tile; }   // pairs of the items before this one
     __device__ __forceinline__ void next(const Pw &P, int stride) {
         if (++strip < P.period) return;
         strip = 0;

@@ -139,7 +139,7 @@ float *fp(const Tensor &t) { return given(t) ? t.data_ptr<float>() : nullptr; }
 std::pair<Tensor, Tensor> scan_forward(const Args &a, bool out_float, bool keep_state) {
     const auto ot = out_float ? at::kFloat : a.u.scalar_type();
     const cs2d_problem p = make_problem(a, ot, "selective_scan_fwd", false);
-    const size_t nbytes = keep_state ? cs2d_saved_bytes(&p) : cs2d_fwd_only_scratch_bytes(&p);
+    const size_t nbytes = keep_state ? cs2d_saved_bytes_dir(&p, nullptr) : cs2d_fwd_only_scratch_bytes_dir(&p, nullptr);
     CS2D_CHECK(nbytes != 0, "cs2d forward: ", cs2d_last_error());
     const c10::cuda::CUDAGuard guard(a.u.device());
     Tensor out = at::empty(a.u.sizes(), a.u.options().dtype(ot)), state = f32(a.u, (int64_t)(nbytes / 4));
@@ -230,7 +230,7 @@ Grads scan_backward(const Args &a, const Tensor &dout, const Tensor &state, cons
     CS2D_CHECK(inner_ok(dout), "dout must be contiguous in the last dimension");
     const cs2d_problem p = make_problem(a, dout.scalar_type(), "selective_scan_bwd", false);
     CS2D_CHECK(given(state), "the saved state x_v returned by fwd is required");
-    const size_t nbytes = cs2d_saved_bytes(&p);
+    const size_t nbytes = cs2d_saved_bytes_dir(&p, nullptr);
     CS2D_CHECK(nbytes != 0, "cs2d backward: ", cs2d_last_error());
     CS2D_CHECK(state.is_cuda() && state.scalar_type() == at::kFloat && state.is_contiguous() && state.numel() * 4 == (int64_t)nbytes,
                "x_v is not the saved state fwd returned for these inputs");
@@ -242,7 +242,7 @@ Grads scan_backward(const Args &a, const Tensor &dout, const Tensor &state, cons
     g.du = at::empty(a.u.sizes(), a.u.options());
     g.ddelta = at::empty(a.u.sizes(), a.u.options());
     const bool own = !param_grads.has_value();   // (a caller that brings its own buffer - the dispatcher operators - wants no shared storage)
-    BwdBuffers buf(a.B, own ? l.total : 0, cs2d_bwd_scratch_bytes(&p), own);
+    BwdBuffers buf(a.B, own ? l.total : 0, deterministic ? cs2d_bwd_scratch_bytes(&p) : cs2d_bwd_scratch_bytes_dir(&p, nullptr), own);
     Tensor flat = buf.params;
     if (!own) {
         flat = *param_grads;
@@ -298,7 +298,7 @@ std::pair<Tensor, Tensor> cross_forward(const Args &a, const Tensor &w, bool ser
     const cs2d_problem p = make_problem(a, at::kFloat, "cross_scan_fwd", true);
     const Tensor wf = w.to(at::kFloat).contiguous();
     const cs2d_dirs o = make_dirs(p.n_groups, 1, serial, wf, nullptr);
-    const size_t nbytes = keep_state ? cs2d_saved_bytes(&p) : cs2d_fwd_only_scratch_bytes(&p);
+    const size_t nbytes = keep_state ? cs2d_saved_bytes_dir(&p, &o) : cs2d_fwd_only_scratch_bytes_dir(&p, &o);
     CS2D_CHECK(nbytes != 0, "cs2d forward: ", cs2d_last_error());
     const c10::cuda::CUDAGuard guard(a.u.device());
     Tensor out = merged_image(a.u, serial), state = f32(a.u, (int64_t)(nbytes / 4));
@@ -314,12 +314,15 @@ Grads cross_backward(const Args &a, const Tensor &w, const Tensor &dy, const Ten
     const ParamLayout l = param_layout(dim, n, given(a.D), given(a.bias), given(a.decay));
     const c10::cuda::CUDAGuard guard(a.u.device());
     Grads g;
-    BwdBuffers buf(a.B, l.total + dim, cs2d_bwd_scratch_bytes(&p), true);   // the parameter gradients, then dw
+    cs2d_dirs o = make_dirs(p.n_groups, 3, serial, wf, nullptr);   // u and dy are shared by the directions
+    CS2D_CHECK(state.is_cuda() && state.scalar_type() == at::kFloat && state.is_contiguous() &&
+               state.numel() * 4 == (int64_t)cs2d_saved_bytes_dir(&p, &o), "the saved state is not the one the forward returned for these inputs");
+    BwdBuffers buf(a.B, l.total + dim, cs2d_bwd_scratch_bytes_dir(&p, &o), true);   // the parameter gradients, then dw
     g.dw = part_of(buf.params, l.total, w.sizes());
     param_views(g, buf.params, l, dim, n);
     Tensor du = merged_image(a.u, serial);
     g.ddelta = at::empty(a.delta.sizes(), a.delta.options());
-    const cs2d_dirs o = make_dirs(p.n_groups, 3, serial, wf, fp(g.dw));   // u and dy are shared by the directions
+    o.merge_dw = fp(g.dw);
     raise_on(cs2d_bwd_dir(&p, &o, dy.const_data_ptr(), dy.stride(0), dy.stride(1), dy.stride(2), state.const_data_ptr(), buf.scratch_ptr,
                           du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), buf.dB, buf.dC, fp(g.dD), fp(g.dbias), fp(g.ddecay),
                           stream_of(a.u)), "backward");

@@ -1,4 +1,5 @@
-"""Sizes of the buffers between the calls.  The built-in scratch array of ``cs2d_bwd_noalloc`` serves every problem whose
+"""Sizes of the buffers between the calls: those of the kernels that run, without places for states and channels that do not
+exist.  The built-in scratch array of ``cs2d_bwd_noalloc`` serves every problem whose
 adjoint rows fit it in the tile kernels' layout, whichever kernels run: those that keep a row per warp take as many CTAs as
 the array has rows for."""
 import ctypes
@@ -19,6 +20,56 @@ def _problem(batch, groups, d, n, h, w, dtype=_lib.BF16):
     for k in ("u", "delta", "A", "B", "C"):
         setattr(p, k, 16)  # never dereferenced: sizing only
     return p
+
+
+SIZES = ("cs2d_saved_bytes", "cs2d_bwd_scratch_bytes", "cs2d_fwd_only_scratch_bytes")
+
+
+def _sizes(p, dirs=None):
+    """(for this set of directions, for every set) of each buffer"""
+    o = ctypes.byref(dirs) if dirs is not None else None
+    return [(getattr(_lib.lib(), n + "_dir")(ctypes.byref(p), o), getattr(_lib.lib(), n)(ctypes.byref(p))) for n in SIZES]
+
+
+CORNERS = _lib.Dirs(0b1100, 0b1010, 3, 0, 16, None)
+SERIAL = _lib.Dirs(0b1100, 0b1010, 3, _lib.DIRS_SERIAL, 16, None)
+
+
+@pytest.mark.parametrize("n,w", [(1, 7), (1, 56), (1, 200), (2, 28), (3, 56), (16, 56), (16, 336)])
+@pytest.mark.parametrize("d", [7, 8, 192])
+def test_one_set_of_directions_needs_no_more_than_every_set(d, n, w):
+    for dirs in (None, CORNERS, SERIAL):
+        for exact, every in _sizes(_problem(2, 4, d, n, 20, w), dirs):
+            assert 0 < exact <= every
+
+
+def test_saved_state_of_the_kernels_that_run():
+    pixels = 8 * 64 * 8 * 100 * 100
+    exact, every = _sizes(_problem(8, 64, 8, 1, 100, 100))[0]
+    assert exact == 8 * 64 * 4 * 25 * 128 * 8          # streaming: channel pairs x row blocks x padded columns
+    assert every < 4 * pixels                          # pair-walk (corner directions): 3.5 bytes per channel and pixel
+    exact, _ = _sizes(_problem(32, 4, 192, 2, 28, 28))[0]
+    bc = 32 * 4 * 7 * 4 * 32 * 8 * 8                   # B and C of 8 state slots, in blocks of 32 pixels
+    assert exact == bc + (6 * 4 + 7 * 3) * 4 * (32 * 4 * 96 * 3) * 16   # rows and columns of two states, and a place for the other six
+
+
+def test_scratch_of_the_kernels_that_run():
+    assert _sizes(_problem(128, 4, 192, 1, 56, 56))[1][0] == 16        # streaming: the adjoint row stays on the chip
+    assert _sizes(_problem(32, 4, 192, 16, 56, 56, _lib.F32))[1][0] == 148 * 3 * 4 * 7 * 2048   # block-walk: 2 KB per warp and 8 columns
+
+
+def test_fake_saved_state_has_the_size_of_the_real_one():
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    import cs2d.library  # noqa: F401
+    with FakeTensorMode():
+        e = lambda *s: torch.empty(*s, dtype=torch.bfloat16, device="cuda")
+        A = torch.empty(96, 1, device="cuda")
+        for softplus in (True, False):      # pair-walk, streaming
+            _, saved = torch.ops.cs2d.scan_fwd(e(2, 96, 7, 7), e(2, 96, 7, 7), A, e(2, 2, 1, 7, 7), e(2, 2, 1, 7, 7), None, None,
+                                               softplus, False, None)
+            p = _problem(2, 2, 48, 1, 7, 7)
+            p.delta_softplus = softplus
+            assert saved.numel() * 4 == _lib.lib().cs2d_saved_bytes_dir(ctypes.byref(p), None)
 
 
 # (batch, groups, channels, states, rows, columns): at most 32 MiB of rows of 8 bytes per channel, state pair and column
