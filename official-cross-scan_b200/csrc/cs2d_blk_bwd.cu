@@ -418,9 +418,9 @@ __global__ void __launch_bounds__(BK_WARPS * 32, BkBwd<NG>::CTAS) blk_bwd_kernel
                 }
                 __syncwarp();
             }
-            if (blk > 0) {   // m of the block's first row
-                bk_st16(arow + 2 * k * 32, make_float4(mb[0].x, mb[0].y, mb[1].x, mb[1].y), mine);
-                bk_st16(arow + (2 * k + 1) * 32, make_float4(mb[2].x, mb[2].y, mb[3].x, mb[3].y), mine);
+            if (blk > 0) {   // m of the block's first row (lanes past the last slot write the zeros that they read above)
+                arow[2 * k * 32] = make_float4(mb[0].x, mb[0].y, mb[1].x, mb[1].y);
+                arow[(2 * k + 1) * 32] = make_float4(mb[2].x, mb[2].y, mb[3].x, mb[3].y);
             }
             if (non) copy_bc(nxt, k);
             // half a block's dB and dC onto the results: four columns at a time where the rows allow it, else one

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
         float4 *trow = nrow, *tcol = ncol;
         if (nxt.strip == 0) { if (non) place(nxt); }
         else { nbc += BK_PX * NG * 8; nrow += 4 * RL(); ncol += 4 * P.NL; }
-        const bool mine = pos.slot + sl_ < P.nsl;
+        const bool mine = !KEEP || pos.slot + sl_ < P.nsl;   // (rolling: every lane has a place)
         {
             const int ch0 = pos.slot * 2, cg = G0 * P.dpg + ch0, nch = P.dpg - ch0, r0 = blk * BK_R;
             const bool pix = r0 + lr < P.H && pos.strip * BK_S + lc < P.W;
