@@ -161,10 +161,17 @@ int cs2d_bwd(const cs2d_problem *p, const void *dout, int64_t dout_bs, int64_t d
  * parameter gradients still sum over channel tiles with atomics).
  */
 #define CS2D_DIRS_SERIAL 1
+/*
+ * CS2D_DIRS_TILE_STATE (forward, and then the backward of the same state): the forward writes the checkpoints
+ * that the deterministic backward reads.  Without it cs2d_bwd_det runs a second forward for them where
+ * cs2d_saved_bytes describes other checkpoints (and needs room for their result in its det_scratch).  cs2d_bwd_dir
+ * takes either state, by the same flag.  The results of the forward differ in the last bits.
+ */
+#define CS2D_DIRS_TILE_STATE 2
 typedef struct {
     uint32_t flip_rows_mask, flip_cols_mask;
     int32_t shared_input;
-    int32_t flags;           /* 0 or CS2D_DIRS_SERIAL (merge only) */
+    int32_t flags;           /* CS2D_DIRS_SERIAL (merge only), CS2D_DIRS_TILE_STATE */
     const float *merge_w;    /* NULL: no merge */
     float *merge_dw;
 } cs2d_dirs;
@@ -180,7 +187,8 @@ int cs2d_bwd_dir(const cs2d_problem *p, const cs2d_dirs *dirs, const void *dout,
 /*
  * Sizes for one set of directions and flags (dirs may be NULL): what the kernels that run for it use, where
  * cs2d_saved_bytes, cs2d_bwd_scratch_bytes and cs2d_fwd_only_scratch_bytes cover every set.  The scratch is that
- * of cs2d_bwd_dir (and of cs2d_bwd, for NULL); cs2d_bwd_det takes the covering size.
+ * of cs2d_bwd_dir (and of cs2d_bwd, for NULL); cs2d_bwd_det takes the covering size.  The saved states with and
+ * without CS2D_DIRS_TILE_STATE differ in size where they differ at all.
  */
 size_t cs2d_saved_bytes_dir(const cs2d_problem *p, const cs2d_dirs *dirs);
 size_t cs2d_bwd_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *dirs);
@@ -197,9 +205,11 @@ size_t cs2d_fwd_only_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *d
  * Results are ADDED to dA, dB, dC, dD, ddelta_bias, dA_decay exactly as in
  * cs2d_bwd (zero-fill them first).  dirs may be NULL.  Limits: ncols <= 256, and
  * for ncols > 64 dstate > 8; otherwise CS2D_ERR_UNSUPPORTED
- * (cs2d_bwd_det_scratch_bytes returns 0).
+ * (cs2d_bwd_det_scratch_bytes returns 0).  cs2d_bwd_det_scratch_bytes_dir: for one set of directions
+ * and flags, without room for a second forward's checkpoints where CS2D_DIRS_TILE_STATE says that it needs none.
  */
 size_t cs2d_bwd_det_scratch_bytes(const cs2d_problem *p);
+size_t cs2d_bwd_det_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *dirs);
 int cs2d_bwd_det(const cs2d_problem *p, const cs2d_dirs *dirs, const void *dout, int64_t dout_bs, int64_t dout_ds,
                  int64_t dout_hs, const void *saved, void *scratch, void *det_scratch, void *du, void *ddelta,
                  float *dA, float *dB, float *dC, float *dD, float *ddelta_bias, float *dA_decay, void *stream);

@@ -10,6 +10,7 @@ LIB_PATH = os.path.join(_HERE, "libcs2d.so")
 F32, F16, BF16 = 0, 1, 2
 NOALLOC_SCRATCH_BYTES = 32 << 20  # CS2D_NOALLOC_SCRATCH_BYTES
 DIRS_SERIAL = 1                   # CS2D_DIRS_SERIAL
+DIRS_TILE_STATE = 2               # CS2D_DIRS_TILE_STATE
 
 
 _i32, _i64, _p = ctypes.c_int32, ctypes.c_int64, ctypes.c_void_p
@@ -67,7 +68,8 @@ def lib():
         L.cs2d_bwd.restype = ctypes.c_int
         L.cs2d_bwd.argtypes = [ctypes.POINTER(Problem), vp, i64, i64, i64, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
         dp = ctypes.POINTER(Dirs)
-        for f in (L.cs2d_saved_bytes_dir, L.cs2d_bwd_scratch_bytes_dir, L.cs2d_fwd_only_scratch_bytes_dir):
+        for f in (L.cs2d_saved_bytes_dir, L.cs2d_bwd_scratch_bytes_dir, L.cs2d_fwd_only_scratch_bytes_dir,
+                  L.cs2d_bwd_det_scratch_bytes_dir):
             f.restype, f.argtypes = ctypes.c_size_t, [ctypes.POINTER(Problem), dp]
         L.cs2d_fwd_dir.restype = ctypes.c_int
         L.cs2d_fwd_dir.argtypes = [ctypes.POINTER(Problem), dp, vp, i64, i64, i64, vp, vp]

@@ -52,7 +52,8 @@ def _saved_numel(u, A, B, delta, delta_softplus, out_float, A_decay):
 def scan_fwd(u: Tensor, delta: Tensor, A: Tensor, B: Tensor, C: Tensor, D: Optional[Tensor],
              delta_bias: Optional[Tensor], delta_softplus: bool, out_float: bool,
              A_decay: Optional[Tensor]) -> Tuple[Tensor, Tensor]:
-    out, _, x_v, _ = ops.fwd(u, delta, A, B, C, D, delta_bias, delta_softplus, out_float, A_decay)
+    # (False: the size of the state must not depend on a mode that can change between tracing and running)
+    out, _, x_v, _ = _lib.native().fwd(u, delta, A, B, C, D, delta_bias, delta_softplus, out_float, A_decay, False)
     return out, x_v
 
 

@@ -101,8 +101,12 @@ def _raise_on(rc, what):
 
 
 def fwd(u, delta, A, B, C, D_=None, delta_bias_=None, delta_softplus=False, out_float=False, A_decay_=None):
-    """Selective nd scan forward.  Returns ``[out, x, x_v, x_sd]``."""
-    return _lib.native().fwd(u, delta, A, B, C, D_, delta_bias_, bool(delta_softplus), bool(out_float), A_decay_)
+    """Selective nd scan forward.  Returns ``[out, x, x_v, x_sd]``.
+
+    Under ``torch.use_deterministic_algorithms(True)`` the state is the one that the deterministic backward reads;
+    the kernels that write it differ from the others in the last bits of ``out``.
+    """
+    return _lib.native().fwd(u, delta, A, B, C, D_, delta_bias_, bool(delta_softplus), bool(out_float), A_decay_, None)
 
 
 def fwd_only(u, delta, A, B, C, D_=None, delta_bias_=None, delta_softplus=False, out_float=False, A_decay_=None):
@@ -146,7 +150,8 @@ def bwd(u, delta, A, B, C, D_, delta_bias_, dout, x_, x_v_, delta_softplus, A_de
 
     ``deterministic`` (default: ``torch.are_deterministic_algorithms_enabled()``)
     selects the backward without floating-point atomics (``cs2d_bwd_det``):
-    bit-identical gradients from run to run, for rows of at most 256 columns.
+    bit-identical gradients from run to run, for rows of at most 256 columns.  Where the forward did not know
+    (``fwd`` outside of that mode) it may run the forward again for the checkpoints it reads.
     """
     return _lib.native().bwd(u, delta, A, B, C, D_, delta_bias_, dout, x_v_, bool(delta_softplus), A_decay_, param_grads,
                              deterministic)

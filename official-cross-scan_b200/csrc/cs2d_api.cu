@@ -279,6 +279,12 @@ static Family family(const cs2d_problem *p, const cs2d_dirs *o);
 static bool walk_fwd_ok(const cs2d_problem *p, const cs2d_dirs *o);
 static bool pair_one(const cs2d_problem *p);
 static bool pair_dirs(const cs2d_problem *p);
+static bool tile_state(const cs2d_dirs *o) { return o && (o->flags & CS2D_DIRS_TILE_STATE); }   // the deterministic backward's checkpoints are wanted
+static cs2d_dirs with_tile_state(const cs2d_dirs *o, bool on) {
+    cs2d_dirs r = o ? *o : cs2d_dirs{};
+    r.flags = on ? r.flags | CS2D_DIRS_TILE_STATE : r.flags & ~CS2D_DIRS_TILE_STATE;
+    return r;
+}
 static int check_dirs(const cs2d_problem *p, const cs2d_dirs *o);
 static size_t stream_state_bytes(const cs2d_problem *p);
 static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o, bool backward);
@@ -366,7 +372,12 @@ static size_t exact_bytes(const cs2d_problem *p, const cs2d_dirs *o, Buffer what
     else if (f == TILE) n = layout_bytes(p, what, walk_fwd_ok(p, o));
     return std::max<size_t>(n, 16);
 }
-size_t cs2d_saved_bytes_dir(const cs2d_problem *p, const cs2d_dirs *o) { return exact_bytes(p, o, SAVED); }
+size_t cs2d_saved_bytes_dir(const cs2d_problem *p, const cs2d_dirs *o) {
+    const size_t n = exact_bytes(p, o, SAVED);
+    if (n == 0 || !tile_state(o)) return n;
+    const cs2d_dirs other = with_tile_state(o, false);   // two states of one problem never have the same size
+    return family(p, &other) != family(p, o) && exact_bytes(p, &other, SAVED) == n ? n + 16 : n;
+}
 size_t cs2d_bwd_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *o) { return exact_bytes(p, o, SCRATCH); }
 size_t cs2d_fwd_only_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *o) { return exact_bytes(p, o, ROLLING); }
 
@@ -435,7 +446,7 @@ static void stream_fill(Dev &d, const cs2d_problem *p, int *L, int *grid) {
 static bool walk_fwd_ok(const cs2d_problem *p, const cs2d_dirs *o) { return walk_shape(p) && !has_dirs(o); }
 
 // ---- block-walk kernels (cs2d_blk_fwd.cu, cs2d_blk_bwd.cu) -------------------------------------------
-static bool blk_ok(const cs2d_problem *p, const cs2d_dirs *o) { return blk_shape(p) && !dirs_serial(o); }
+static bool blk_ok(const cs2d_problem *p, const cs2d_dirs *o) { return blk_shape(p) && !dirs_serial(o) && !tile_state(o); }
 // the parts of the saved state (or of the forward-only scratch)
 static void blk_state(Blk &k, int NG, const void *saved, bool roll) {
     char *q = const_cast<char *>(static_cast<const char *>(saved));
@@ -511,7 +522,7 @@ static bool pair_one(const cs2d_problem *p) {    // streaming kernels
     return W < 16 || (W % 2 ? W <= 45 : W % 4 && W <= 24);
 }
 static bool pair_ok(const cs2d_problem *p, const cs2d_dirs *o) {
-    if (!pair_shape(p) || dirs_serial(o)) return false;
+    if (!pair_shape(p) || dirs_serial(o) || tile_state(o)) return false;
     return has_dirs(o) || p->ncols > 16 * STRIP ? pair_dirs(p) : pair_one(p);
 }
 static Family family(const cs2d_problem *p, const cs2d_dirs *o) {
@@ -599,7 +610,7 @@ static void pair_out(Pw &k, int es, int vout) {
 }
 
 static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_t out_bs, int64_t out_ds,
-                    int64_t out_hs, void *saved, void *stream, bool rolling = false, bool tile = false) {
+                    int64_t out_hs, void *saved, void *stream, bool rolling = false) {
     int rc = validate(p);
     if (rc) return rc;
     if ((rc = check_dirs(p, o))) return rc;
@@ -610,7 +621,8 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
     if (reinterpret_cast<uintptr_t>(saved) & 15) return fail(CS2D_ERR_INVALID, "saved must be 16-byte aligned");
     int *status = status_ptr();
     if (!status) return fail(CS2D_ERR_CUDA, "cannot locate the device status word");
-    if (!tile && pair_ok(p, o)) {
+    const Family fam = family(p, o);
+    if (fam == PAIR) {
         Pw k;
         pair_fill(k, p, o, false, out, out_bs, out_ds, out_hs);
         k.out = out; k.o_bs = out_bs; k.o_ds = out_ds; k.o_hs = out_hs;
@@ -623,7 +635,7 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
         g_launches.fetch_add(1);
         return CS2D_OK;
     }
-    if (stream_ok(p, o)) {
+    if (fam == STREAM) {
         Dev d;
         int L, grid;
         stream_fill(d, p, &L, &grid);
@@ -639,7 +651,7 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
         g_launches.fetch_add(1);
         return CS2D_OK;
     }
-    if (!tile && blk_ok(p, o)) {
+    if (fam == BLK) {
         Blk k;
         int NG;
         blk_fill(k, NG, p, o, false);
@@ -748,7 +760,7 @@ static cudaError_t launch_sum(float *out, const float *part, int64_t n, int coun
 
 // layout of the deterministic backward's scratch, in floats
 struct DetLayout { int64_t nB, dB, dC, dA, dD, dbias, ddecay, state, total; int ntiles, grid, zero; };
-static int det_layout(const cs2d_problem *p, DetLayout *l) {
+static int det_layout(const cs2d_problem *p, DetLayout *l, bool remake) {   // remake: room for the checkpoints, made again
     if (n_tiles(p->ncols) > 1)
         return fail(CS2D_ERR_UNSUPPORTED, "the deterministic backward covers ncols <= %d", kTileCols);
     TileView tv;
@@ -766,8 +778,8 @@ static int det_layout(const cs2d_problem *p, DetLayout *l) {
     l->dB = 0; l->dC = l->dB + l->ntiles * l->nB; l->dA = l->dC + l->ntiles * l->nB;
     l->dD = l->dA + (int64_t)p->batch * p->dim * p->dstate; l->dbias = l->dD + (int64_t)p->batch * p->dim;
     l->ddecay = l->dbias + (int64_t)p->batch * p->dim; l->total = l->ddecay + l->grid;
-    l->state = (l->total + 3) & ~int64_t(3);   // problems of the block-walk and pair-walk kernels: other kernels' checkpoints
-    if (blk_shape(p) || pair_shape(p)) l->total = l->state + (int64_t)(layout_bytes(p, SAVED, walk_shape(p)) / 4);
+    l->state = (l->total + 3) & ~int64_t(3);
+    if (remake) l->total = l->state + (int64_t)(layout_bytes(p, SAVED, walk_shape(p)) / 4);
     return CS2D_OK;
 }
 
@@ -789,7 +801,9 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
     if (rc) return rc;
     if ((rc = check_dirs(p, o))) return rc;
     DetLayout dl = {};
-    if (det && (rc = det_layout(p, &dl))) return rc;
+    const Family fam = family(p, o);
+    const bool remake = det && (fam == BLK || fam == PAIR);
+    if (det && (rc = det_layout(p, &dl, remake))) return rc;
     const bool dirs = has_dirs(o);
     if (o && o->merge_w && (det || !(o->shared_input & 2)))
         return fail(CS2D_ERR_INVALID, "the direction merge needs the shared gradient image (shared_input bit 1) "
@@ -801,7 +815,7 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
     if (dA_decay && !p->A_decay) return fail(CS2D_ERR_INVALID, "dA_decay requested without A_decay");
     int *status = status_ptr();
     if (!status) return fail(CS2D_ERR_CUDA, "cannot locate the device status word");
-    if (!det && pair_ok(p, o)) {
+    if (!det && fam == PAIR) {
         Pw k;
         pair_fill(k, p, o, true, dout, dout_bs, dout_ds, dout_hs);
         pair_state(k, saved);
@@ -818,7 +832,7 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
         g_launches.fetch_add(1);
         return CS2D_OK;
     }
-    if (!det && blk_ok(p, o)) {
+    if (!det && fam == BLK) {
         Blk k;
         int NG;
         blk_fill(k, NG, p, o, true);
@@ -833,17 +847,18 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
         g_launches.fetch_add(1);
         return CS2D_OK;
     }
-    if (det && (blk_ok(p, o) || pair_ok(p, o))) {
-        // The deterministic backward is the tile kernels'; the checkpoints it reads are made again (y goes to du, which is
-        // written later).
+    const cs2d_dirs tile = with_tile_state(o, true);
+    if (remake) {
+        // The deterministic backward is the tile kernels'; a forward that did not know of it (CS2D_DIRS_TILE_STATE) is made
+        // again for the checkpoints (y goes to du, which is written later).
         cs2d_problem q = *p;
         q.out_dtype = p->io_dtype;
         void *st = det + dl.state;
-        if ((rc = fwd_impl(&q, o, du, (int64_t)p->dim * p->nrows * p->ncols, (int64_t)p->nrows * p->ncols, p->ncols, st, stream, false, true)))
+        if ((rc = fwd_impl(&q, &tile, du, (int64_t)p->dim * p->nrows * p->ncols, (int64_t)p->nrows * p->ncols, p->ncols, st, stream)))
             return rc;
         saved = st;
     }
-    const bool streamed = stream_ok(p, o);   // the forward of this problem ran on the streaming kernel
+    const bool streamed = family(p, remake ? &tile : o) == STREAM;   // the checkpoints are the streaming kernel's
     if (streamed && !det) {
         Dev d;
         int L, grid;
@@ -943,7 +958,14 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
 
 size_t cs2d_bwd_det_scratch_bytes(const cs2d_problem *p) {
     DetLayout dl = {};
-    if (validate(p) != CS2D_OK || det_layout(p, &dl) != CS2D_OK) return 0;
+    if (validate(p) != CS2D_OK || det_layout(p, &dl, blk_shape(p) || pair_shape(p)) != CS2D_OK) return 0;
+    return (size_t)dl.total * sizeof(float);
+}
+size_t cs2d_bwd_det_scratch_bytes_dir(const cs2d_problem *p, const cs2d_dirs *o) {
+    DetLayout dl = {};
+    if (validate(p) != CS2D_OK || check_dirs(p, o) != CS2D_OK) return 0;
+    const Family f = family(p, o);
+    if (det_layout(p, &dl, f == BLK || f == PAIR) != CS2D_OK) return 0;
     return (size_t)dl.total * sizeof(float);
 }
 

@@ -136,14 +136,17 @@ Tensor zeros_f32(const Tensor &like, int64_t n) {
 float *fp(const Tensor &t) { return given(t) ? t.data_ptr<float>() : nullptr; }
 
 // ---- forward ---------------------------------------------------------------------------------------
-std::pair<Tensor, Tensor> scan_forward(const Args &a, bool out_float, bool keep_state) {
+// deterministic: a deterministic backward will read the state, which is then the one that it takes without a second forward
+std::pair<Tensor, Tensor> scan_forward(const Args &a, bool out_float, bool keep_state, bool deterministic) {
     const auto ot = out_float ? at::kFloat : a.u.scalar_type();
     const cs2d_problem p = make_problem(a, ot, "selective_scan_fwd", false);
-    const size_t nbytes = keep_state ? cs2d_saved_bytes_dir(&p, nullptr) : cs2d_fwd_only_scratch_bytes_dir(&p, nullptr);
+    cs2d_dirs o{};
+    if (deterministic && keep_state && cs2d_bwd_det_scratch_bytes_dir(&p, nullptr) != 0) o.flags = CS2D_DIRS_TILE_STATE;
+    const size_t nbytes = keep_state ? cs2d_saved_bytes_dir(&p, &o) : cs2d_fwd_only_scratch_bytes_dir(&p, nullptr);
     CS2D_CHECK(nbytes != 0, "cs2d forward: ", cs2d_last_error());
     const c10::cuda::CUDAGuard guard(a.u.device());
     Tensor out = at::empty(a.u.sizes(), a.u.options().dtype(ot)), state = f32(a.u, (int64_t)(nbytes / 4));
-    const int rc = keep_state ? cs2d_fwd(&p, out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), state.data_ptr(), stream_of(a.u))
+    const int rc = keep_state ? cs2d_fwd_dir(&p, &o, out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), state.data_ptr(), stream_of(a.u))
                               : cs2d_fwd_only(&p, nullptr, out.data_ptr(), out.stride(0), out.stride(1), out.stride(2),
                                               state.data_ptr(), stream_of(a.u));
     raise_on(rc, "forward");
@@ -230,9 +233,12 @@ Grads scan_backward(const Args &a, const Tensor &dout, const Tensor &state, cons
     CS2D_CHECK(inner_ok(dout), "dout must be contiguous in the last dimension");
     const cs2d_problem p = make_problem(a, dout.scalar_type(), "selective_scan_bwd", false);
     CS2D_CHECK(given(state), "the saved state x_v returned by fwd is required");
-    const size_t nbytes = cs2d_saved_bytes_dir(&p, nullptr);
+    cs2d_dirs o{};
+    const size_t nbytes = cs2d_saved_bytes_dir(&p, &o);
     CS2D_CHECK(nbytes != 0, "cs2d backward: ", cs2d_last_error());
-    CS2D_CHECK(state.is_cuda() && state.scalar_type() == at::kFloat && state.is_contiguous() && state.numel() * 4 == (int64_t)nbytes,
+    if (state.numel() * 4 != (int64_t)nbytes) o.flags = CS2D_DIRS_TILE_STATE;   // written for a deterministic backward
+    CS2D_CHECK(state.is_cuda() && state.scalar_type() == at::kFloat && state.is_contiguous() &&
+               state.numel() * 4 == (int64_t)(o.flags ? cs2d_saved_bytes_dir(&p, &o) : nbytes),
                "x_v is not the saved state fwd returned for these inputs");
     const int64_t dim = p.dim, n = p.dstate;
     const ParamLayout l = param_layout(dim, n, given(a.D), given(a.bias), given(a.decay));
@@ -242,7 +248,7 @@ Grads scan_backward(const Args &a, const Tensor &dout, const Tensor &state, cons
     g.du = at::empty(a.u.sizes(), a.u.options());
     g.ddelta = at::empty(a.u.sizes(), a.u.options());
     const bool own = !param_grads.has_value();   // (a caller that brings its own buffer - the dispatcher operators - wants no shared storage)
-    BwdBuffers buf(a.B, own ? l.total : 0, deterministic ? cs2d_bwd_scratch_bytes(&p) : cs2d_bwd_scratch_bytes_dir(&p, nullptr), own);
+    BwdBuffers buf(a.B, own ? l.total : 0, deterministic ? cs2d_bwd_scratch_bytes(&p) : cs2d_bwd_scratch_bytes_dir(&p, &o), own);
     Tensor flat = buf.params;
     if (!own) {
         flat = *param_grads;
@@ -251,14 +257,14 @@ Grads scan_backward(const Args &a, const Tensor &dout, const Tensor &state, cons
     }
     param_views(g, flat, l, dim, n);
     if (deterministic) {
-        const size_t ndet = cs2d_bwd_det_scratch_bytes(&p);
+        const size_t ndet = cs2d_bwd_det_scratch_bytes_dir(&p, &o);
         CS2D_CHECK(ndet != 0, "cs2d backward has no deterministic implementation for this shape: ", cs2d_last_error());
         const Tensor det = f32(a.u, (int64_t)(ndet / 4));
-        raise_on(cs2d_bwd_det(&p, nullptr, dout.const_data_ptr(), dout.stride(0), dout.stride(1), dout.stride(2), state.const_data_ptr(),
+        raise_on(cs2d_bwd_det(&p, &o, dout.const_data_ptr(), dout.stride(0), dout.stride(1), dout.stride(2), state.const_data_ptr(),
                               buf.scratch_ptr, det.data_ptr(), g.du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), buf.dB, buf.dC,
                               fp(g.dD), fp(g.dbias), fp(g.ddecay), st), "backward");
     } else {
-        raise_on(cs2d_bwd(&p, dout.const_data_ptr(), dout.stride(0), dout.stride(1), dout.stride(2), state.const_data_ptr(),
+        raise_on(cs2d_bwd_dir(&p, &o, dout.const_data_ptr(), dout.stride(0), dout.stride(1), dout.stride(2), state.const_data_ptr(),
                           buf.scratch_ptr, g.du.data_ptr(), g.ddelta.data_ptr(), fp(g.dA), buf.dB, buf.dC, fp(g.dD), fp(g.dbias),
                           fp(g.ddecay), st), "backward");
     }
@@ -343,7 +349,7 @@ struct ScanFunction : torch::autograd::Function<ScanFunction> {
     static Tensor forward(AutogradContext *ctx, const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor &B, const Tensor &C,
                           const OptT &D, const OptT &bias, const OptT &decay, bool softplus, bool out_float) {
         at::AutoDispatchBelowADInplaceOrView below;
-        auto r = scan_forward(Args{u, delta, A, B, C, opt(D), opt(bias), opt(decay), softplus}, out_float, true);
+        auto r = scan_forward(Args{u, delta, A, B, C, opt(D), opt(bias), opt(decay), softplus}, out_float, true, deterministic_mode());
         ctx->saved_data["softplus"] = softplus;
         ctx->save_for_backward({u, delta, A, B, C, opt(D), opt(bias), opt(decay), r.second});
         return r.first;
@@ -390,15 +396,15 @@ Args args_of(const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor
 }
 
 std::vector<Tensor> py_fwd(const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor &B, const Tensor &C, const OptT &D,
-                           const OptT &bias, bool softplus, bool out_float, const OptT &decay) {
+                           const OptT &bias, bool softplus, bool out_float, const OptT &decay, const std::optional<bool> &deterministic) {
     at::NoGradGuard no_grad;
-    auto r = scan_forward(args_of(u, delta, A, B, C, D, bias, softplus, decay), out_float, true);
+    auto r = scan_forward(args_of(u, delta, A, B, C, D, bias, softplus, decay), out_float, true, deterministic.value_or(deterministic_mode()));
     return {r.first, f32(u, 0), r.second, f32(u, 0)};
 }
 Tensor py_fwd_only(const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor &B, const Tensor &C, const OptT &D,
                    const OptT &bias, bool softplus, bool out_float, const OptT &decay) {
     at::NoGradGuard no_grad;
-    return scan_forward(args_of(u, delta, A, B, C, D, bias, softplus, decay), out_float, false).first;
+    return scan_forward(args_of(u, delta, A, B, C, D, bias, softplus, decay), out_float, false, false).first;
 }
 std::vector<OptT> py_bwd(const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor &B, const Tensor &C, const OptT &D,
                          const OptT &bias, const Tensor &dout, const OptT &state, bool softplus, const OptT &decay,
@@ -413,7 +419,7 @@ std::vector<OptT> py_bwd(const Tensor &u, const Tensor &delta, const Tensor &A, 
 Tensor py_scan(const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor &B, const Tensor &C, const OptT &D, const OptT &bias,
                bool softplus, bool out_float, const OptT &decay) {
     const Args a = args_of(u, delta, A, B, C, D, bias, softplus, decay);
-    if (!any_grad(a)) return scan_forward(a, out_float, false).first;   // nothing can ask for a gradient: no saved state
+    if (!any_grad(a)) return scan_forward(a, out_float, false, false).first;   // nothing can ask for a gradient: no saved state
     return ScanFunction::apply(u, delta, A, B, C, D, bias, decay, softplus, out_float);
 }
 Tensor py_cross(const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor &B, const Tensor &C, const Tensor &w, const OptT &D,

@@ -58,6 +58,52 @@ def test_scratch_of_the_kernels_that_run():
     assert _sizes(_problem(32, 4, 192, 16, 56, 56, _lib.F32))[1][0] == 148 * 3 * 4 * 7 * 2048   # block-walk: 2 KB per warp and 8 columns
 
 
+TILE = _lib.Dirs(0, 0, 0, _lib.DIRS_TILE_STATE, None, None)
+
+
+@pytest.mark.parametrize("d,n,h,w", [(192, 16, 56, 56), (40, 16, 14, 14), (192, 4, 28, 28), (8, 2, 3, 5), (192, 1, 7, 7), (192, 1, 56, 56), (4, 16, 9, 9)])
+def test_state_of_the_deterministic_backward(d, n, h, w):
+    """It has another size wherever it is another state, and the scratch then has no room for a second forward's."""
+    L, p = _lib.lib(), _problem(2, 4, d, n, h, w)
+    state, tile = _sizes(p)[0][0], _sizes(p, TILE)[0][0]
+    det = [L.cs2d_bwd_det_scratch_bytes_dir(ctypes.byref(p), o) for o in (None, ctypes.byref(TILE))]
+    remade = d >= 8 and (n > 1 or w == 7)
+    assert 0 < det[1] <= det[0] <= L.cs2d_bwd_det_scratch_bytes(ctypes.byref(p))
+    assert (state != tile) == remade and (det[0] > det[1]) == remade
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2, 2, 16, 16, 9, 14), (1, 2, 14, 16, 13, 56), (2, 1, 9, 4, 11, 30), (1, 2, 10, 16, 6, 100), (2, 2, 33, 1, 9, 7)], ids=str)
+def test_deterministic_step_runs_one_forward(shape):
+    """The forward of a deterministic step writes the checkpoints that its backward reads: the launches of the backward and
+    its sums only, the bits of the backward that makes them again, and a state that the other backward takes as well."""
+    d = {k: v.cuda() for k, v in make_inputs(*shape, dtype=torch.float32, seed=3).items() if v is not None}
+    names = ("u", "delta", "A", "B", "C", "D", "delta_bias")
+    a = [d[k] for k in names]
+    o = cs2d.fwd(*a, True, False, None)
+    remade = cs2d.bwd(*a, d["dout"], o[1], o[2], True, None, o[3], deterministic=True)
+    leaves = [t.clone().requires_grad_(True) for t in a]
+    torch.use_deterministic_algorithms(True)
+    try:
+        y = cs2d.selective_scan_2d(*leaves, True)
+        before = cs2d.launch_count()
+        grads = torch.autograd.grad(y, leaves, d["dout"])
+        assert cs2d.launch_count() - before == 6       # the backward, and the sums of dB, dC, dA, dD, ddelta_bias
+        od = cs2d.fwd(*a, True, False, None)
+        pair = cs2d.bwd(*a, d["dout"], od[1], od[2], True, None, od[3])
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert od[2].numel() != o[2].numel()
+    for g, p, r in zip(grads, pair, remade):
+        assert torch.equal(g, r) and torch.equal(p, r)
+    rtol, atol = TOL["float32"]
+    check_close("out", y.detach().cpu().numpy(), o[0].cpu().numpy(), rtol, atol)
+    mixed = cs2d.bwd(*a, d["dout"], od[1], od[2], True, None, od[3], deterministic=False)
+    for k, x, r in zip(names, mixed, remade):
+        check_close("d" + k, x.cpu().numpy(), r.cpu().numpy(), rtol, atol * 10)   # two orders of summation
+    assert cs2d.device_status() == 0
+
+
 def test_fake_saved_state_has_the_size_of_the_real_one():
     from torch._subclasses.fake_tensor import FakeTensorMode
     import cs2d.library  # noqa: F401
