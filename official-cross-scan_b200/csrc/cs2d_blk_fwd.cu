@@ -47,8 +47,7 @@ struct BkFwd {   // a warp's shared memory
     static constexpr int total = (top + SPW * 9 * 8 + 15) & ~15;
 };
 
-// HALF: the last block of a row has its left half only, whose right half is left out
-template <int NG, int DT, bool KEEP, bool HALF>
+template <int NG, int DT, bool KEEP>
 __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_constant__ Blk P) {
     using S = BkFwd<NG>;
     using T = typename bk_type<DT>::t;
@@ -65,7 +64,6 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
     const int first = blockIdx.x * nsub, lmax = (P.items - first + stride - 1) / stride * P.npass * P.period;
     const int steps = lmax + BK_LAG * (rw - 1);
     const bool softplus = P.softplus != 0, drep1 = P.drep == 1;
-    const bool chain = P.nstrip == 1 && rw == 1;           // the next block is always the one below
     const float2 lgd = bc(P.decay ? log2f(__ldg(P.decay)) : 0.f);
 
     BkPos pos;
@@ -125,9 +123,8 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
 
     float2 A2 = bc(0.f), hcorner = bc(0.f);
     float2 hl[BK_R], al[BK_R], ql[BK_R], sl[BK_R];         // column left of the block
-    float2 hup[BK_S];                                      // the row of h above the block; hcorner: its value left of the current column
-#pragma unroll
-    for (int c = 0; c < BK_S; ++c) hup[c] = bc(0.f);
+    float4 up0, up1;                                       // the row of h above: of the next quarter block and the one after it; hcorner: left of the current column
+    up0 = up1 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int r = 0; r < BK_R; ++r) { hl[r] = al[r] = ql[r] = sl[r] = bc(0.f); }
     int64_t oo = 0;
@@ -144,23 +141,13 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
         else nrow = P.row + (int64_t)(first + (warp >> P.rwl)) * P.nstrip * 4 * 32 + lane;   // (an item's first row of blocks reads nothing)
         ncol = P.col + ((int64_t)blk * (P.nstrip - 1) - 1) * 4 * P.NL + lin;
     };
-    // half k of the row of h above block `q`, whose row of h goes to nrow
-    auto fetch = [&](const BkPos &q, int k) {
-        const bool there = q.pass * rw + w > 0;
-        const float4 *src = nrow - up + 2 * k * RL();
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if constexpr (NG == 16 || !KEEP) v = bk_ld16<false>(src + i * RL(), there);   // (8 slots, KEEP: 2 to 10 % slower than the branch)
-            else if (there) v = src[i * RL()];
-            hup[4 * k + 2 * i] = f2(v.x, v.y); hup[4 * k + 2 * i + 1] = f2(v.z, v.w);
-        }
-    };
+    auto above = [&](const float4 *row, int qt, bool there) { return bk_ld16<false>(row - up + qt * RL(), there); };   // a quarter of the row above the one at `row`
     auto enter = [&](const BkPos &q) {   // the first block after a pause: everything its predecessor would have started
         place(q);
         load_raw(q);
         copy_bc(nbc, 0, true); copy_bc(nbc, 1, true); copy_bc(nbc, 2, true);
-        if (!chain) { fetch(q, 0); fetch(q, 1); }
+        const bool there = q.pass * rw + w > 0;
+        up0 = above(nrow, 0, there); up1 = above(nrow, 1, there);
     };
     if (w == 0 && live(pos, 0)) enter(pos);
     for (int g = 0; g < steps; ++g) {
@@ -229,63 +216,63 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
         }
         __syncwarp();
         if (non) load_raw(nxt);
-        // Software pipeline over the block's pixels (column by column): the shared-memory loads of a pixel are issued two
-        // pixels ahead, its exponential and products one ahead.
+        // Two columns - a quarter block - at a time; quarters that the image does not have are left out.  Software pipeline over
+        // their pixels (column by column): the shared-memory loads of a pixel are issued two pixels ahead.  Only two quarters of the
+        // row of h above are held (the whole of it, and instances that left out the right half of a row's last block, spilled 36
+        // to 352 bytes): 32x4x192x16x56x56 fp32 forward 1355 -> 1218 us, 128x4x384x16x28x28 bf16 3057 -> 2480, and without a backward
+        // 64x4x768x16x10x10 bf16 550 -> 446, 4x4x192x16x56x56 bf16 210 -> 192.  Not unrolled it is the slower one (1500 us; by halves
+        // 1298), and so is a test per column (1394).
         const float4 *tIn = sIn + sl_ * 33;
         const float2 *tTop = sTop + sl_ * 9;
+        const bool nthere = non && nxt.pass * rw + w > 0;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const bool there = !HALF || k == 0 || pos.strip * BK_S + 4 < P.W;   // the image has this half of the block
-            float2 hb[4];
-            if constexpr (HALF) hb[0] = hb[1] = hb[2] = hb[3] = bc(0.f);
+        for (int qt = 0; qt < 4; ++qt) {
+            bk_wait<2>();
+            __syncwarp();   // this quarter's B and C are here, the quarter before it has been read by all lanes
+            copy_bc(qt == 0 ? tbc : nbc, (qt + 3) & 3, qt == 0 || non);
+            // The row of h above travels two quarters ahead.  What a load reads was written two quarters (by this thread) or at least two
+            // steps ago (by another worker).
+            const float4 hup = up0;
+            up0 = up1;
+            up1 = qt < 2 ? above(trow, qt + 2, blk > 0) : above(nrow, qt - 2, nthere);
+            if (pos.strip * BK_S + 2 * qt < P.W) {
+                const float4 *qIn = tIn + qt * 2;
+                const float2 *tBC = sBC + qt * 8 * NG + (NG == 16 ? (n & 7) * 2 + (n >> 3) : n);
+                float2 *qY = sY + (qt & 1) * 2 * YP + lane;
+                float4 rin[2];
+                float2 rbc[2], hb[2];
+                float2 hd, hu, au;
 #pragma unroll
-            for (int qt = 2 * k; qt < 2 * k + 2; ++qt) {
-                bk_wait<2>();
-                __syncwarp();   // this quarter's B and C are here, the quarter before it has been read by all lanes
-                copy_bc(qt == 0 ? tbc : nbc, (qt + 3) & 3, qt == 0 || non);
-                if (there) {
-                    const float2 *tBC = sBC + qt * 8 * NG + (NG == 16 ? (n & 7) * 2 + (n >> 3) : n);
-                    float4 rin[2];
-                    float2 rbc[2];
-                    float2 hd, hu, au;
+                for (int x = 0; x < 2; ++x) { rin[x] = qIn[x * BK_S]; rbc[x] = tBC[x * NG]; }
 #pragma unroll
-                    for (int x = 0; x < 2; ++x) { rin[x] = tIn[(x % 4) * BK_S + qt * 2 + x / 4]; rbc[x] = tBC[x * NG]; }
-#pragma unroll
-                    for (int x = 0; x < 8; ++x) {
-                        const int c = qt * 2 + x / 4, r = x % 4, cc = c & 3;
-                        const float4 in = rin[x & 1];
-                        const float2 b = rbc[x & 1];
-                        if (x + 2 < 8) { rin[x & 1] = tIn[((x + 2) % 4) * BK_S + qt * 2 + (x + 2) / 4]; rbc[x & 1] = tBC[(x + 2) * NG]; }
-                        if (r == 0) { hd = hcorner; hu = hcorner = hup[c]; au = blk > 0 ? ex2_2(fma2(tTop[c], A2, lgd)) : bc(0.f); }
-                        const float2 a = ex2_2(fma2(f2(in.x, in.y), A2, lgd));
-                        const float2 p = mul2(bc(b.x), f2(in.z, in.w));
-                        const float2 t = mul2(add2(au, al[r]), hd);
-                        const float2 z = add2(ql[r], fma2(t, bc(-0.5f), hu));
-                        const float2 s = fma2(a, sl[r], p);
-                        const float2 q = mul2(a, z), h = fma2(a, z, s);
-                        sY[(r * 4 + cc) * YP + lane] = mul2(bc(b.y), fma2(p, bc(0.25f), q));
-                        hd = hl[r]; hu = h; au = a;
-                        hl[r] = h; al[r] = a; ql[r] = q; sl[r] = s;
-                        if (r == BK_R - 1) hb[cc] = h;
-                    }
+                for (int x = 0; x < 8; ++x) {
+                    const int c = x / 4, r = x % 4;
+                    const float4 in = rin[x & 1];
+                    const float2 b = rbc[x & 1];
+                    if (x + 2 < 8) { rin[x & 1] = qIn[((x + 2) % 4) * BK_S + (x + 2) / 4]; rbc[x & 1] = tBC[(x + 2) * NG]; }
+                    if (r == 0) { hd = hcorner; hu = hcorner = c ? f2(hup.z, hup.w) : f2(hup.x, hup.y); au = blk > 0 ? ex2_2(fma2(tTop[qt * 2 + c], A2, lgd)) : bc(0.f); }
+                    const float2 a = ex2_2(fma2(f2(in.x, in.y), A2, lgd));
+                    const float2 p = mul2(bc(b.x), f2(in.z, in.w));
+                    const float2 t = mul2(add2(au, al[r]), hd);
+                    const float2 z = add2(ql[r], fma2(t, bc(-0.5f), hu));
+                    const float2 s = fma2(a, sl[r], p);
+                    const float2 q = mul2(a, z), h = fma2(a, z, s);
+                    qY[(r * 4 + c) * YP] = mul2(bc(b.y), fma2(p, bc(0.25f), q));
+                    hd = hl[r]; hu = h; au = a;
+                    hl[r] = h; al[r] = a; ql[r] = q; sl[r] = s;
+                    if (r == BK_R - 1) hb[c] = h;
                 }
+                bk_st16(trow + qt * RL(), make_float4(hb[0].x, hb[0].y, hb[1].x, hb[1].y), mine && blk + 1 < P.nblk);   // the block's last row of h
+            } else if (KEEP && pos.strip * BK_S + 4 * (qt >> 1) < P.W) {   // (the backward recomputes whole halves)
+                bk_st16(trow + qt * RL(), make_float4(0.f, 0.f, 0.f, 0.f), mine && blk + 1 < P.nblk);
             }
-            if (blk + 1 < P.nblk && there) {   // the block's last row of h
-                bk_st16(trow + 2 * k * RL(), make_float4(hb[0].x, hb[0].y, hb[1].x, hb[1].y), mine);
-                bk_st16(trow + (2 * k + 1) * RL(), make_float4(hb[2].x, hb[2].y, hb[3].x, hb[3].y), mine);
-            }
-            // Half k of the row of h above the next block into the registers of half k of this one's, which are done with: the
-            // loads travel while the other half is computed.  What they read was written at least two steps ago.
-            if (chain) {   // the block below is next
-#pragma unroll
-                for (int cc = 0; cc < 4; ++cc) hup[k * 4 + cc] = nxt.pass > 0 ? hb[cc] : bc(0.f);
-            } else if (non) {
-                fetch(nxt, k);
-            }
+            if (!(qt & 1)) continue;
+            const int k = qt >> 1, c0 = pos.strip * BK_S + k * 4;
+            if (c0 >= P.W) continue;
             __syncwarp();
-            if (there) {   // sums over the states of half a block: a lane takes one pixel of every second slot
+            {   // sums over the states of half a block: a lane takes one pixel of every second slot
                 const bool fw = (P.flip_w >> G0) & 1u;
-                const int px = lane & 15, c0 = pos.strip * BK_S + k * 4, nch = P.dpg - pos.slot * 2 - 2 * (lane >> 4);
+                const int px = lane & 15, nch = P.dpg - pos.slot * 2 - 2 * (lane >> 4);
                 const bool okp = blk * BK_R + (px >> 2) < P.H && c0 + (px & 3) < P.W;
                 const int64_t o = oo + (fw ? -c0 : c0);
 #pragma unroll
@@ -322,9 +309,9 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
     bk_wait<0>();
 }
 
-template <int NG, int DT, bool KEEP, bool HALF>
+template <int NG, int DT, bool KEEP>
 static cudaError_t launch(const Blk &P, cudaStream_t st) {
-    auto kernel = blk_fwd_kernel<NG, DT, KEEP, HALF>;
+    auto kernel = blk_fwd_kernel<NG, DT, KEEP>;
     constexpr int smem = BkFwd<NG>::total * BK_WARPS;
     static bool attr_done[64] = {};
     int dev = 0;
@@ -339,17 +326,13 @@ static cudaError_t launch(const Blk &P, cudaStream_t st) {
     return cudaGetLastError();
 }
 template <int NG, int DT>
-static cudaError_t launch_half(const Blk &P, cudaStream_t st) {
-    const bool half = ((P.W - 1) & 7) < 4;   // columns in the last block: at most 4
-    if (P.roll) return half ? launch<NG, DT, false, true>(P, st) : launch<NG, DT, false, false>(P, st);
-    return half ? launch<NG, DT, true, true>(P, st) : launch<NG, DT, true, false>(P, st);
-}
+static cudaError_t launch_keep(const Blk &P, cudaStream_t st) { return P.roll ? launch<NG, DT, false>(P, st) : launch<NG, DT, true>(P, st); }
 template <int NG>
 static cudaError_t launch_dt(const Blk &P, cudaStream_t st) {
     switch (P.io_dt) {
-        case CS2D_F32: return launch_half<NG, CS2D_F32>(P, st);
-        case CS2D_F16: return launch_half<NG, CS2D_F16>(P, st);
-        default: return launch_half<NG, CS2D_BF16>(P, st);
+        case CS2D_F32: return launch_keep<NG, CS2D_F32>(P, st);
+        case CS2D_F16: return launch_keep<NG, CS2D_F16>(P, st);
+        default: return launch_keep<NG, CS2D_BF16>(P, st);
     }
 }
 

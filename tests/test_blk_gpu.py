@@ -62,6 +62,23 @@ def test_block_walk_against_oracle(shape, dtype, kw, det):
     assert cs2d.device_status() == 0
 
 
+@pytest.mark.parametrize("w", [1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 13, 15, 17])
+@pytest.mark.parametrize("n", [3, 16])
+def test_every_number_of_columns_in_the_last_block(n, w):
+    """The forward leaves out the pairs of columns that a row's last block does not have, the backward its right half."""
+    inp = make_inputs(2, 1, 9, n, 9, w, dtype=torch.float32, seed=w)
+    d = _dev(inp)
+    args = (d["u"], d["delta"], d["A"], d["B"], d["C"], d["D"], d["delta_bias"])
+    out, x, xv, xsd = cs2d.fwd(*args, True, False, None)
+    g = cs2d.bwd(*args, d["dout"], x, xv, True, None, xsd)
+    assert torch.equal(cs2d.fwd_only(*args, True, False, None), out)
+    yo, go = _oracle(inp)
+    check_close("out", out.cpu().numpy(), yo, *TOL["float32"])
+    for name, t in zip(NAMES[:7], g):
+        check_close(name, t.cpu().numpy(), go[name], *TOL["float32"])
+    assert cs2d.device_status() == 0
+
+
 def test_fp32_results_of_strided_16bit_inputs_without_softplus():
     inp = make_inputs(2, 2, 10, 6, 11, 19, dtype=torch.bfloat16, seed=5, with_bias=False)
     inp["delta"] = (inp["delta"].float().abs() * 0.1).to(torch.bfloat16)
