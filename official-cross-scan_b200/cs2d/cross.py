@@ -35,6 +35,8 @@ maps, much slower when batch x channel tiles cannot fill the GPU).
 """
 from __future__ import annotations
 
+import torch
+
 from . import _lib
 
 
@@ -64,13 +66,13 @@ def _dir_backward(u, delta, A, B, C, w, D, delta_bias, dy, saved, delta_softplus
                                          bool(deterministic)))
 
 
-class CrossScan2D:
-    """The operator as a function object: ``CrossScan2D.apply(u, delta, A, B, C, w, D, delta_bias, delta_softplus,
+class CrossScan2D(torch.autograd.Function):
+    """The operator as a Function: ``CrossScan2D.apply(u, delta, A, B, C, w, D, delta_bias, delta_softplus,
     A_decay, deterministic)``.  The autograd node itself is native (``csrc/cs2d_torch.cpp``)."""
 
     @staticmethod
     def apply(u, delta, A, B, C, w, D=None, delta_bias=None, delta_softplus=True, A_decay=None, deterministic=False):
-        return _lib.native().cross(u, delta, A, B, C, w, D, delta_bias, bool(delta_softplus), A_decay, bool(deterministic))
+        return cross_scan_2d(u, delta, A, B, C, w, D, delta_bias, delta_softplus, A_decay, bool(deterministic))
 
 
 def cross_scan_2d(u, delta, A, B, C, w, D=None, delta_bias=None, delta_softplus=True, A_decay=None,

@@ -19,8 +19,6 @@ Differences a caller can observe:
 """
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from . import _lib
@@ -29,69 +27,14 @@ _DT = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF
 MAX_DSTATE = 16
 
 
-def _check(cond, msg="check failed"):
-    if not cond:
-        raise RuntimeError(msg)
-
-
-def _inner_ok(t):
-    return t.stride(-1) == 1 or t.size(-1) == 1
-
-
-def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
-
-
 def _problem(u, delta, A, B, C, D, delta_bias, A_decay, delta_softplus, out_dtype, who, shared_u_dim=None):
-    input_type = u.dtype
-    _check(input_type in _DT, f"{who} not implemented for input type '{input_type}'")
-    _check(A.dtype == torch.float32, "A must be float32")
-    _check(delta.dtype == input_type and B.dtype == input_type and C.dtype == input_type,
-           "delta, B, C must have the dtype of u")
-    for name, t in (("u", u), ("delta", delta), ("A", A), ("B", B), ("C", C)):
-        _check(t.is_cuda, f"{name} must be a CUDA tensor")
-    _check(u.dim() == 4, "u must have shape (batch_size, dim, nrows, ncols)")
-    _check(_inner_ok(u) and _inner_ok(delta), "u and delta must be contiguous in the last dimension")
-    batch, dim, nrows, ncols = u.shape
-    if shared_u_dim is not None:  # u holds the channels of ONE group, read by all groups (cs2d_dirs)
-        _check(B.dim() == 5 and dim * B.size(1) == shared_u_dim, "u must have dim / n_groups channels")
-        dim = shared_u_dim
-    _check(A.dim() == 2 and B.dim() == 5 and delta.dim() == 4, "A, B, delta have the wrong rank")
-    dstate, n_groups, delta_dim = A.size(1), B.size(1), delta.size(1)
-    _check(dim % n_groups == 0, "dims should be dividable by n_groups")
-    _check(dim % delta_dim == 0, "dims should be dividable by delta_dim")
-    _check(dstate <= MAX_DSTATE, f"selective_scan only supports state dimension <= {MAX_DSTATE}")
-    _check(tuple(delta.shape) == (batch, delta_dim, nrows, ncols),
-           "delta must have shape (batch_size, delta_dim, nrows, ncols)")
-    _check(tuple(A.shape) == (dim, dstate), "A must have shape (dim, dstate)")
-    if A_decay is not None:
-        _check(tuple(A_decay.shape) == (1,), "A_decay must have shape (1)")
-        _check(A_decay.dtype == torch.float32 and A_decay.is_cuda, "A_decay must be a float32 CUDA tensor")
-    _check(tuple(B.shape) == (batch, n_groups, dstate, nrows, ncols),
-           "B must have shape (batch_size, n_groups, dstate, nrows, ncols)")
-    _check(_inner_ok(B), "B must be contiguous in the last dimension")
-    _check(tuple(C.shape) == (batch, n_groups, dstate, nrows, ncols),
-           "C must have shape (batch_size, n_groups, dstate, nrows, ncols)")
-    _check(_inner_ok(C), "C must be contiguous in the last dimension")
-    if D is not None:
-        _check(D.dtype == torch.float32 and D.is_cuda and _inner_ok(D), "D must be a contiguous float32 CUDA tensor")
-        _check(tuple(D.shape) == (dim,), "D must have shape (dim)")
-    if delta_bias is not None:
-        _check(delta_bias.dtype == torch.float32 and delta_bias.is_cuda and _inner_ok(delta_bias),
-               "delta_bias must be a contiguous float32 CUDA tensor")
-        _check(tuple(delta_bias.shape) == (delta_dim,), "delta_bias must have shape (delta_dim)")
-    p = _lib.Problem()
-    p.batch, p.dim, p.nrows, p.ncols = batch, dim, nrows, ncols
-    p.dstate, p.n_groups, p.delta_dim = dstate, n_groups, delta_dim
-    p.io_dtype, p.out_dtype, p.delta_softplus = _DT[input_type], _DT[out_dtype], int(bool(delta_softplus))
-    p.u, p.u_bs, p.u_ds, p.u_hs = u.data_ptr(), u.stride(0), u.stride(1), u.stride(2)
-    p.delta, p.delta_bs, p.delta_ds, p.delta_hs = delta.data_ptr(), delta.stride(0), delta.stride(1), delta.stride(2)
-    p.A, p.A_ds, p.A_ns = A.data_ptr(), A.stride(0), A.stride(1)
-    p.B, p.B_bs, p.B_gs, p.B_ns, p.B_hs = B.data_ptr(), B.stride(0), B.stride(1), B.stride(2), B.stride(3)
-    p.C, p.C_bs, p.C_gs, p.C_ns, p.C_hs = C.data_ptr(), C.stride(0), C.stride(1), C.stride(2), C.stride(3)
-    p.D = D.data_ptr() if D is not None else None
-    p.delta_bias = delta_bias.data_ptr() if delta_bias is not None else None
-    p.A_decay = A_decay.data_ptr() if A_decay is not None else None
+    """The C ABI's description of a problem, after the checks that the operators make (``shared_u_dim``: ``u`` holds the channels
+    of one group, read by all groups, ``shared_u_dim`` in all)."""
+    raw = _lib.native().problem(u, delta, A, B, C, D, delta_bias, A_decay, bool(delta_softplus), out_dtype, who,
+                                shared_u_dim is not None)
+    p = _lib.Problem.from_buffer_copy(raw)
+    if shared_u_dim is not None and p.dim != shared_u_dim:
+        raise RuntimeError("u must have dim / n_groups channels")
     return p
 
 
@@ -158,25 +101,12 @@ def bwd(u, delta, A, B, C, D_, delta_bias_, dout, x_, x_v_, delta_softplus, A_de
 
 
 class SelectiveScan2D(torch.autograd.Function):
-    """Autograd wrapper over ``fwd`` / ``bwd`` (the reference ships none)."""
+    """The operator as a Function: ``SelectiveScan2D.apply(u, delta, A, B, C, D, delta_bias, delta_softplus, out_float,
+    A_decay)``.  The autograd node itself is native (``csrc/cs2d_torch.cpp``)."""
 
     @staticmethod
-    def forward(ctx, u, delta, A, B, C, D=None, delta_bias=None, delta_softplus=False, out_float=False,
-                A_decay=None):
-        out, x, x_v, x_sd = fwd(u, delta, A, B, C, D, delta_bias, delta_softplus, out_float, A_decay)
-        ctx.delta_softplus = delta_softplus
-        ctx.has = (D is not None, delta_bias is not None, A_decay is not None)
-        ctx.save_for_backward(u, delta, A, B, C, D, delta_bias, A_decay, x, x_v, x_sd)
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        u, delta, A, B, C, D, delta_bias, A_decay, x, x_v, x_sd = ctx.saved_tensors
-        if dout.stride(-1) != 1:
-            dout = dout.contiguous()
-        du, ddelta, dA, dB, dC, dD, dbias, ddecay = bwd(u, delta, A, B, C, D, delta_bias, dout, x, x_v,
-                                                        ctx.delta_softplus, A_decay, x_sd)
-        return du, ddelta, dA, dB, dC, dD, dbias, None, None, ddecay
+    def apply(u, delta, A, B, C, D=None, delta_bias=None, delta_softplus=False, out_float=False, A_decay=None):
+        return selective_scan_2d(u, delta, A, B, C, D, delta_bias, delta_softplus, out_float, A_decay)
 
 
 def selective_scan_2d(u, delta, A, B, C, D=None, delta_bias=None, delta_softplus=False, out_float=False,

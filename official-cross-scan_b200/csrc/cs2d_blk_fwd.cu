@@ -51,7 +51,7 @@ template <int NG, int DT, bool KEEP>
 __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_constant__ Blk P) {
     using S = BkFwd<NG>;
     using T = typename bk_type<DT>::t;
-    constexpr int SPW = S::SPW, YP = S::YP, NCP = NG / 8 > 0 ? NG / 8 : 1;   // NCP: 16-byte copies per lane and quarter block
+    constexpr int SPW = S::SPW, YP = S::YP, NCP = NG / 8;   // NCP: 16-byte copies per lane and quarter block
     extern __shared__ __align__(16) unsigned char smem_[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char *sm = smem_ + warp * S::total;
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
     auto copy_bc = [&](const unsigned char *src, int qt, bool on) {
         unsigned char *dst = reinterpret_cast<unsigned char *>(sBC + qt * 8 * NG) + lane * 16;
         src += qt * 64 * NG + lane * 16;
-        if (on && (NG >= 8 || lane < 4 * NG)) {
+        if (on) {
 #pragma unroll
             for (int i = 0; i < NCP; ++i) bk_cp16(dst + 512 * i, src + 512 * i);
         }

@@ -389,6 +389,13 @@ struct CrossFunction : torch::autograd::Function<CrossFunction> {
     }
 };
 
+// The problem as the bytes of a cs2d_problem, for the callers that own their buffers
+py::bytes py_problem(const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor &B, const Tensor &C, const OptT &D, const OptT &bias,
+                     const OptT &decay, bool softplus, at::ScalarType out_type, const std::string &who, bool shared_u) {
+    const cs2d_problem p = make_problem(Args{u, delta, A, B, C, opt(D), opt(bias), opt(decay), softplus}, out_type, who.c_str(), shared_u);
+    return py::bytes(reinterpret_cast<const char *>(&p), sizeof(p));
+}
+
 // ---- Python entry points -----------------------------------------------------------------------------
 Args args_of(const Tensor &u, const Tensor &delta, const Tensor &A, const Tensor &B, const Tensor &C, const OptT &D, const OptT &bias,
              bool softplus, const OptT &decay) {
@@ -460,6 +467,7 @@ std::vector<OptT> py_cross_bwd(const Tensor &u, const Tensor &delta, const Tenso
 
 PYBIND11_MODULE(_native, m) {
     m.doc() = "native host path of the cs2d operators (see cs2d/ops.py and cs2d/cross.py)";
+    m.def("problem", &py_problem);
     m.def("fwd", &py_fwd, py::call_guard<py::gil_scoped_release>());
     m.def("fwd_only", &py_fwd_only, py::call_guard<py::gil_scoped_release>());
     m.def("bwd", &py_bwd, py::call_guard<py::gil_scoped_release>());
