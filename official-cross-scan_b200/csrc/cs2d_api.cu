@@ -507,19 +507,26 @@ static size_t blk_bc_bytes(const Blk &k, int NG) { return (size_t)(k.items / k.n
 static size_t blk_col_bytes(const Blk &k) { return (size_t)k.nblk * (k.nstrip - 1) * 4 * k.NL * sizeof(float4); }
 
 // ---- pair-walk kernels (cs2d_pair_fwd.cu, cs2d_pair_bwd.cu) -------------------------------------------
-// One scan orientation and rows of at most 128 columns also have the streaming kernels, which lose where they load a row
-// element by element or word by word (measured, training step with 6k to 200k channels, streaming / pair-walk us: 16-bit
-// 7 columns 494 / 178, 14: 395 / 281, 22: 338 / 265, 37: 1120 / 861, but 16: 260 / 258, 28: 259 / 340, 30: 357 / 415, 61: 733 / 843;
-// fp32 7 columns 513 / 192, 16: 637 / 424, 56: 738 / 785).  The alternative of directions and of wider rows are the tile
-// kernels (28x28 cross 2133 / 398, 150x150 scan 21944 / 4273), except where a few warps' worth of channels on a large map
-// would leave the GPU idle (8 items of 224x224: 4265 / 7178; of 56x56: 794 / 507).
-static bool pair_dirs(const cs2d_problem *p) {   // the alternative: tile kernels
-    return p->ncols <= 64 || (int64_t)p->batch * p->n_groups * ((p->dim / p->n_groups + PW_CH - 1) / PW_CH) >= 16;
+// Directions, and rows of more than 128 columns: the alternative is the tile kernels, a CTA of which takes eight channels.  While
+// those run in one round of CTAs they are the faster ones on long rows, until rows are cut into tiles (training step with flips
+// and merge, bf16, tile / pair-walk us; 144 CTAs: 96 columns 1444 / 1126, 128: 2025 / 2189, 150: 3049 / 3171, 200: 3943 / 5186, 336: 39108 /
+// 16668; 160 CTAs: 128: 3280 / 2164, 150: 5724 / 3516, 200: 7362 / 6131; fp32 144: 96: 1508 / 1412, 200: 3666 / 6659, 156: 7015 / 6673).
+static bool pair_dirs(const cs2d_problem *p) {
+    return p->ncols <= 96 || p->ncols > kTileCols || (int64_t)p->batch * p->n_groups * ((p->dim / p->n_groups + 7) / 8) > kSMs;
 }
-static bool pair_one(const cs2d_problem *p) {    // streaming kernels
-    const int W = p->ncols;
-    if (p->io_dtype == CS2D_F32) return W <= 16;
-    return W < 16 || (W % 2 ? W <= 45 : W % 4 && W <= 24);
+// One orientation: the alternative is the streaming kernels, which lose where they load a row element by element or word by word,
+// once there are more warps' worth of channels (items) than SMs (training step, streaming / pair-walk us.  16-bit, 192 items:
+// 9 columns 103 / 84, 10: 92 / 64, 12: 76 / 68, 14: 123 / 95, 21: 246 / 217, 37: 641 / 490, but at 128: 82 / 84, 60 / 64, 53 / 68, 79 / 95, 184 / 217,
+// 379 / 361; 512 items of 18 columns 246 / 188, 22: 305 / 254, 256 of them 129 / 154, 158 / 188; 1152 items of 16: 155 / 157, 704 of 20: 258 / 314,
+// 320 of 30: 321 / 382, 768 of 45: 2509 / 2567; a quarter of the channels per item, 37 columns: 635 / 723.  fp32, 768 items: 16 columns
+// 236 / 229, 18: 610 / 510, 19: 617 / 574, 20: 380 / 572, 22: 794 / 742, 25: 848 / 1186; 64 items: 9: 82 / 78, 14: 125 / 88, 16: 90 / 91, 17: 115 / 170).
+static bool pair_one(const cs2d_problem *p) {
+    const int W = p->ncols, dpg = p->dim / p->n_groups;
+    const int64_t items = (int64_t)p->batch * p->n_groups * ((dpg + PW_CH - 1) / PW_CH);
+    if (p->io_dtype == CS2D_F32) return W <= 16 || (W % 4 && W < 24 && items > kSMs);
+    if (W <= 8) return true;
+    if (W % 2) return items > kSMs && (W <= 24 || (W < 45 && dpg >= PW_CH));
+    return W < 16 ? items > kSMs : W % 4 && W <= 24 && items > 2 * kSMs;
 }
 static bool pair_ok(const cs2d_problem *p, const cs2d_dirs *o) {
     if (!pair_shape(p) || dirs_serial(o) || tile_state(o)) return false;

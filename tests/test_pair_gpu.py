@@ -27,6 +27,15 @@ CASES = [
     ((2, 8, 10, 1, 9, 300), torch.bfloat16, {"with_bias": False}),
     ((4, 4, 8, 1, 5, 131), torch.float32, {}),
     ((60, 1, 1300, 1, 3, 5), torch.float32, {}),        # more warps than the GPU holds at once
+    # One orientation, 16-bit: with few warps' worth of channels most of the shapes above run on the streaming kernels
+    ((150, 1, 64, 1, 5, 9), torch.bfloat16, {}),        # a full warp of channels; odd rows (element by element)
+    ((75, 1, 65, 1, 5, 13), torch.float16, {}),         # a channel more than a warp holds
+    ((150, 1, 40, 1, 6, 14), torch.bfloat16, {}),       # pieces of four bytes
+    ((150, 1, 24, 1, 6, 12), torch.float16, {}),        # eight
+    ((150, 2, 9, 1, 5, 22), torch.bfloat16, {}),        # two blocks per band; a short last band
+    ((150, 1, 64, 1, 3, 43), torch.float16, {"with_D": False}),
+    ((150, 1, 11, 1, 9, 19), torch.float32, {"with_bias": False}),
+    ((40, 4, 8, 1, 5, 131), torch.float32, {}),         # wider than the streaming kernels' rows
 ]
 
 
@@ -66,10 +75,11 @@ def test_pair_walk_against_oracle(shape, dtype, kw, det):
     _check(out, g, inp, dtype)
 
 
-@pytest.mark.parametrize("w", [14, 22, 23])
-def test_fp32_results_of_16_bit_views(w):
-    """fp32 results and gradients; u, delta and dout are views whose rows are not contiguous and start at odd elements."""
-    inp = make_inputs(2, 2, 20, 1, 9, w, dtype=torch.bfloat16, seed=3)
+@pytest.mark.parametrize("w,batch", [(14, 2), (22, 2), (23, 2), (14, 75), (22, 150), (23, 75)])
+def test_fp32_results_of_16_bit_views(w, batch):
+    """fp32 results and gradients; u, delta and dout are views whose rows are not contiguous and start at odd elements.  (The
+    small batches run on the streaming kernels.)"""
+    inp = make_inputs(batch, 2, 20, 1, 9 if batch == 2 else 5, w, dtype=torch.bfloat16, seed=3)
     d = _dev(inp)
 
     def view(t, left):
@@ -86,7 +96,8 @@ def test_fp32_results_of_16_bit_views(w):
 
 @pytest.mark.parametrize("shape,dtype", [((1, 4, 9, 1, 6, 20), torch.float32), ((2, 4, 66, 1, 7, 7), torch.bfloat16),
                                          ((1, 4, 12, 1, 10, 14), torch.float16), ((3, 4, 8, 1, 28, 56), torch.bfloat16),
-                                         ((4, 4, 10, 1, 11, 100), torch.float32), ((1, 4, 10, 1, 6, 21), torch.bfloat16),
+                                         ((4, 4, 10, 1, 11, 100), torch.float32), ((10, 4, 30, 1, 5, 100), torch.float32), ((40, 4, 8, 1, 5, 130), torch.bfloat16),
+                                         ((1, 4, 10, 1, 6, 21), torch.bfloat16),
                                          ((1, 4, 10, 1, 9, 7), torch.float32), ((4, 4, 14, 1, 9, 9), torch.bfloat16)])
 def test_corner_directions_and_merge(shape, dtype):
     b, K, d, n, h, w = shape
