@@ -27,6 +27,7 @@ CASES = [
     ((1, 1, 1, 1, 1, 1), torch.float32, {}),          # a single pixel of a single channel
     ((1, 4, 70, 1, 12, 20), torch.float32, {}),       # more pairs than one CTA holds
     ((2, 1, 33, 1, 4, 9), torch.float16, {}),
+    ((2, 4, 7, 1, 7, 7), torch.bfloat16, {"with_D": False, "with_bias": False}),   # (with eight channels: the pair-walk kernels)
 ]
 
 

@@ -2,7 +2,10 @@
 one image row apart, so the recurrence along the row needs no scan) against the float64 oracle, and the
 backward that follows it, which reads the checkpoints this forward wrote: every lane count, strips of 7
 and of 8 columns, ragged rows, channel counts that leave warps or lanes idle, 9 to 16 states, all three
-input types, fp32 output, shared delta, A_decay, missing optionals, strided views."""
+input types, fp32 output, shared delta, A_decay, missing optionals, strided views.
+
+It serves groups of fewer than eight channels, and every shape in a deterministic step; otherwise groups of eight and more run
+on the block-walk kernels."""
 import numpy as np
 import pytest
 import torch
@@ -57,6 +60,28 @@ def test_row_walk_forward_and_the_backward_behind_it(shape, dtype, kw):
         if t is None:
             assert go[name] is None, name
             continue
+        check_close(name, t.float().cpu().numpy(), go[name], rtol, atol)
+    assert cs2d.device_status() == 0
+
+
+@pytest.mark.parametrize("shape,dtype,kw", [c for c in CASES if c[0][2] >= 8] + [((2, 4, 7, 16, 13, 56), torch.bfloat16, {})],
+                         ids=lambda v: str(v)[-40:])
+def test_row_walk_forward_of_a_deterministic_step(shape, dtype, kw):
+    """Channel counts of more than one CTA per group among them (12 warps; a channel each at 56 columns)."""
+    inp = make_inputs(*shape, dtype=dtype, seed=4, **kw)
+    names = [k for k in ("u", "delta", "A", "B", "C", "D", "delta_bias") if inp[k] is not None]
+    d = {k: inp[k].cuda().requires_grad_(True) for k in names}
+    torch.use_deterministic_algorithms(True)
+    try:
+        y = cs2d.selective_scan_2d(*(d.get(k) for k in ("u", "delta", "A", "B", "C", "D", "delta_bias")), True)
+        grads = torch.autograd.grad(y, [d[k] for k in names], inp["dout"].cuda())
+    finally:
+        torch.use_deterministic_algorithms(False)
+    yo, go = _oracle(inp)
+    rtol, atol = TOL[str(dtype)[6:]]
+    check_close("out", y.detach().float().cpu().numpy(), yo, rtol, atol)
+    for k, t in zip(names, grads):
+        name = "ddelta_bias" if k == "delta_bias" else "d" + k
         check_close(name, t.float().cpu().numpy(), go[name], rtol, atol)
     assert cs2d.device_status() == 0
 
