@@ -294,7 +294,7 @@ static size_t blk_col_bytes(const Blk &k);
 static size_t blk_bc_bytes(const Blk &k, int NG);
 
 // (two states fill a quarter of the lanes and are still 1.2 to 2.2 times as fast as on the tile kernels: 32x4x192x28x28 bf16
-// training step 2171 -> 1125 us)
+// training step 2171 -> 1194 us)
 static bool blk_shape(const cs2d_problem *p) { return p->dstate > 1 && p->dim / p->n_groups >= 8; }
 
 static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool backward, const void *img = nullptr, int64_t img_bs = 0,
