@@ -153,10 +153,11 @@ int cs2d_bwd(const cs2d_problem *p, const void *dout, int64_t dout_bs, int64_t d
  *                     writer: no atomics, the same bits on every run.  For ncols <= 256 the
  *                     images are WRITTEN (they need not be initialised); wider rows run as
  *                     column tiles in several launches, which add onto them: zero-fill them
- *                     first.  Slower (measured +17 % to +24 % on the stage-1 and
+ *                     first.  Slower (measured 2.2 times on the stage-1 and
  *                     segmentation-scale maps, far more when batch x channel tiles leave
- *                     most SMs idle): a quarter of the CTAs, and the read-modify-write of
- *                     the merged image sits in the write-out path.
+ *                     most SMs idle or the channels have a single state): a quarter of the
+ *                     CTAs, the read-modify-write of the merged image sits in the write-out
+ *                     path, and only the tile kernels have this form.
  * The deterministic backward (cs2d_bwd_det) is not combined with the merge (dB, dC and the
  * parameter gradients still sum over channel tiles with atomics).
  */

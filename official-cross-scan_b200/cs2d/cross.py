@@ -30,7 +30,7 @@ order).  With ``deterministic=True`` one CTA owns the channel tile for all K
 directions and walks them one after the other, so it alone writes its part of the
 merged images - stored by the first direction, read-modify-written by the others
 in a fixed order: no atomics, no zero fills, bit-identical ``y`` and ``du`` from run
-to run, at a quarter of the CTAs (measured 17-24 % slower on 56x56 and 128x128
+to run, at a quarter of the CTAs (measured 2.2 times slower on 56x56 and 128x128
 maps, much slower when batch x channel tiles cannot fill the GPU).
 """
 from __future__ import annotations
