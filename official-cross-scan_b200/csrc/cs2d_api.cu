@@ -569,7 +569,7 @@ static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool bac
     }
     k.f32 = p->io_dtype != CS2D_F32 && p->out_dtype == CS2D_F32;
     k.nblk = (k.H + PW_R - 1) / PW_R; k.nsub = (k.W + 7) / 8; k.wp = (k.W + 1) & ~1;
-    k.np = (k.dpg + 1) / 2;
+    k.nl = std::min(32, (k.dpg + 1) / 2 + 1);
     k.ntile = (k.dpg + PW_CH - 1) / PW_CH; k.items = p->batch * k.G * k.ntile;
     // How blocks are moved (see cs2d_pair.cuh): whole bands where every tensor's rows are contiguous and a band fits
     struct In { const void *p; int64_t bs, ds, hs; } in[3] = {{p->u, p->u_bs, p->u_ds, p->u_hs}, {p->delta, p->delta_bs, p->delta_ds, p->delta_hs}, {img, img_bs, img_ds, img_hs}};
@@ -602,9 +602,9 @@ static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool bac
     const int64_t need = ((int64_t)k.items + (PW_WARPS >> k.rwl) - 1) / (PW_WARPS >> k.rwl), cap = ctas * kSMs;
     k.grid = (int)(need < cap ? need : cap);
 }
-static size_t pair_row_bytes(const Pw &k) { return (size_t)(k.items / k.ntile) * (k.nblk - 1) * k.wp * k.np * sizeof(float4); }
+static size_t pair_row_bytes(const Pw &k) { return (size_t)k.items * (k.nblk - 1) * k.wp * k.nl * sizeof(float4); }
 static size_t pair_team_bytes(const Pw &k, bool backward) { return (size_t)resident(k.items, pair_ctas(backward), PW_WARPS) * k.wp * 32 * sizeof(float4); }
-static size_t pair_col_bytes(const Pw &k) { return (size_t)(k.items / k.ntile) * k.nblk * (k.nsub - 1) * PW_R * k.np * 24; }
+static size_t pair_col_bytes(const Pw &k) { return (size_t)k.items * k.nblk * (k.nsub - 1) * PW_R * k.nl * 24; }
 // pieces of results that take the place of inputs in shared memory
 static int pair_vout(const Pw &k, const void *ptr, int es, int64_t bs, int64_t ds, int64_t hs) {
     if (k.el && es == 2) return 2;

@@ -23,7 +23,8 @@
 //        per warp, or team of row workers, that is on the GPU at a time)
 //   colq [item][band][column / 8 - 1][4 rows][nl] float4 (q, q', s, s') of the column left of a group of 8
 //   cola the same, float2 (a, a')
-// (q = h - s; an item is a warp's 64 channels of one image and group; nl: its pairs of channels, 32 but for a group's last.)
+// (q = h - s; an item is a warp's 64 channels of one image and group.  nl: 32, or in groups of less than 63 channels their
+// pairs and one place for all lanes past them, which hold the same values: lane i uses place min(i, nl - 1).)
 //
 // Few items run with 2 or 4 row WORKERS per CTA of four warps: worker w takes every RW-th band, one step behind worker
 // w - 1; the CTA's warps then meet on its barrier once per step.
@@ -41,7 +42,7 @@ struct Pw {
     int nblk, nstrip, nsub, wp;   // bands; fetched blocks per band; groups of 8 columns; columns, even
     int period, rwl, npass;       // steps per band, log2 of the row workers, bands per worker
     int ntile, items, grid;       // warps' worth of channels per group; batch * G * ntile
-    int np;                       // pairs of channels per group
+    int nl;                       // places of an item (see above)
     unsigned flip_h, flip_w;
     int shared;                   // bit 0: u has dpg channels shared by the groups, bit 1: dout
     int fs, lin, el;              // columns of a fetched block; whole bands; element by element
@@ -79,8 +80,6 @@ struct PwPos {   // position in a warp's stream of blocks
         g = bg % P.G;
         tile = item % P.ntile;
     }
-    __device__ __forceinline__ int pairs(const Pw &P) const { return min(32, P.np - 32 * tile); }
-    __device__ __forceinline__ int64_t first(const Pw &P) const { return (int64_t)bg * P.np + 32 * tile; }   // pairs of the items before this one
     __device__ __forceinline__ void next(const Pw &P, int stride) {
         if (++strip < P.period) return;
         strip = 0;

@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
     pos.decode(P);
     auto blk_of = [&](const PwPos &q) { return P.nblk - 1 - (q.pass * rw + w); };     // bands from the bottom up, blocks from the right
     auto live = [&](const PwPos &q, int L) { return L >= 0 && L < lmax && q.item < P.items && q.strip < P.nstrip && q.pass * rw + w < P.nblk; };
+    const int lp = min(lane, P.nl - 1);   // this lane's place in the checkpoints
     PwBC<DT> bcr;
     auto blocks = [&](const PwPos &q, auto &&f) {   // f(delta's block, u's, dout's) of a position
         const int r0 = blk_of(q) * PW_R, c0 = (P.nstrip - 1 - q.strip) * P.fs, ch0 = q.tile * PW_CH, cg = q.g * P.dpg + ch0, b = q.bg / P.G, nch = P.dpg - ch0;
@@ -100,9 +101,8 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
         const int blk = blk_of(pos), r0 = blk * PW_R, c0 = (P.nstrip - 1 - pos.strip) * P.fs, ch0 = pos.tile * PW_CH, cg = pos.g * P.dpg + ch0, nch = P.dpg - ch0, b = pos.bg / P.G;
         const bool fh = DIRS && ((P.flip_h >> pos.g) & 1u), fw = DIRS && ((P.flip_w >> pos.g) & 1u);
         const int nc = min(P.fs, P.W - c0);
-        const int nl = pos.pairs(P);
-        const float4 *above = P.row + pos.first(P) * (P.nblk - 1) * P.wp + (int64_t)((blk - 1) * P.wp + c0) * nl + lane;
-        const bool mine = 2 * lane < nch;
+        const int nl = P.nl;
+        const float4 *above = P.row + (((int64_t)pos.item * (P.nblk - 1) + blk - 1) * P.wp + c0) * nl + lp;
         float4 *arow = P.adj + ((int64_t)(first + (warp >> P.rwl)) * P.wp + c0) * 32 + lane;
         if (pos.strip == 0) {
             if (pos.pass == 0) {   // a new item
@@ -122,12 +122,12 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
         float4 up[2], colq[PW_R], dn[2];
         float2 cola[PW_R], cnr = bc(0.f), hup[2];
         auto load_up = [&](int c) {
-            up[0] = bk_ld16<true>(above + c * nl, blk > 0 && mine);
-            up[1] = bk_ld16<true>(above + (c + 1) * nl, blk > 0 && mine);
+            up[0] = bk_ld16<true>(above + c * nl, blk > 0);
+            up[1] = bk_ld16<true>(above + (c + 1) * nl, blk > 0);
         };
         auto load_group = [&](int c) {
-            const bool left = c0 + c > 0 && mine;
-            const int64_t o = ((pos.first(P) * P.nblk + blk * nl) * (P.nsub - 1) + (((c0 + c) >> 3) - 1) * nl) * 4 + lane;
+            const bool left = c0 + c > 0;
+            const int64_t o = ((((int64_t)pos.item * P.nblk + blk) * (P.nsub - 1) + ((c0 + c) >> 3) - 1) * 4) * nl + lp;
 #pragma unroll
             for (int r = 0; r < PW_R; ++r) {
                 colq[r] = bk_ld16<true>(P.colq + o + r * nl, left);
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 dn[i] = bk_ld16<false>(arow + (c + i) * 32, blk + 1 < P.nblk);
-                hup[i] = pw_ld8(above + (c + i) * nl, blk > 0 && mine);
+                hup[i] = pw_ld8(above + (c + i) * nl, blk > 0);
             }
         };
         load_group((nc - 1) & ~7);

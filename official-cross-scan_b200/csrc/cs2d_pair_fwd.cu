@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
     pos.item = first + (warp >> P.rwl); pos.pass = pos.strip = 0;
     pos.decode(P);
     auto live = [&](const PwPos &q, int L) { return L >= 0 && L < lmax && q.item < P.items && q.strip < P.nstrip && q.pass * rw + w < P.nblk; };
+    const int lp = min(lane, P.nl - 1);   // this lane's place in the checkpoints
     PwBC<DT> bcr;
     auto blocks = [&](const PwPos &q, auto &&f) {   // f(delta's block, u's block) of a position
         const int r0 = (q.pass * rw + w) * PW_R, c0 = q.strip * P.fs, ch0 = q.tile * PW_CH, cg = q.g * P.dpg + ch0, b = q.bg / P.G, nch = P.dpg - ch0;
@@ -59,14 +60,13 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
         const bool fh = DIRS && ((P.flip_h >> pos.g) & 1u), fw = DIRS && ((P.flip_w >> pos.g) & 1u);
         const int nc = min(P.fs, P.W - c0);
         // row of the band above (rolling: the same row), row of this band (rolling: the team's)
-        const int nl = KEEP ? pos.pairs(P) : 32;
-        float4 *row = P.row + (KEEP ? pos.first(P) * (P.nblk - 1) : 32 * (int64_t)(first + (warp >> P.rwl))) * P.wp + (int64_t)(KEEP ? blk * P.wp + c0 : c0) * nl + lane;
-        const float4 *above = KEEP ? row - P.wp * nl : row;
-        const bool mine = 2 * lane < nch;
+        const int nl = KEEP ? P.nl : 32;
+        float4 *row = P.row + ((KEEP ? (int64_t)pos.item * (P.nblk - 1) + blk : (int64_t)(first + (warp >> P.rwl))) * P.wp + c0) * nl + (KEEP ? lp : lane);
+        const float4 *above = KEEP ? row - (int64_t)P.wp * nl : row;
         float4 up[2];
         auto fetch_up = [&](int c) {
-            up[0] = bk_ld16<false>(above + c * nl, blk > 0 && mine);
-            up[1] = bk_ld16<false>(above + (c + 1) * nl, blk > 0 && mine);
+            up[0] = bk_ld16<false>(above + c * nl, blk > 0);
+            up[1] = bk_ld16<false>(above + (c + 1) * nl, blk > 0);
         };
         fetch_up(0);
         if (pos.strip == 0) {
@@ -89,13 +89,11 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
 #pragma unroll 1
         for (int c = 0; c < nc; c += 2) {
             if (KEEP && c0 + c > 0 && ((c0 + c) & 7) == 0) {   // the column left of a group of 8
-                const int64_t o = ((pos.first(P) * P.nblk + blk * nl) * (P.nsub - 1) + (((c0 + c) >> 3) - 1) * nl) * 4 + lane;
-                if (mine) {
+                const int64_t o = ((((int64_t)pos.item * P.nblk + blk) * (P.nsub - 1) + ((c0 + c) >> 3) - 1) * 4) * nl + lp;
 #pragma unroll
-                    for (int r = 0; r < PW_R; ++r) {
-                        P.colq[o + r * nl] = make_float4(ql[r].x, ql[r].y, sl[r].x, sl[r].y);
-                        P.cola[o + r * nl] = al[r];
-                    }
+                for (int r = 0; r < PW_R; ++r) {
+                    P.colq[o + r * nl] = make_float4(ql[r].x, ql[r].y, sl[r].x, sl[r].y);
+                    P.cola[o + r * nl] = al[r];
                 }
             }
             const bool on1 = c + 1 < nc;
@@ -126,7 +124,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
                     hd = hl[r]; hu = h; au = a;
                     hl[r] = h; al[r] = a; ql[r] = q; sl[r] = s;
                 }
-                bk_st16(row + (c + cc) * nl, make_float4(hl[PW_R - 1].x, hl[PW_R - 1].y, al[PW_R - 1].x, al[PW_R - 1].y), blk + 1 < P.nblk && mine);
+                bk_st16(row + (c + cc) * nl, make_float4(hl[PW_R - 1].x, hl[PW_R - 1].y, al[PW_R - 1].x, al[PW_R - 1].y), blk + 1 < P.nblk);
             }
             if (DIRS && (P.mw || P.f32)) {   // straight to the fp32 results (merge: onto the image)
                 const int fc = fw ? P.W - 1 - c0 - c : c0 + c;

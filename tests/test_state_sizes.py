@@ -47,7 +47,7 @@ def test_saved_state_of_the_kernels_that_run():
     pixels = 8 * 64 * 8 * 100 * 100
     exact, every = _sizes(_problem(8, 64, 8, 1, 100, 100))[0]
     assert exact == 8 * 64 * 4 * 25 * 128 * 8          # streaming: channel pairs x row blocks x padded columns
-    assert every < 4 * pixels                          # pair-walk (corner directions): 3.5 bytes per channel and pixel
+    assert every < 4.5 * pixels                        # pair-walk (corner directions): 3.5 bytes per channel and pixel, of five pairs for four
     exact, _ = _sizes(_problem(32, 4, 192, 2, 28, 28))[0]
     bc = 32 * 4 * 7 * 4 * 32 * 8 * 8                   # B and C of 8 state slots, in blocks of 32 pixels
     assert exact == bc + (6 * 4 + 7 * 3) * 4 * (32 * 4 * 96 * 3) * 16   # rows and columns of two states, and a place for the other six
