@@ -480,28 +480,31 @@ static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o,
     k.NL = (int64_t)p->batch * k.G * k.nsl * k.NS;
     const int spw = 32 / NG, ctas = blk_ctas(backward, NG);   // slots per warp, CTAs per SM
     k.ntile = (k.nsl + spw - 1) / spw; k.items = p->batch * k.G * k.ntile;
-    // Row workers: as few as fill the GPU; with short rows a worker waits for the others at the end of a row
-    const int64_t slots = (int64_t)kSMs * ctas * BK_WARPS;
+    // Row workers: the number for which the longest chain of blocks that a worker walks takes the least time.  A block's time grows
+    // with the warps that share a scheduler (measured, 56x56 maps, 1 / full: forward 2.6 / 4.8 us at 4, backward 6.4 / 11.2 us at 3), the
+    // last round of CTAs is seldom full, a worker is 1.3 (forward) or 1 blocks behind the one before it, which makes it wait where rows
+    // are short, and waiting for each other costs a little (us with 1, 2, 4, 8 workers; stage-1 backward, 3.46 rounds: 3880, 3854, 3870,
+    // 4040; forward, 2.59: 1240, 1258, 1208, 1595; 16x4x192x16x28x28 forward: 200, 179, 220, 220; 2x4x192x16x200x336 backward: 14100,
+    // 8750, 6190, 6580; one 56x56 image: 632, 311, 236, 224; 3x4x51x7x45x61: 733, 371, 197, 156).
+    const double slope = backward ? 0.375 : 0.28, lag = backward ? 1 : 1.3;
     double best = 1e300;
-    for (int rwl = 0; rwl < 3; ++rwl) {
-        const int rw = 1 << rwl;
-        if (rw > 1 && k.nblk < rw) break;
-        const int period = k.nstrip < BK_LAG * rw && rw > 1 ? BK_LAG * rw : k.nstrip;
-        const int64_t npass = (k.nblk + rw - 1) / rw, rounds = ((int64_t)k.items * rw + slots - 1) / slots;
-        // rounds of warps, each slower the more of them share an SM
-        const double cost = (double)rounds * (npass * period + BK_LAG * (rw - 1));
-        if (cost < best * 0.98) { best = cost; k.rwl = rwl; k.npass = (int)npass; k.period = period; }
+    for (int rwl = 0; (1 << rwl) <= std::min(k.nblk, BK_MAXRW); ++rwl) {
+        const int rw = 1 << rwl, warps = std::max(BK_WARPS, rw), cap = ctas * BK_WARPS / warps;   // CTAs per SM
+        const int64_t teams = warps / rw, n = ((int64_t)k.items + teams - 1) / teams, full = n / (cap * kSMs), rest = n % (cap * kSMs);
+        auto block = [&](int64_t per_sm) { return 1 + slope * (std::max<double>(1, per_sm * warps / 4.0) - 1); };
+        const double last = rest ? block((rest + kSMs - 1) / kSMs) : 0;
+        const double chain = (double)k.nblk / rw * (rw > 1 ? std::max<double>(k.nstrip, lag * rw) : k.nstrip) * (1 + (backward ? 0.03 : 0.015) * rwl);
+        const double cost = chain * (full * block(cap) + last) + lag * (rw - 1) * (last > 0 ? last : block(cap));
+        if (cost < best) { best = cost; k.rwl = rwl; k.warps = warps; k.grid = (int)std::min<int64_t>(n, cap * kSMs); }
     }
-    const int64_t need = ((int64_t)k.items + (BK_WARPS >> k.rwl) - 1) / (BK_WARPS >> k.rwl);
-    const int64_t cap = ctas * kSMs;   // CTAs that fit at once
-    k.grid = (int)(need < cap ? need : cap);
 }
 static size_t blk_row_bytes(const Blk &k) { return (size_t)(k.nblk - 1) * k.nstrip * 4 * k.NL * sizeof(float4); }
 // One row (the forward's rolling h, the backward's adjoint) per warp, or team of row workers, that is on the GPU at a time: a
 // team is done with it before its next item.  The bound does not depend on how the items are split, and so grows with the batch only.
 static int64_t resident(int64_t items, int ctas, int warps) { return std::min(items, (int64_t)ctas * kSMs * warps); }
+static size_t blk_team_row(const Blk &k) { return (size_t)k.nstrip * 4 * 32 * sizeof(float4); }
 static size_t blk_team_bytes(const Blk &k, bool backward, int NG) {
-    return (size_t)resident(k.items, blk_ctas(backward, NG), BK_WARPS) * k.nstrip * 4 * 32 * sizeof(float4);
+    return (size_t)resident(k.items, blk_ctas(backward, NG), BK_WARPS) * blk_team_row(k);
 }
 static size_t blk_bc_bytes(const Blk &k, int NG) { return (size_t)(k.items / k.ntile) * k.nblk * k.nstrip * BK_PX * NG * sizeof(float2); }
 static size_t blk_col_bytes(const Blk &k) { return (size_t)k.nblk * (k.nstrip - 1) * 4 * k.NL * sizeof(float4); }
@@ -535,9 +538,9 @@ static bool pair_ok(const cs2d_problem *p, const cs2d_dirs *o) {
 static Family family(const cs2d_problem *p, const cs2d_dirs *o) {
     return pair_ok(p, o) ? PAIR : stream_ok(p, o) ? STREAM : blk_ok(p, o) ? BLK : TILE;
 }
-// Bytes that may be moved at once, 8 at most: a divisor of every size and stride (in bytes) and of the address
-static int move_bytes(const void *ptr, std::initializer_list<int64_t> sizes) {
-    uintptr_t x = reinterpret_cast<uintptr_t>(ptr) | 8;
+// Bytes that may be moved at once, `most` at most: a divisor of every size and stride (in bytes) and of the address
+static int move_bytes(const void *ptr, std::initializer_list<int64_t> sizes, int most = 8) {
+    uintptr_t x = reinterpret_cast<uintptr_t>(ptr) | (uintptr_t)most;
     for (int64_t s : sizes) x |= (uintptr_t)s;
     return (int)(x & (~x + 1));
 }
@@ -662,6 +665,7 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
         Blk k;
         int NG;
         blk_fill(k, NG, p, o, false);
+        k.status = status;
         k.out = out; k.o_bs = out_bs; k.o_ds = out_ds; k.o_hs = out_hs;
         blk_state(k, NG, saved, rolling);
         cudaError_t e = launch_blk_fwd(k, NG, reinterpret_cast<cudaStream_t>(stream));
@@ -843,12 +847,17 @@ static int bwd_impl(const cs2d_problem *p, const cs2d_dirs *o, const void *dout,
         Blk k;
         int NG;
         blk_fill(k, NG, p, o, true);
+        k.status = status;
         blk_state(k, NG, saved, false);
         k.out = const_cast<void *>(dout); k.o_bs = dout_bs; k.o_ds = dout_ds; k.o_hs = dout_hs;
         k.adj = reinterpret_cast<float4 *>(scratch);
         k.du = du; k.ddelta = ddelta; k.dA = dA; k.dB = dB; k.dC = dC; k.dD = dD; k.dbias = ddelta_bias; k.ddecay = dA_decay;
         k.vec_dbc = vec_ok(dB, 4, p->ncols, {}) && vec_ok(dC, 4, p->ncols, {});
-        if (!fit_grid(&k.grid, k.items, BK_WARPS >> k.rwl, (size_t)k.nstrip * 4 * 32 * sizeof(float4), scratch_limit)) return CS2D_ERR_UNSUPPORTED;
+        const int es = esize(p->io_dtype), eso = esize(p->out_dtype);
+        k.vin = std::min(std::min(move_bytes(p->u, {p->u_bs * es, p->u_ds * es, p->u_hs * es, (int64_t)k.W * es}, 16),
+                                  move_bytes(p->delta, {p->delta_bs * es, p->delta_ds * es, p->delta_hs * es, (int64_t)k.W * es}, 16)),
+                         move_bytes(dout, {dout_bs * eso, dout_ds * eso, dout_hs * eso, (int64_t)k.W * eso}, 16));
+        if (!fit_grid(&k.grid, k.items, k.warps >> k.rwl, blk_team_row(k), scratch_limit)) return CS2D_ERR_UNSUPPORTED;
         cudaError_t e = launch_blk_bwd(k, NG, reinterpret_cast<cudaStream_t>(stream));
         if (e != cudaSuccess) return fail(CS2D_ERR_CUDA, "backward launch failed: %s", cudaGetErrorString(e));
         g_launches.fetch_add(1);
@@ -1063,7 +1072,7 @@ int cs2d_device_status(void) {
     if (v != 0) {
         cudaMemcpyToSymbol(g_cs2d_status, &zero, sizeof(int));
         fail(CS2D_ERR_CUDA, "a kernel gave up on a bounded wait (status %d: %s%s); its outputs are invalid", v,
-             (v & ERR_BULK_COPY_TIMEOUT) ? "bulk copy " : "", (v & ERR_STAGE_TIMEOUT) ? "staging warps" : "");
+             (v & ERR_BULK_COPY_TIMEOUT) ? "bulk copy " : "", (v & ERR_STAGE_TIMEOUT) ? "staging warps " : "", (v & ERR_WORKER_TIMEOUT) ? "row workers" : "");
     }
     return v;
 }

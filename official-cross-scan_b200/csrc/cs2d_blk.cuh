@@ -13,9 +13,10 @@
 // the SM's load unit when neighbouring lanes share their address, 4 otherwise, whatever else is broadcast - and that unit,
 // not arithmetic, bounds these kernels).  No barriers; sixteen warps per SM hide each other's latencies.
 //
-// Images with few recurrences run with 2 or 4 row WORKERS per CTA of four warps: worker w takes every RW-th row of
-// blocks, LAG steps behind worker w-1, which has then left the row of h it needs; the CTA's warps then meet on its
-// barrier once per block.
+// Images with few recurrences run with 2, 4 or 8 row WORKERS (warps of one CTA): the rows of blocks of a team's items are one
+// sequence, and worker w takes every RW-th of them.  A block needs the row of h (backward: of m) that the row before it in the
+// sequence left for the same columns, so a worker follows its predecessor a block behind: every worker counts its finished
+// blocks in shared memory, and waits for the count of the worker before it (RowSeq).
 #pragma once
 
 #include "cs2d_common.cuh"
@@ -23,19 +24,18 @@
 namespace cs2d {
 
 constexpr int BK_R = 4, BK_S = 8, BK_PX = BK_R * BK_S;   // a block: rows, columns, pixels
-constexpr int BK_WARPS = 4;                               // warps per CTA
-constexpr int BK_LAG = 2;                                 // steps between neighbouring row workers
+constexpr int BK_WARPS = 4;                               // warps per CTA (8 with 8 row workers)
+constexpr int BK_MAXRW = 8;                               // row workers per CTA
 static_assert(BK_R == RB, "row blocks and checkpoint cadence agree with the other kernels");
 
 struct Blk {
     int H, W, N, G, dpg, drep, io_dt, out_dt, softplus;
     int nblk, nstrip;       // rows of blocks, blocks per row
-    int period;             // steps per row of blocks: nstrip, or more when a worker has to wait for the others
     int rwl;                // log2 of the row workers per CTA
     int nsl;                // slots per group
     int ntile, items;       // warps' worth of slots per group; work items = batch * G * ntile
-    int grid;
-    int npass;              // rows of blocks per worker: ceil(nblk / workers)
+    int grid, warps;        // CTAs, warps of a CTA
+    int *status;            // device status word (see ERR_*)
     unsigned flip_h, flip_w;
     int shared;             // bit 0: u has dpg channels shared by the groups, bit 1: dout
     int roll;               // forward: one rolling row of h instead of the checkpoints
@@ -58,6 +58,7 @@ struct Blk {
     float4 *adj;                            // [teams][nstrip][4][32]: the adjoint row m between rows of blocks
     void *du, *ddelta;
     float *dA, *dB, *dC, *dD, *dbias, *ddecay;
+    int vin;                                // bytes of u, delta and dout that are copied at once: 16, 8, 4 or 2
     int vec_dbc;                            // dB, dC: rows of whole aligned groups of four columns
 };
 
@@ -70,21 +71,68 @@ __device__ __forceinline__ void bk_cp16(void *dst, const void *src) {
 __device__ __forceinline__ void bk_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void bk_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Position in a warp's stream of blocks: its items, passes of an item, blocks of a row.
+// Position in a worker's stream of blocks: the rows of blocks of its team's items, blocks of a row.
 struct BkPos {
-    int item, pass, strip, bg, g, slot;   // batch * G + group, group, first slot of the item inside its group
+    int item, row, strip, bg, b, g, slot;    // row of blocks in walking order; batch * G + group, batch, group, first slot of the item inside its group
+    int seq;                              // blocks of the team's sequence before this one
     __device__ __forceinline__ void decode(const Blk &P, int spw) {
         bg = item / P.ntile;
-        g = bg % P.G;
-        slot = (item % P.ntile) * spw;
+        b = bg / P.G;
+        g = bg - b * P.G;
+        slot = (item - bg * P.ntile) * spw;
     }
-    __device__ __forceinline__ void next(const Blk &P, int spw, int stride) {
-        if (++strip < P.period) return;
+    __device__ __forceinline__ void start(const Blk &P, int spw, int first, int w) {
+        item = first; row = w; strip = 0; seq = w * P.nstrip;   // (there are no more workers than rows)
+        decode(P, spw);
+    }
+    // returns whether the next block is of another item
+    __device__ __forceinline__ bool next(const Blk &P, int spw, int rw, int stride) {
+        ++seq;
+        if (++strip < P.nstrip) return false;
         strip = 0;
-        if (++pass < P.npass) return;
-        pass = 0;
+        seq += (rw - 1) * P.nstrip;
+        row += rw;
+        if (row < P.nblk) return false;
+        row -= P.nblk;
         item += stride;
         decode(P, spw);
+        return true;
+    }
+};
+
+// How many blocks of the sequence the workers of a CTA have left behind, and the wait of a worker for the one before it.
+struct RowSeq {
+    uint32_t mine, before;   // shared-memory addresses of the two counts
+    int nstrip;
+    __device__ __forceinline__ void init(int *count, int warp, int rw, int nstrip_) {   // all threads of the CTA, before a CTA barrier
+        nstrip = nstrip_;
+        const int w = warp & (rw - 1);
+        mine = smem_addr(count + warp); before = smem_addr(count + warp - w + ((w - 1) & (rw - 1)));
+        if ((threadIdx.x & 31) == 0) count[warp] = 0;
+    }
+    // what the warp's threads have written is there for whoever sees the count
+    __device__ __forceinline__ void done(int seq) const {
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(mine), "r"(seq + 1) : "memory");
+    }
+    // until the block above (in walking order) block `seq` is done.  Bounded: 2^22 polls of 20 ns or more, then false.
+    __device__ __forceinline__ bool wait(int seq) const {
+        const int need = seq + 1 - nstrip;   // (of the first row of a sequence: 0 or less)
+#pragma unroll 1
+        for (int i = 0; i < (1 << 22); ++i) {
+            int have;
+            asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(have) : "r"(before) : "memory");
+            if (__all_sync(0xffffffffu, have >= need)) return true;
+            __nanosleep(20);
+        }
+        return false;
+    }
+    // gives up: flags the error and lets the other workers run to their ends
+    __device__ __forceinline__ void abandon(int *status) const {
+        if ((threadIdx.x & 31) == 0) {
+            atomicOr(status, ERR_WORKER_TIMEOUT);
+            asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(mine), "r"(0x7fffffff) : "memory");
+        }
     }
 };
 
@@ -122,8 +170,8 @@ __device__ __forceinline__ uint32_t bk_ldp(const typename bk_type<DT>::t *p, boo
         asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.nc.b32 %0, [%1];\n\t}" : "=r"(v) : "l"(p), "r"((int)on));
         return v;
     } else {
-        unsigned short v;
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b16 %0, 0;\n\t@p ld.global.nc.b16 %0, [%1];\n\t}" : "=h"(v) : "l"(p), "r"((int)on));
+        uint32_t v;   // (a 32-bit register: nothing converts the value, and so waits for it, before it is used)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.nc.u16 %0, [%1];\n\t}" : "=r"(v) : "l"(p), "r"((int)on));
         return v;
     }
 }

@@ -48,34 +48,35 @@ struct BkFwd {   // a warp's shared memory
 };
 
 template <int NG, int DT, bool KEEP>
-__global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_constant__ Blk P) {
+__global__ void __launch_bounds__(BK_MAXRW * 32, 2) blk_fwd_kernel(const __grid_constant__ Blk P) {
     using S = BkFwd<NG>;
     using T = typename bk_type<DT>::t;
     constexpr int SPW = S::SPW, YP = S::YP, NCP = NG / 8;   // NCP: 16-byte copies per lane and quarter block
     extern __shared__ __align__(16) unsigned char smem_[];
+    __shared__ int sCount[BK_MAXRW];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char *sm = smem_ + warp * S::total;
     float4 *sIn = reinterpret_cast<float4 *>(sm + S::in), *sPar = reinterpret_cast<float4 *>(sm + S::par);
     float2 *sY = reinterpret_cast<float2 *>(sm + S::y), *sBC = reinterpret_cast<float2 *>(sm + S::bc);
     float2 *sY0 = reinterpret_cast<float2 *>(sm + S::y0), *sTop = reinterpret_cast<float2 *>(sm + S::top);
-    const int rw = 1 << P.rwl, w = warp & (rw - 1), nsub = BK_WARPS >> P.rwl, stride = gridDim.x * nsub;
+    const int rw = 1 << P.rwl, w = warp & (rw - 1), nsub = P.warps >> P.rwl, stride = gridDim.x * nsub;
     const int n = lane % NG, sl_ = lane / NG;              // this thread's state and slot of the warp
     const int lr = lane >> 3, lc = lane & 7;               // its pixel when staging
-    const int first = blockIdx.x * nsub, lmax = (P.items - first + stride - 1) / stride * P.npass * P.period;
-    const int steps = lmax + BK_LAG * (rw - 1);
+    const int first = blockIdx.x * nsub + (warp >> P.rwl);   // this team's first item
     const bool softplus = P.softplus != 0, drep1 = P.drep == 1;
     const float2 lgd = bc(P.decay ? log2f(__ldg(P.decay)) : 0.f);
 
     BkPos pos;
-    pos.item = first + (warp >> P.rwl); pos.pass = pos.strip = 0;
-    pos.decode(P, SPW);
-    auto live = [&](const BkPos &q, int L) { return L >= 0 && L < lmax && q.item < P.items && q.strip < P.nstrip && q.pass * rw + w < P.nblk; };
+    pos.start(P, SPW, first, w);
+    RowSeq rs;
+    rs.init(sCount, warp, rw, P.nstrip);
+    if (rw > 1) __syncthreads();
 
     // ---- loads of the next block: raw delta and u of the lane's pixel for every channel of the warp, delta of the row above ----
     uint32_t vd[2 * SPW], vu[2 * SPW], vt[SPW / 2];
     const T *pd = nullptr, *pu = nullptr, *pt = nullptr;   // at the first block of the row of blocks
     auto load_raw = [&](const BkPos &q) {
-        const int r0 = (q.pass * rw + w) * BK_R, ch0 = q.slot * 2, cg = q.g * P.dpg + ch0;
+        const int r0 = q.row * BK_R, ch0 = q.slot * 2, cg = q.g * P.dpg + ch0;
         const bool fw = (P.flip_w >> q.g) & 1u;
         if (q.strip == 0) {
             const bool fh = (P.flip_h >> q.g) & 1u;
@@ -134,34 +135,31 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
     auto RL = [&]() -> int64_t { return KEEP ? P.NL : 32; };      // between the four parts of a block's row of h
     const int64_t up = KEEP ? (int64_t)P.nstrip * 4 * P.NL : 0;   // from a block's row of h back to the one above it
     auto place = [&](const BkPos &q) {   // at the start of a row of blocks
-        const int blk = q.pass * rw + w;
+        const int blk = q.row;
         const int64_t lin = ((int64_t)q.bg * P.nsl + min(q.slot + sl_, P.nsl - 1)) * P.NS + min(n, P.NS - 1);
         nbc = reinterpret_cast<const unsigned char *>(P.bc + ((int64_t)q.bg * P.nblk + blk) * P.nstrip * BK_PX * NG);
         if constexpr (KEEP) nrow = P.row + (int64_t)blk * P.nstrip * 4 * P.NL + lin;
-        else nrow = P.row + (int64_t)(first + (warp >> P.rwl)) * P.nstrip * 4 * 32 + lane;   // (an item's first row of blocks reads nothing)
+        else nrow = P.row + (int64_t)first * P.nstrip * 4 * 32 + lane;   // (an item's first row of blocks reads nothing)
         ncol = P.col + ((int64_t)blk * (P.nstrip - 1) - 1) * 4 * P.NL + lin;
     };
     auto above = [&](const float4 *row, int qt, bool there) { return bk_ld16<false>(row - up + qt * RL(), there); };   // a quarter of the row above the one at `row`
-    auto enter = [&](const BkPos &q) {   // the first block after a pause: everything its predecessor would have started
-        place(q);
-        load_raw(q);
-        copy_bc(nbc, 0, true); copy_bc(nbc, 1, true); copy_bc(nbc, 2, true);
-        const bool there = q.pass * rw + w > 0;
-        up0 = above(nrow, 0, there); up1 = above(nrow, 1, there);
+    // the first half of the row above of a row of blocks' first block; false: the wait for it ran out
+    auto enter_row = [&](const BkPos &q) {
+        if (rw > 1 && !rs.wait(q.seq)) return false;
+        up0 = above(nrow, 0, q.row > 0); up1 = above(nrow, 1, q.row > 0);
+        return true;
     };
-    if (w == 0 && live(pos, 0)) enter(pos);
-    for (int g = 0; g < steps; ++g) {
-        const int L = g - BK_LAG * w;
+    bool fresh = true, ok = true;   // the block is the first of its item; no wait has run out
+    if (pos.item < P.items) {
+        place(pos);
+        load_raw(pos);
+        copy_bc(nbc, 0, true); copy_bc(nbc, 1, true); copy_bc(nbc, 2, true);
+        ok = enter_row(pos);
+    }
+    while (ok && pos.item < P.items) {
         BkPos nxt = pos;
-        if (L >= 0) nxt.next(P, SPW, stride);
-        const bool non = live(nxt, L + 1);
-        if (!live(pos, L)) {   // before the worker's first block, past its last row of blocks, or past its items
-            if (non) enter(nxt);
-            if (rw > 1) __syncthreads();
-            pos = nxt;
-            continue;
-        }
-        const int blk = pos.pass * rw + w, G0 = pos.g;
+        const bool leave = nxt.next(P, SPW, rw, stride), non = nxt.item < P.items;
+        const int blk = pos.row, G0 = pos.g;
         const unsigned char *tbc = nbc;
         float4 *trow = nrow, *tcol = ncol;
         if (nxt.strip == 0) { if (non) place(nxt); }
@@ -175,7 +173,7 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
                 const int r = r0 + ((lane >> 2) & 3), c = lane & 3;
                 oo = (int64_t)(pos.bg / P.G) * P.o_bs + (int64_t)((P.mw ? ch0 : cg) + 2 * (lane >> 4)) * P.o_ds +
                      (int64_t)(fh ? P.H - 1 - r : r) * P.o_hs + (fw ? P.W - 1 - c : c);
-                if (pos.pass == 0) {   // a new item
+                if (fresh) {   // a new item
                     const int c0 = min(2 * sl_, nch - 1), c1 = min(2 * sl_ + 1, nch - 1);
                     const float *a = P.A + (int64_t)cg * P.A_ds + n * P.A_ns;
                     A2 = n < P.N ? f2(__ldg(a + c0 * P.A_ds) * LOG2E, __ldg(a + c1 * P.A_ds) * LOG2E) : bc(0.f);
@@ -224,17 +222,18 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
         // 1298), and so is a test per column (1394).
         const float4 *tIn = sIn + sl_ * 33;
         const float2 *tTop = sTop + sl_ * 9;
-        const bool nthere = non && nxt.pass * rw + w > 0;
+        const bool ahead = non && (rw == 1 || nxt.strip > 0);   // (with row workers the first block of a row is waited for when this one is done)
 #pragma unroll
         for (int qt = 0; qt < 4; ++qt) {
             bk_wait<2>();
             __syncwarp();   // this quarter's B and C are here, the quarter before it has been read by all lanes
             copy_bc(qt == 0 ? tbc : nbc, (qt + 3) & 3, qt == 0 || non);
-            // The row of h above travels two quarters ahead.  What a load reads was written two quarters (by this thread) or at least two
-            // steps ago (by another worker).
+            // The row of h above travels two quarters ahead.  What a load reads was written two quarters ago by this thread, or by a worker
+            // that has been waited for.
+            if (qt == 2 && rw > 1 && ahead) ok = rs.wait(nxt.seq);
             const float4 hup = up0;
             up0 = up1;
-            up1 = qt < 2 ? above(trow, qt + 2, blk > 0) : above(nrow, qt - 2, nthere);
+            up1 = qt < 2 ? above(trow, qt + 2, blk > 0) : above(nrow, qt - 2, ahead && nxt.row > 0);
             if (pos.strip * BK_S + 2 * qt < P.W) {
                 const float4 *qIn = tIn + qt * 2;
                 const float2 *tBC = sBC + qt * 8 * NG + (NG == 16 ? (n & 7) * 2 + (n >> 3) : n);
@@ -303,16 +302,21 @@ __global__ void __launch_bounds__(BK_WARPS * 32, 4) blk_fwd_kernel(const __grid_
             }
             __syncwarp();
         }
-        if (rw > 1) __syncthreads();   // the rows of h written in this step are there for the other workers
+        if (rw > 1) {
+            rs.done(pos.seq);
+            if (non && nxt.strip == 0) ok = enter_row(nxt);
+        }
         pos = nxt;
+        fresh = leave;
     }
+    if (!ok) rs.abandon(P.status);
     bk_wait<0>();
 }
 
 template <int NG, int DT, bool KEEP>
 static cudaError_t launch(const Blk &P, cudaStream_t st) {
     auto kernel = blk_fwd_kernel<NG, DT, KEEP>;
-    constexpr int smem = BkFwd<NG>::total * BK_WARPS;
+    constexpr int smem = BkFwd<NG>::total * BK_MAXRW;
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -322,7 +326,7 @@ static cudaError_t launch(const Blk &P, cudaStream_t st) {
         if (dev >= 0 && dev < 64) attr_done[dev] = true;
     }
     blk_bc_kernel<DT><<<P.nblk * P.nstrip * (P.items / P.ntile), 128, 0, st>>>(P, NG);
-    kernel<<<P.grid, BK_WARPS * 32, smem, st>>>(P);
+    kernel<<<P.grid, P.warps * 32, BkFwd<NG>::total * P.warps, st>>>(P);
     return cudaGetLastError();
 }
 template <int NG, int DT>

@@ -121,7 +121,7 @@ enum { VEC_U = 1, VEC_DELTA = 2, VEC_B = 4, VEC_C = 8, VEC_OUT = 16, VEC_DU = 32
 // Device-side status word of the library (0 = fine).  A kernel that gives up on a
 // bounded wait records why here instead of spinning; the host reads and clears it
 // through cs2d_device_status().
-enum { ERR_BULK_COPY_TIMEOUT = 1, ERR_STAGE_TIMEOUT = 2 };
+enum { ERR_BULK_COPY_TIMEOUT = 1, ERR_STAGE_TIMEOUT = 2, ERR_WORKER_TIMEOUT = 4 };
 
 // ---- packed fp32x2 helpers -------------------------------------------------
 __device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }

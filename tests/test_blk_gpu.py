@@ -1,5 +1,5 @@
 """The block-walk kernels (two or more states, at least eight channels per group) against the float64 oracle: images of
-one block and less, ragged in both directions, one to four row workers per CTA, odd channel counts (a slot with one live
+one block and less, ragged in both directions, one to eight row workers per CTA, odd channel counts (a slot with one live
 half), every number of state slots, delta shared by channels (the addresses of neighbouring channels coincide), fp32
 results of 16-bit inputs, rows that do and do not allow groups of four, state decay, and the deterministic
 backward, which makes the tile kernels' checkpoints again."""
@@ -22,6 +22,8 @@ CASES = [
     ((1, 1, 11, 9, 40, 7), torch.float32, {}),         # one block per row: the row of h stays in registers or waits for the workers
     ((3, 1, 10, 16, 9, 33), torch.bfloat16, {}),       # 5 blocks per row, two row workers with a short last pass
     ((1, 2, 12, 5, 27, 70), torch.float16, {}),        # 9 blocks per row, four row workers
+    ((1, 1, 9, 16, 61, 21), torch.bfloat16, {}),       # 16 rows of 3 blocks, eight row workers: none starts before the one before it
+    ((1, 1, 12, 6, 35, 130), torch.float32, {}),       # 9 rows, eight row workers: one of them has two
     ((1, 1, 16, 16, 16, 64), torch.float32, {"delta_dim": 4}),
     ((2, 1, 8, 7, 13, 20), torch.float32, {"a_decay": 0.9, "with_bias": False}),
     ((1, 4, 8, 16, 12, 300), torch.float32, {"with_D": False}),   # wider than a tile launch
@@ -117,3 +119,35 @@ def test_four_corner_merge(shape, dtype):
     for k in host:
         check_close("d" + k, dev[k].grad.float().cpu().numpy(), ref[k].grad.numpy(), rtol, atol)
     assert cs2d.device_status() == 0
+
+
+def _places(t, how, n):
+    """The same values `n` elements into a buffer, or in rows that are `n` elements longer than the image is wide."""
+    if how == "offset":
+        buf = torch.zeros(t.numel() + n, dtype=t.dtype, device=t.device)
+        v = buf[n:].view(t.shape)
+    else:
+        v = torch.zeros(*t.shape[:-1], t.shape[-1] + n, dtype=t.dtype, device=t.device)[..., :t.shape[-1]]
+    v.copy_(t)
+    return v
+
+
+@pytest.mark.parametrize("dtype,out_float", [(torch.float32, False), (torch.bfloat16, False), (torch.float16, True)], ids=["fp32", "bf16", "fp16-fp32"])
+@pytest.mark.parametrize("how,n", [("offset", 1), ("offset", 2), ("offset", 4), ("pitch", 1), ("pitch", 2), ("pitch", 4)])
+@pytest.mark.parametrize("W,N", [(16, 5), (20, 12), (9, 16)])
+def test_backward_copies_of_every_width(W, N, how, n, dtype, out_float):
+    """The inputs are copied 16, 8, 4 bytes or a shifted word at a time, as their addresses and strides allow: the
+    gradients are those of contiguous inputs.  dB, dC and the parameters' gradients are sums in another order (fp32 atomics)."""
+    inp = _dev(make_inputs(2, 2, 9, N, 11, W, dtype=dtype, seed=5))
+    dout = inp["dout"].float() if out_float else inp["dout"]
+    rest = (inp["A"], inp["B"], inp["C"], inp["D"], inp["delta_bias"])
+    def grads(u, delta, g):
+        _, x, xv, xsd = cs2d.fwd(u, delta, *rest, True, out_float, None)
+        return cs2d.bwd(u, delta, *rest, g, x, xv, True, None, xsd)
+    ref = grads(inp["u"], inp["delta"], dout)
+    got = grads(_places(inp["u"], how, n), _places(inp["delta"], how, n), _places(dout, how, n))
+    for name, a, b in zip(NAMES, ref, got):
+        if name in ("du", "ddelta"):
+            assert torch.equal(a, b), name
+        elif a is not None:
+            check_close(name, b.float().cpu().numpy(), a.float().cpu().numpy(), *TOL[str(dtype)[6:]])
