@@ -584,9 +584,14 @@ static void pair_fill(Pw &k, const cs2d_problem *p, const cs2d_dirs *o, bool bac
     for (int i = 0; i < ni; ++i)
         k.vin = std::min(k.vin, k.lin ? move_bytes(in[i].p, {in[i].bs * es, in[i].ds * es, (int64_t)PW_R * k.W * es, (int64_t)k.H * k.W * es})
                                       : move_bytes(in[i].p, {in[i].bs * es, in[i].ds * es, in[i].hs * es, (int64_t)k.W * es}));
+    k.al = 16;
+    for (int i = 0; i < ni; ++i)
+        k.al = std::min(k.al, k.lin ? move_bytes(in[i].p, {in[i].bs * es, in[i].ds * es, (int64_t)PW_R * k.W * es, (int64_t)k.H * k.W * es}, 16)
+                                    : move_bytes(in[i].p, {in[i].bs * es, in[i].ds * es, in[i].hs * es, (int64_t)k.W * es}, 16));
     if (k.W & 1) k.vin = std::min(k.vin, es);
     k.el = k.vin < 2 * es;
     if (k.vin < 4) k.vin = 4;
+    k.ck = !k.el && (k.al == 16 || (!backward && k.lin && 16 - k.al + PW_R * k.W * es <= 128));   // (how far that is worth it: see there)
     k.fs = k.el && es == 2 && !k.lin ? 8 : 32 / es;
     k.nstrip = k.lin ? 1 : (k.W + k.fs - 1) / k.fs;
     k.lpin = k.lin ? lanes_for((PW_R * k.W * es + (k.el && es == 2 ? 2 : 0) + k.vin - 1) / k.vin) : 4 * (k.el && es == 2 ? 8 : 32 / k.vin);
@@ -611,11 +616,11 @@ static size_t pair_col_bytes(const Pw &k) { return (size_t)k.items * k.nblk * (k
 // pieces of results that take the place of inputs in shared memory
 static int pair_vout(const Pw &k, const void *ptr, int es, int64_t bs, int64_t ds, int64_t hs) {
     if (k.el && es == 2) return 2;
-    if (k.lin) return move_bytes(ptr, {bs * es, ds * es, (int64_t)PW_R * k.W * es, (int64_t)k.H * k.W * es});
-    return move_bytes(ptr, {bs * es, ds * es, hs * es, (int64_t)k.W * es});
+    if (k.lin) return move_bytes(ptr, {bs * es, ds * es, (int64_t)PW_R * k.W * es, (int64_t)k.H * k.W * es}, k.ck ? 16 : 8);
+    return move_bytes(ptr, {bs * es, ds * es, hs * es, (int64_t)k.W * es}, k.ck ? 16 : 8);
 }
 static void pair_out(Pw &k, int es, int vout) {
-    k.vout = std::min(vout, k.vin);
+    k.vout = std::min(vout, k.ck ? k.al : k.vin);
     k.lpout = k.lin ? lanes_for(PW_R * k.W * es / k.vout) : 4 * k.fs * es / k.vout;
 }
 

@@ -18,6 +18,15 @@
 // ("EL"; so are fp32 blocks that only allow 4-byte pieces).  A channel's pitch in shared memory is 132 or 136 bytes, an odd
 // number of pieces.
 //
+// Where rows are whole pairs and a linear block's chunks fit 128 bytes, or rows are whole 16-byte chunks ("CK"), the 16-byte chunks of memory that
+// a block touches are copied instead (a chunk that holds an element of the tensor can be read): copies of 16 bytes pass the L1 cache
+// by - measured, 64 channels of 112 bytes: 570 cycles of a warp, in pieces of 8 or 4 bytes 3660, as 64 bulk copies 3800.  A channel then has
+// 128 bytes, a linear block's byte the place that it has in its chunks, a row's one of 32 that the low bits of its address say, chunks
+// swizzled over the lanes; an address takes an instruction more, and four lanes share a bank.  So blocks read element by element stay as they
+// are (13x13 fp32 forward and backward 150 + 322 -> 168 + 369 us, 7x7 bf16 166 + 330 -> 188 + 401), and in the backward those
+// that are not whole chunks (128x3072x14x14 bf16 607 -> 620).  us, pieces / chunks: 128x3072x14x14 bf16 forward 283 / 235,
+// 64x1536x16x16 fp32 129 + 277 / 103 + 264, four corners 8x384x112x112 bf16 655 + 1199 / 501 + 1064.
+//
 // What crosses a band or 8 columns goes through global memory, threads innermost (512 bytes per warp and access):
 //   row  [item][band][column][nl] float4 (h, h', a, a') of a band's last row (rolling: [team][column][32], one row
 //        per warp, or team of row workers, that is on the GPU at a time)
@@ -46,7 +55,8 @@ struct Pw {
     unsigned flip_h, flip_w;
     int shared;                   // bit 0: u has dpg channels shared by the groups, bit 1: dout
     int fs, lin, el;              // columns of a fetched block; whole bands; element by element
-    int vin, vout;                // bytes of a piece of the inputs (8 or 4) and of the results (8, 4 or 2)
+    int ck, al;                   // chunks; what the addresses of blocks (linear) or rows are multiples of, 16 at most
+    int vin, vout;                // bytes of a piece of the inputs (8 or 4) and of the results (16, 8, 4 or 2)
     int lpin, lpout;              // lanes (a power of two) that move a channel's block
     int v32;                      // fp32 results of 16-bit inputs (merge: images) take two elements at once
     int f32;                      // 16-bit inputs with an fp32 result (forward) or gradient (backward)
@@ -70,6 +80,16 @@ template <int DT> struct pw_io {
 __device__ __forceinline__ float2 pw_ld8(const void *p, bool on) {
     float2 v;
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t@p ld.global.nc.v2.f32 {%0,%1}, [%2];\n\t}" : "=f"(v.x), "=f"(v.y) : "l"(p), "r"((int)on));
+    return v;
+}
+
+// bk_ldp through a 16-bit register (through a 32-bit one, whose value nothing waits for, the backward is 1 to 2 % slower)
+template <int DT>
+__device__ __forceinline__ uint32_t pw_ldp(const typename bk_type<DT>::t *p, bool on) {
+    if constexpr (DT == CS2D_F32) return bk_ldp<DT>(p, on);
+    unsigned short v = 0;
+    if constexpr (DT != CS2D_F32)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b16 %0, 0;\n\t@p ld.global.nc.b16 %0, [%1];\n\t}" : "=h"(v) : "l"(p), "r"((int)on));
     return v;
 }
 
@@ -170,6 +190,52 @@ __device__ __forceinline__ void pw_store(uint32_t from, const PwBlock &b, const 
     else pw_store_v<2>(from, b, in, P);
 }
 
+// CK: place of the byte whose address has the low bits x (linear blocks: x bytes from the block's first chunk) of segment seg of channel ch
+__device__ __forceinline__ uint32_t pw_place(const Pw &P, int ch, int seg, uint32_t x) {
+    return (ch & 1) * PW_HALF + (ch >> 1) * 128 + ((P.lin ? x : seg * 32 + (x & 31)) ^ (((ch >> 1) & 7) << 4));
+}
+__device__ __forceinline__ void pw_fetch_ck(uint32_t dst, const PwBlock &b, const Pw &P, const void *safe) {
+    const int lane = threadIdx.x & 31, x = lane & 7, seg = P.lin ? 0 : x >> 1, o = P.lin ? x * 16 : (x & 1) * 16;
+    const char *src = b.p + (lane >> 3) * b.ds + seg * b.hs;
+    const int64_t add = 4 * b.ds;
+#pragma unroll 4
+    for (int ch = lane >> 3; ch < PW_CH; ch += 4) {
+        const int od = (int)(reinterpret_cast<uintptr_t>(src) & 15);
+        const char *s = src + (o - od);
+        const bool on = ch < b.nch && seg < b.nseg && o + 16 > b.lo + od && o < b.hi + od;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + pw_place(P, ch, seg, P.lin ? o : (uint32_t)reinterpret_cast<uintptr_t>(s))), "l"(on ? s : reinterpret_cast<const char *>(safe)), "r"(on ? 16 : 0) : "memory");
+        src += add;
+    }
+}
+// The way back: pieces of P.vout bytes
+template <int V>
+__device__ __forceinline__ void pw_store_ckv(uint32_t from, const PwBlock &b, const PwBlock &in, const Pw &P) {
+    const int lane = threadIdx.x & 31, step = 32 / P.lpout, x = lane & (P.lpout - 1);   // (a channel is 32 pieces at most)
+    const int seg = P.lin ? 0 : x / (P.lpout / 4), o = (P.lin ? x : x % (P.lpout / 4)) * V;
+    const bool ok = seg < b.nseg && o >= b.lo && o < b.hi;
+    char *dst = const_cast<char *>(b.p) + (lane / P.lpout) * b.ds + seg * b.hs + o;
+    const int64_t add = step * b.ds;
+    uint32_t at = (uint32_t)reinterpret_cast<uintptr_t>(in.p) + (lane / P.lpout) * (uint32_t)in.ds + seg * (uint32_t)in.hs;
+    const uint32_t iadd = step * (uint32_t)in.ds;
+#pragma unroll 8
+    for (int ch = lane / P.lpout; ch < PW_CH; ch += step) {
+        const uint32_t a = from + pw_place(P, ch, seg, (P.lin ? at & 15 : at) + o);
+        const int on = ok && ch < b.nch;
+        if constexpr (V == 16)
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 x, y, z, w;\n\tsetp.ne.b32 p, %2, 0;\n\tld.shared.v4.b32 {x,y,z,w}, [%1];\n\t@p st.global.v4.b32 [%0], {x,y,z,w};\n\t}" ::"l"(dst), "r"(a), "r"(on) : "memory");
+        else if constexpr (V == 8)
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 x, y;\n\tsetp.ne.b32 p, %2, 0;\n\tld.shared.v2.b32 {x,y}, [%1];\n\t@p st.global.v2.b32 [%0], {x,y};\n\t}" ::"l"(dst), "r"(a), "r"(on) : "memory");
+        else
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 x;\n\tsetp.ne.b32 p, %2, 0;\n\tld.shared.b32 x, [%1];\n\t@p st.global.b32 [%0], x;\n\t}" ::"l"(dst), "r"(a), "r"(on) : "memory");
+        dst += add; at += iadd;
+    }
+}
+__device__ __forceinline__ void pw_store_ck(uint32_t from, const PwBlock &b, const PwBlock &in, const Pw &P) {
+    if (P.vout == 16) pw_store_ckv<16>(from, b, in, P);
+    else if (P.vout == 8) pw_store_ckv<8>(from, b, in, P);
+    else pw_store_ckv<4>(from, b, in, P);
+}
+
 // This lane's view of an input's block: elements of two neighbouring columns
 template <int DT, bool EL>
 struct PwView {
@@ -243,15 +309,78 @@ struct PwView {
         }
     }
 };
+// The same for chunks
+struct PwLane {   // what the views of a lane share: where its channels' rows lie, the bits of an address that count
+    uint32_t base[PW_R], mask;
+    __device__ __forceinline__ void at(const Pw &P, uint32_t sm) {
+        const int lane = threadIdx.x & 31;
+        mask = P.lin ? 127 : 31;
+#pragma unroll
+        for (int r = 0; r < PW_R; ++r) base[r] = sm + lane * 128 + (((lane & 7) << 4) ^ (P.lin ? 0 : r * 32));   // (sm is a multiple of 128)
+    }
+};
+template <int DT, int AT>   // AT: where the input's block lies in the warp's shared memory
+struct PwViewCk {
+    static constexpr int ES = pw_io<DT>::ES;
+    uint32_t a[2], hs;   // low bits of the channels' addresses, or their offsets in the first chunk of linear blocks; of the step to the next segment
+    __device__ __forceinline__ void at(const Pw &P, const PwBlock &b) {
+        const uint32_t ds = (uint32_t)b.ds, m = P.lin ? 15 : ~0u, p = (uint32_t)reinterpret_cast<uintptr_t>(b.p) + 2 * (threadIdx.x & 31) * ds;
+        a[0] = p & m; a[1] = (p + ds) & m;
+        hs = (uint32_t)b.hs;
+    }
+    __device__ __forceinline__ uint32_t pair(const PwLane &L, int r, int k, int o) const { return (L.base[r] ^ ((a[k] + (r * hs + o)) & L.mask)) + (AT + k * PW_HALF); }
+    __device__ __forceinline__ void load(const PwLane &L, int r, int k, int o1, bool rev, float (&x)[2]) const {
+        const uint32_t p = pair(L, r, k, o1);
+        if constexpr (ES == 4) {
+            float lo, hi;
+            asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(lo), "=f"(hi) : "r"(p) : "memory");
+            x[0] = rev ? hi : lo; x[1] = rev ? lo : hi;
+        } else {
+            uint32_t w;
+            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w) : "r"(p) : "memory");
+            if constexpr (DT == CS2D_BF16) {
+                x[0] = __uint_as_float(rev ? w & 0xffff0000u : w << 16); x[1] = __uint_as_float(rev ? w << 16 : w & 0xffff0000u);
+            } else {
+                x[0] = bk_cvt<DT>(rev ? w >> 16 : w & 0xffffu); x[1] = bk_cvt<DT>(rev ? w & 0xffffu : w >> 16);
+            }
+        }
+    }
+    __device__ __forceinline__ void store(const PwLane &L, int r, int k, int o1, bool rev, float x0, float x1) const {
+        const uint32_t p = pair(L, r, k, o1);
+        const float lo = rev ? x1 : x0, hi = rev ? x0 : x1;
+        if constexpr (ES == 4) {
+            asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(p), "f"(lo), "f"(hi) : "memory");
+        } else {
+            uint32_t w;
+            if constexpr (DT == CS2D_BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(hi), "f"(lo));
+            else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(hi), "f"(lo));
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(p), "r"(w) : "memory");
+        }
+    }
+};
 // Offsets of the columns c, c + 1 (c counts from the block's first) in a block's rows: o[r], and o1[r] for PwView
-template <int ES, bool EL>
+template <int ES, bool EL, bool CK = false>
 __device__ __forceinline__ void pw_offsets(const Pw &P, int c, bool fh, bool fw, int (&o)[PW_R], int (&o1)[PW_R]) {
     const int width = P.lin ? P.W : P.fs, mc = fw ? width - 1 - c : c, mc1 = EL ? (fw ? mc - 1 : mc + 1) : (fw ? mc - 1 : mc);
 #pragma unroll
     for (int r = 0; r < PW_R; ++r) {
-        const int row = P.lin ? (fh ? PW_R - 1 - r : r) * P.W * ES : r * 32;
+        const int row = P.lin ? (fh ? PW_R - 1 - r : r) * P.W * ES : CK ? 0 : r * 32;   // (CK: the views count the rows)
         o[r] = row + mc * ES;
         o1[r] = row + mc1 * ES;
+    }
+}
+
+// CK: rows of a linear block that the image does not have share chunks with others: zeros in their place
+template <int ES, typename... Views>
+__device__ __forceinline__ void pw_clear(const Pw &P, const PwLane &L, int r0, bool fh, bool fw, const Views &...v) {
+    if (!P.lin || r0 + PW_R <= P.H) return;
+#pragma unroll 1
+    for (int c = 0; c < P.W; c += 2) {
+        int o[PW_R], o1[PW_R];
+        pw_offsets<ES, false, true>(P, c, fh, fw, o, o1);
+#pragma unroll
+        for (int r = 1; r < PW_R; ++r)
+            if (r0 + r >= P.H) { (v.store(L, r, 0, o1[r], false, 0.f, 0.f), ...); (v.store(L, r, 1, o1[r], false, 0.f, 0.f), ...); }
     }
 }
 
@@ -269,8 +398,8 @@ template <int DT> struct PwBC {
             const int px = i * 32 + lane, r = r0 + px / FS, cc = c0 + px % FS;   // (more columns than a narrow block has: not used)
             const bool on = r < P.H && cc < P.W;
             const int fr = fh ? P.H - 1 - r : r, fc = fw ? P.W - 1 - cc : cc;
-            b[i] = bk_ldp<DT>(B + (int64_t)fr * P.B_hs + fc, on);
-            c[i] = bk_ldp<DT>(C + (int64_t)fr * P.C_hs + fc, on);
+            b[i] = pw_ldp<DT>(B + (int64_t)fr * P.B_hs + fc, on);
+            c[i] = pw_ldp<DT>(C + (int64_t)fr * P.C_hs + fc, on);
         }
     }
     __device__ __forceinline__ void put(float2 *s) const {

@@ -32,7 +32,7 @@ __device__ __forceinline__ void tm_wait_ld8(float2 (&x)[4]) {
 }
 
 // DIRS: flips, shared channels or the merge.  G32: 16-bit inputs with an fp32 gradient (read without staging).
-template <int DT, bool DIRS, bool EL, bool G32>
+template <int DT, bool DIRS, bool EL, bool G32, bool CK>
 __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid_constant__ Pw P) {
     using S = PwBwd;
     constexpr int ES = pw_io<DT>::ES, FS = pw_io<DT>::FS;
@@ -60,6 +60,8 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
     auto blk_of = [&](const PwPos &q) { return P.nblk - 1 - (q.pass * rw + w); };     // bands from the bottom up, blocks from the right
     auto live = [&](const PwPos &q, int L) { return L >= 0 && L < lmax && q.item < P.items && q.strip < P.nstrip && q.pass * rw + w < P.nblk; };
     const int lp = min(lane, P.nl - 1);   // this lane's place in the checkpoints
+    PwLane PL;
+    if constexpr (CK) PL.at(P, sm);
     PwBC<DT> bcr;
     auto blocks = [&](const PwPos &q, auto &&f) {   // f(delta's block, u's, dout's) of a position
         const int r0 = blk_of(q) * PW_R, c0 = (P.nstrip - 1 - q.strip) * P.fs, ch0 = q.tile * PW_CH, cg = q.g * P.dpg + ch0, b = q.bg / P.G, nch = P.dpg - ch0;
@@ -70,6 +72,11 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
     };
     auto start = [&](const PwPos &q) {   // fetch a block
         blocks(q, [&](const PwBlock &d, const PwBlock &u, const PwBlock &g) {
+            if constexpr (CK) {
+                pw_fetch_ck(sm + S::delta, d, P, P.delta); pw_fetch_ck(sm + S::u, u, P, P.u);
+                if constexpr (!G32) pw_fetch_ck(sm + S::g, g, P, P.out);
+                return;
+            }
             if (!EL && P.vin == 8) {
                 pw_fetch<8, false>(sm + S::delta, d, P, P.delta); pw_fetch<8, false>(sm + S::u, u, P, P.u);
                 if constexpr (!G32) pw_fetch<8, false>(sm + S::g, g, P, P.out);
@@ -145,7 +152,15 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
         };
         load_group((nc - 1) & ~7);
         PwView<DT, EL> vd, vu, vg;
+        PwViewCk<DT, S::delta> cd;
+        PwViewCk<DT, S::u> cu;
+        PwViewCk<DT, S::g> cg_;
         blocks(pos, [&](const PwBlock &d, const PwBlock &u, const PwBlock &g) {
+            if constexpr (CK) {
+                cd.at(P, d); cu.at(P, u);
+                if constexpr (!G32) cg_.at(P, g);
+                return;
+            }
             const int pit = P.vin == 8 ? 136 : 132;
             vd.at(sm + S::delta, d, pit); vu.at(sm + S::u, u, pit);
             if constexpr (!G32) vg.at(sm + S::g, g, pit);
@@ -153,6 +168,8 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
         bcr.put(sBC);
         bk_wait<0>();
         __syncwarp();
+        if constexpr (CK && G32) pw_clear<ES>(P, PL, r0, fh, fw, cd, cu);
+        else if constexpr (CK) pw_clear<ES>(P, PL, r0, fh, fw, cd, cu, cg_);
         const int64_t HW = (int64_t)P.H * P.W;
         const bool merge = DIRS && P.mw;
 #pragma unroll 1
@@ -175,12 +192,15 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
                     else load_back(c);
                     const bool on1 = c + 1 < nc;
                     int o[PW_R], o1[PW_R];
-                    pw_offsets<ES, EL>(P, c, fh, fw, o, o1);
+                    pw_offsets<ES, EL, CK>(P, c, fh, fw, o, o1);
                     float xd[PW_R][2][2], xu[PW_R][2][2];   // row, channel, column
 #pragma unroll
                     for (int r = 0; r < PW_R; ++r)
 #pragma unroll
-                        for (int k = 0; k < 2; ++k) { vd.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xd[r][k]); vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]); }
+                        for (int k = 0; k < 2; ++k) {
+                            if constexpr (CK) { cd.load(PL, r, k, o1[r], fw, xd[r][k]); cu.load(PL, r, k, o1[r], fw, xu[r][k]); continue; }
+                            vd.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xd[r][k]); vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]);
+                        }
                     const uint32_t tt = tm + (c - c1) * 32;
 #pragma unroll
                     for (int cc = 0; cc < 2; ++cc) {
@@ -213,7 +233,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
                 if (c > c1) load_back(c - 2);
                 else if (c1 > 0) load_group(c1 - 8);
                 int o[PW_R], o1[PW_R];
-                pw_offsets<ES, EL>(P, c, fh, fw, o, o1);
+                pw_offsets<ES, EL, CK>(P, c, fh, fw, o, o1);
                 const bool on1 = c + 1 < nc;
                 float xg[PW_R][2][2], xu[PW_R][2][2];   // row, channel, column
 #pragma unroll
@@ -226,9 +246,11 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
                             const bool on = r0 + r < P.H && 2 * lane + k < nch;
                             xg[r][k][0] = __uint_as_float(bk_ldp<CS2D_F32>(src + fc, on)); xg[r][k][1] = __uint_as_float(bk_ldp<CS2D_F32>(src + (fw ? fc - 1 : fc + 1), on && on1));
                         } else {
-                            vg.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xg[r][k]);
+                            if constexpr (CK) cg_.load(PL, r, k, o1[r], fw, xg[r][k]);
+                            else vg.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xg[r][k]);
                         }
-                        vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]);
+                        if constexpr (CK) cu.load(PL, r, k, o1[r], fw, xu[r][k]);
+                        else vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]);
                     }
                 const uint32_t tt = tm + (c - c1) * 32;
                 float2 rv[2][4];
@@ -281,10 +303,16 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
                     }
                 } else {
 #pragma unroll
-                    for (int r = 0; r < PW_R; ++r) { vu.store(r, 0, o[r], o1[r], fw, du[r][0].x, du[r][1].x, on1); vu.store(r, 1, o[r], o1[r], fw, du[r][0].y, du[r][1].y, on1); }
+                    for (int r = 0; r < PW_R; ++r) {
+                        if constexpr (CK) { cu.store(PL, r, 0, o1[r], fw, du[r][0].x, du[r][1].x); cu.store(PL, r, 1, o1[r], fw, du[r][0].y, du[r][1].y); continue; }
+                        vu.store(r, 0, o[r], o1[r], fw, du[r][0].x, du[r][1].x, on1); vu.store(r, 1, o[r], o1[r], fw, du[r][0].y, du[r][1].y, on1);
+                    }
                 }
 #pragma unroll
-                for (int r = 0; r < PW_R; ++r) { vd.store(r, 0, o[r], o1[r], fw, dd[r][0].x, dd[r][1].x, on1); vd.store(r, 1, o[r], o1[r], fw, dd[r][0].y, dd[r][1].y, on1); }
+                for (int r = 0; r < PW_R; ++r) {
+                        if constexpr (CK) { cd.store(PL, r, 0, o1[r], fw, dd[r][0].x, dd[r][1].x); cd.store(PL, r, 1, o1[r], fw, dd[r][0].y, dd[r][1].y); continue; }
+                        vd.store(r, 0, o[r], o1[r], fw, dd[r][0].x, dd[r][1].x, on1); vd.store(r, 1, o[r], o1[r], fw, dd[r][0].y, dd[r][1].y, on1);
+                    }
                 // dB, dC of the two columns: a lane sums a quarter of a pixel's 32 pairs
                 __syncwarp();
                 const float4 *src = reinterpret_cast<const float4 *>(sPart + (lane & 7) * S::PP + (lane >> 3) * 8);
@@ -309,6 +337,11 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
         {
             const int64_t o = ((int64_t)b * P.dpg * P.G + cg) * HW;
             blocks(pos, [&](const PwBlock &d, const PwBlock &u, const PwBlock &) {
+                if constexpr (CK) {
+                    if (!merge) pw_store_ck(sm + S::u, pw_block<DT>(P.du, o, HW, P.W, nch, r0, c0, P, fh, fw), u, P);
+                    pw_store_ck(sm + S::delta, pw_block<DT>(P.ddelta, o, HW, P.W, nch, r0, c0, P, fh, fw), d, P);
+                    return;
+                }
                 if (!merge) pw_store(sm + S::u, pw_block<DT>(P.du, o, HW, P.W, nch, r0, c0, P, fh, fw), u, P);
                 pw_store(sm + S::delta, pw_block<DT>(P.ddelta, o, HW, P.W, nch, r0, c0, P, fh, fw), d, P);
             });
@@ -337,9 +370,9 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 2) pair_bwd_kernel(const __grid
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm_base), "r"(256));
 }
 
-template <int DT, bool DIRS, bool EL, bool G32>
+template <int DT, bool DIRS, bool EL, bool G32, bool CK>
 static cudaError_t launch(const Pw &P, cudaStream_t st) {
-    auto kernel = pair_bwd_kernel<DT, DIRS, EL, G32>;
+    auto kernel = pair_bwd_kernel<DT, DIRS, EL, G32, CK>;
     constexpr int smem = PwBwd::total * PW_WARPS;
     static bool attr_done[64] = {};
     int dev = 0;
@@ -355,10 +388,12 @@ static cudaError_t launch(const Pw &P, cudaStream_t st) {
 template <int DT>
 static cudaError_t launch_dt(const Pw &P, cudaStream_t st) {
     if constexpr (DT != CS2D_F32) {
-        if (P.f32) return P.el ? launch<DT, true, true, true>(P, st) : launch<DT, true, false, true>(P, st);
+        if (P.f32) return P.ck ? launch<DT, true, false, true, true>(P, st) : P.el ? launch<DT, true, true, true, false>(P, st) : launch<DT, true, false, true, false>(P, st);
     }
-    if (P.flip_h || P.flip_w || P.shared || P.mw) return P.el ? launch<DT, true, true, false>(P, st) : launch<DT, true, false, false>(P, st);
-    return P.el ? launch<DT, false, true, false>(P, st) : launch<DT, false, false, false>(P, st);
+    const bool dirs = P.flip_h || P.flip_w || P.shared || P.mw;
+    if (P.ck) return dirs ? launch<DT, true, false, false, true>(P, st) : launch<DT, false, false, false, true>(P, st);
+    if (dirs) return P.el ? launch<DT, true, true, false, false>(P, st) : launch<DT, true, false, false, false>(P, st);
+    return P.el ? launch<DT, false, true, false, false>(P, st) : launch<DT, false, false, false, false>(P, st);
 }
 cudaError_t launch_pair_bwd(const Pw &P, cudaStream_t st) {
     switch (P.io_dt) {

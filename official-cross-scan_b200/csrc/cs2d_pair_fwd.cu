@@ -9,7 +9,7 @@ struct PwFwd {   // a warp's shared memory
 };
 
 // KEEP: a backward follows.  DIRS: flips, shared channels, the merge, or fp32 results of 16-bit inputs.
-template <int DT, bool KEEP, bool DIRS, bool EL>
+template <int DT, bool KEEP, bool DIRS, bool EL, bool CK>
 __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid_constant__ Pw P) {
     constexpr int ES = pw_io<DT>::ES, FS = pw_io<DT>::FS;
     extern __shared__ __align__(128) unsigned char smem_[];
@@ -25,6 +25,8 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
     pos.decode(P);
     auto live = [&](const PwPos &q, int L) { return L >= 0 && L < lmax && q.item < P.items && q.strip < P.nstrip && q.pass * rw + w < P.nblk; };
     const int lp = min(lane, P.nl - 1);   // this lane's place in the checkpoints
+    PwLane PL;
+    if constexpr (CK) PL.at(P, sm);
     PwBC<DT> bcr;
     auto blocks = [&](const PwPos &q, auto &&f) {   // f(delta's block, u's block) of a position
         const int r0 = (q.pass * rw + w) * PW_R, c0 = q.strip * P.fs, ch0 = q.tile * PW_CH, cg = q.g * P.dpg + ch0, b = q.bg / P.G, nch = P.dpg - ch0;
@@ -34,6 +36,7 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
     };
     auto start = [&](const PwPos &q) {   // fetch a block
         blocks(q, [&](const PwBlock &d, const PwBlock &u) {
+            if constexpr (CK) { pw_fetch_ck(sm + PwFwd::delta, d, P, P.delta); pw_fetch_ck(sm + PwFwd::u, u, P, P.u); return; }
             if (!EL && P.vin == 8) { pw_fetch<8, false>(sm + PwFwd::delta, d, P, P.delta); pw_fetch<8, false>(sm + PwFwd::u, u, P, P.u); }
             else { pw_fetch<4, EL>(sm + PwFwd::delta, d, P, P.delta); pw_fetch<4, EL>(sm + PwFwd::u, u, P, P.u); }
         });
@@ -82,10 +85,16 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
             hcorner = bc(0.f);
         }
         PwView<DT, EL> vd, vu;
-        blocks(pos, [&](const PwBlock &d, const PwBlock &u) { vd.at(sm + PwFwd::delta, d, P.vin == 8 ? 136 : 132); vu.at(sm + PwFwd::u, u, P.vin == 8 ? 136 : 132); });
+        PwViewCk<DT, PwFwd::delta> cd;
+        PwViewCk<DT, PwFwd::u> cu;
+        blocks(pos, [&](const PwBlock &d, const PwBlock &u) {
+            if constexpr (CK) { cd.at(P, d); cu.at(P, u); }
+            else { vd.at(sm + PwFwd::delta, d, P.vin == 8 ? 136 : 132); vu.at(sm + PwFwd::u, u, P.vin == 8 ? 136 : 132); }
+        });
         bcr.put(sBC);
         bk_wait<0>();
         __syncwarp();
+        if constexpr (CK) pw_clear<ES>(P, PL, r0, fh, fw, cd, cu);
 #pragma unroll 1
         for (int c = 0; c < nc; c += 2) {
             if (KEEP && c0 + c > 0 && ((c0 + c) & 7) == 0) {   // the column left of a group of 8
@@ -98,12 +107,15 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
             }
             const bool on1 = c + 1 < nc;
             int o[PW_R], o1[PW_R];
-            pw_offsets<ES, EL>(P, c, fh, fw, o, o1);
+            pw_offsets<ES, EL, CK>(P, c, fh, fw, o, o1);
             float xd[PW_R][2][2], xu[PW_R][2][2];   // row, channel, column
 #pragma unroll
             for (int r = 0; r < PW_R; ++r)
 #pragma unroll
-                for (int k = 0; k < 2; ++k) { vd.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xd[r][k]); vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]); }
+                for (int k = 0; k < 2; ++k) {
+                    if constexpr (CK) { cd.load(PL, r, k, o1[r], fw, xd[r][k]); cu.load(PL, r, k, o1[r], fw, xu[r][k]); continue; }
+                    vd.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xd[r][k]); vu.load(r, k, o[r], o1[r], fw, r0 + r < P.H, on1, xu[r][k]);
+                }
             const float2 hu2[2] = {f2(up[0].x, up[0].y), f2(up[1].x, up[1].y)}, au2[2] = {f2(up[0].z, up[0].w), f2(up[1].z, up[1].w)};
             if (c + 2 < nc) fetch_up(c + 2);
             float2 y[PW_R][2];
@@ -137,13 +149,18 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
                 }
             } else {
 #pragma unroll
-                for (int r = 0; r < PW_R; ++r) { vu.store(r, 0, o[r], o1[r], fw, y[r][0].x, y[r][1].x, on1); vu.store(r, 1, o[r], o1[r], fw, y[r][0].y, y[r][1].y, on1); }
+                for (int r = 0; r < PW_R; ++r) {
+                    if constexpr (CK) { cu.store(PL, r, 0, o1[r], fw, y[r][0].x, y[r][1].x); cu.store(PL, r, 1, o1[r], fw, y[r][0].y, y[r][1].y); continue; }
+                    vu.store(r, 0, o[r], o1[r], fw, y[r][0].x, y[r][1].x, on1); vu.store(r, 1, o[r], o1[r], fw, y[r][0].y, y[r][1].y, on1);
+                }
             }
         }
         __syncwarp();
         if (!DIRS || !(P.mw || P.f32)) {
             blocks(pos, [&](const PwBlock &, const PwBlock &u) {
-                pw_store(sm + PwFwd::u, pw_block<DT>(P.out, (int64_t)b * P.o_bs + (int64_t)cg * P.o_ds, P.o_ds, P.o_hs, nch, r0, c0, P, fh, fw), u, P);
+                const PwBlock y = pw_block<DT>(P.out, (int64_t)b * P.o_bs + (int64_t)cg * P.o_ds, P.o_ds, P.o_hs, nch, r0, c0, P, fh, fw);
+                if constexpr (CK) pw_store_ck(sm + PwFwd::u, y, u, P);
+                else pw_store(sm + PwFwd::u, y, u, P);
             });
             __syncwarp();
         }
@@ -154,9 +171,9 @@ __global__ void __launch_bounds__(PW_WARPS * 32, 3) pair_fwd_kernel(const __grid
     bk_wait<0>();
 }
 
-template <int DT, bool KEEP, bool DIRS, bool EL>
+template <int DT, bool KEEP, bool DIRS, bool EL, bool CK>
 static cudaError_t launch(const Pw &P, cudaStream_t st) {
-    auto kernel = pair_fwd_kernel<DT, KEEP, DIRS, EL>;
+    auto kernel = pair_fwd_kernel<DT, KEEP, DIRS, EL, CK>;
     constexpr int smem = PwFwd::total * PW_WARPS;
     static bool attr_done[64] = {};
     int dev = 0;
@@ -171,8 +188,10 @@ static cudaError_t launch(const Pw &P, cudaStream_t st) {
 }
 template <int DT, bool KEEP>
 static cudaError_t launch_el(const Pw &P, cudaStream_t st) {
-    if (P.flip_h || P.flip_w || P.shared || P.mw || P.f32) return P.el ? launch<DT, KEEP, true, true>(P, st) : launch<DT, KEEP, true, false>(P, st);
-    return P.el ? launch<DT, KEEP, false, true>(P, st) : launch<DT, KEEP, false, false>(P, st);
+    const bool dirs = P.flip_h || P.flip_w || P.shared || P.mw || P.f32;
+    if (P.ck) return dirs ? launch<DT, KEEP, true, false, true>(P, st) : launch<DT, KEEP, false, false, true>(P, st);
+    if (dirs) return P.el ? launch<DT, KEEP, true, true, false>(P, st) : launch<DT, KEEP, true, false, false>(P, st);
+    return P.el ? launch<DT, KEEP, false, true, false>(P, st) : launch<DT, KEEP, false, false, false>(P, st);
 }
 template <int DT>
 static cudaError_t launch_dt(const Pw &P, bool keep, cudaStream_t st) { return keep ? launch_el<DT, true>(P, st) : launch_el<DT, false>(P, st); }

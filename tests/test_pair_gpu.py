@@ -33,6 +33,12 @@ CASES = [
     ((150, 1, 40, 1, 6, 14), torch.bfloat16, {}),       # pieces of four bytes
     ((150, 1, 24, 1, 6, 12), torch.float16, {}),        # eight
     ((150, 2, 9, 1, 5, 22), torch.bfloat16, {}),        # two blocks per band; a short last band
+    # copied in 16-byte chunks
+    ((150, 1, 66, 1, 7, 14), torch.bfloat16, {}),       # planes and bands in the middle of chunks; a short last band
+    ((150, 1, 66, 1, 7, 16), torch.float16, {}),        # 64 of 128 bytes of a short band missing: the chunks that remain are whole
+    ((75, 2, 65, 1, 6, 8), torch.float32, {}),          # 128 bytes exactly
+    ((40, 4, 9, 1, 6, 136), torch.bfloat16, {}),        # whole chunks per row, half a block at the end of a row
+    ((5, 4, 70, 1, 7, 132), torch.float32, {}),
     ((150, 1, 64, 1, 3, 43), torch.float16, {"with_D": False}),
     ((150, 1, 11, 1, 9, 19), torch.float32, {"with_bias": False}),
     ((40, 4, 8, 1, 5, 131), torch.float32, {}),         # wider than the streaming kernels' rows
