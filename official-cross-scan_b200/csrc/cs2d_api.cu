@@ -619,7 +619,11 @@ static int pair_vout(const Pw &k, const void *ptr, int es, int64_t bs, int64_t d
     if (k.lin) return move_bytes(ptr, {bs * es, ds * es, (int64_t)PW_R * k.W * es, (int64_t)k.H * k.W * es}, k.ck ? 16 : 8);
     return move_bytes(ptr, {bs * es, ds * es, hs * es, (int64_t)k.W * es}, k.ck ? 16 : 8);
 }
+// `vout`: bytes of a piece that every result which leaves through shared memory allows (16: none of the call's does)
 static void pair_out(Pw &k, int es, int vout) {
+    // Chunks have no stores of single 16-bit elements, and their blocks are 32 pieces per channel at most: results that lie in the middle of
+    // words (a view's, given by the caller) leave the form without chunks instead
+    if (vout < 4) k.ck = 0;
     k.vout = std::min(vout, k.ck ? k.al : k.vin);
     k.lpout = k.lin ? lanes_for(PW_R * k.W * es / k.vout) : 4 * k.fs * es / k.vout;
 }
@@ -642,7 +646,7 @@ static int fwd_impl(const cs2d_problem *p, const cs2d_dirs *o, void *out, int64_
         pair_fill(k, p, o, false, out, out_bs, out_ds, out_hs);
         k.out = out; k.o_bs = out_bs; k.o_ds = out_ds; k.o_hs = out_hs;
         const int es = esize(p->io_dtype);
-        pair_out(k, es, pair_vout(k, out, es, out_bs, out_ds, out_hs));
+        pair_out(k, es, k.mw || k.f32 ? 16 : pair_vout(k, out, es, out_bs, out_ds, out_hs));
         k.v32 = move_bytes(out, {out_bs * 4, out_ds * 4, out_hs * 4, (int64_t)k.W * 4}) == 8;
         pair_state(k, saved);
         cudaError_t e = launch_pair_fwd(k, !rolling, reinterpret_cast<cudaStream_t>(stream));

@@ -2,6 +2,8 @@
 directions, one to four row workers per CTA, odd and partial channel tiles, every size of piece that rows allow, fp32
 results and gradients of 16-bit inputs, strided and misaligned views, the corner directions with their merge, and the
 deterministic backward, which makes other kernels' checkpoints again."""
+import ctypes
+
 import pytest
 import torch
 
@@ -35,7 +37,7 @@ CASES = [
     ((150, 2, 9, 1, 5, 22), torch.bfloat16, {}),        # two blocks per band; a short last band
     # copied in 16-byte chunks
     ((150, 1, 66, 1, 7, 14), torch.bfloat16, {}),       # planes and bands in the middle of chunks; a short last band
-    ((150, 1, 66, 1, 7, 16), torch.float16, {}),        # 64 of 128 bytes of a short band missing: the chunks that remain are whole
+    ((150, 1, 66, 1, 7, 16), torch.float16, {}),        # (16 columns of one orientation: the streaming kernels; chunks of them below, flipped)
     ((75, 2, 65, 1, 6, 8), torch.float32, {}),          # 128 bytes exactly
     ((40, 4, 9, 1, 6, 136), torch.bfloat16, {}),        # whole chunks per row, half a block at the end of a row
     ((5, 4, 70, 1, 7, 132), torch.float32, {}),
@@ -125,3 +127,71 @@ def test_corner_directions_and_merge(shape, dtype):
     for k in host:
         check_close("d" + k, dev[k].grad.float().cpu().numpy(), ref[k].grad.numpy(), rtol, atol)
     assert cs2d.device_status() == 0
+
+
+def _placed(shape, dtype, off, pad=0, row_pad=0, fill=None):
+    """A tensor `off` elements into its buffer, whose channels and rows end `pad` and `row_pad` elements before the next; and the rest of
+    that buffer, as a check that nothing is written there."""
+    b, c, h, w = shape
+    hs = w + row_pad
+    ds = h * hs + pad
+    buf = torch.full((off + b * c * ds + 16,), 7.0, dtype=dtype, device="cuda")
+    t = buf.as_strided(shape, (c * ds, ds, hs, 1), off)
+    if fill is not None:
+        t.copy_(fill)
+    return t, buf
+
+
+def _untouched(t, buf):
+    seen = torch.zeros_like(buf, dtype=torch.bool)
+    seen.as_strided(t.shape, t.stride(), t.storage_offset()).fill_(True)
+    return bool((buf[~seen] == 7.0).all())
+
+
+def _c_abi(d, dtype, flip=(False, False), at=0, pad=0, row_pad=0):
+    """Forward, evaluation forward and backward through the C ABI with results at `at` elements into their buffers (`out`: with
+    `pad` and `row_pad` too); every group is walked from the bottom (flip[0]) or from the right (flip[1])."""
+    p = cs2d.ops._problem(d["u"], d["delta"], d["A"], d["B"], d["C"], d["D"], d["delta_bias"], None, True, dtype, "test")
+    L, every = cs2d._lib.lib(), (1 << p.n_groups) - 1
+    dirs = cs2d._lib.Dirs(every * flip[0], every * flip[1], 0, 0, None, None)
+    ref, o, st = ctypes.byref(p), ctypes.byref(dirs), torch.cuda.current_stream().cuda_stream
+    saved, scratch, rolling = (torch.empty(f(ref, o), dtype=torch.uint8, device="cuda") for f in (
+        L.cs2d_saved_bytes_dir, L.cs2d_bwd_scratch_bytes_dir, L.cs2d_fwd_only_scratch_bytes_dir))
+    shape, dout = tuple(d["u"].shape), d["dout"]
+    out, out2 = (_placed(shape, dtype, at, pad, row_pad) for _ in range(2))
+    du, ddelta = (_placed(shape, dtype, at) for _ in range(2))
+    sums = [torch.zeros(s, device="cuda") for s in (d["A"].shape, d["B"].shape, d["C"].shape, p.dim, p.dim)]
+    assert L.cs2d_fwd_dir(ref, o, out[0].data_ptr(), *out[0].stride()[:3], saved.data_ptr(), st) == 0
+    assert L.cs2d_fwd_only(ref, o, out2[0].data_ptr(), *out2[0].stride()[:3], rolling.data_ptr(), st) == 0
+    assert L.cs2d_bwd_dir(ref, o, dout.data_ptr(), *dout.stride()[:3], saved.data_ptr(), scratch.data_ptr(), du[0].data_ptr(), ddelta[0].data_ptr(),
+                          *[t.data_ptr() for t in sums], None, st) == 0
+    assert torch.equal(out[0], out2[0])
+    for r in (out, out2, du, ddelta):
+        assert _untouched(*r)
+    return out[0], (du[0], ddelta[0], *sums)
+
+
+def _check_flipped(out, g, inp, dtype, flip):
+    """Walked from another corner: what the oracle gives for the mirrored images, mirrored."""
+    dims = [i for i, f in zip((-2, -1), flip) if f]
+    image = ("u", "delta", "B", "C", "dout")
+    m = lambda t: t.flip(dims)
+    _check(m(out), [m(t) if i in (0, 1, 3, 4) else t for i, t in enumerate(g)], {k: m(v) if k in image and dims else v for k, v in inp.items()}, dtype)
+
+
+# blocks of whole chunks, linear and by rows; linear ones that start at every fourth byte, in both directions and in the forward alone; fp32; the
+# last: element by element.  (A flip, where one orientation alone would run on the streaming kernels.)
+PLACES = [((2, 1, 66, 1, 7, 8), torch.bfloat16, (False, False)), ((150, 1, 66, 1, 8, 14), torch.bfloat16, (False, False)),
+          ((150, 1, 66, 1, 7, 14), torch.bfloat16, (False, False)), ((3, 1, 66, 1, 7, 16), torch.float16, (True, False)),
+          ((3, 2, 65, 1, 6, 8), torch.float32, (False, False)), ((3, 1, 65, 1, 6, 6), torch.float32, (False, True)),
+          ((3, 4, 9, 1, 6, 64), torch.bfloat16, (False, True)), ((2, 2, 70, 1, 7, 20), torch.float32, (True, True)),
+          ((3, 1, 66, 1, 5, 9), torch.bfloat16, (False, True))]
+
+
+@pytest.mark.parametrize("at,pad,row_pad", [(1, 0, 0), (2, 0, 0), (4, 0, 0), (0, 1, 0), (0, 2, 0), (3, 3, 1), (0, 0, 2)])
+@pytest.mark.parametrize("shape,dtype,flip", PLACES, ids=[f"{s}-{str(t)[6:]}" for s, t, _ in PLACES])
+def test_results_at_any_address(shape, dtype, flip, at, pad, row_pad):
+    """The inputs allow 16-byte chunks, the results, which a caller of the C ABI places, start at any element."""
+    inp = make_inputs(*shape, dtype=dtype, seed=at + 2)
+    out, g = _c_abi(_dev(inp), dtype, flip, at, pad, row_pad)
+    _check_flipped(out, g, inp, dtype, flip)
