@@ -142,20 +142,23 @@ __device__ __forceinline__ PwBlock pw_block(const void *base, int64_t off, int64
     return b;
 }
 
+// What copies of nothing name as their source: it has to be a multiple of the copy's size even so, which a tensor's own address need not be
+__device__ __forceinline__ const char *pw_nothing(const void *tensor) { return reinterpret_cast<const char *>(reinterpret_cast<uintptr_t>(tensor) & ~(uintptr_t)15); }
 // Fetch a block, V bytes at a time; pieces without anything that exists become zero.  EL: from the word of the first element.
 template <int V, bool EL>
-__device__ __forceinline__ void pw_fetch(uint32_t dst, const PwBlock &b, const Pw &P, const void *safe) {   // `safe`: an aligned address, named by copies of nothing
+__device__ __forceinline__ void pw_fetch(uint32_t dst, const PwBlock &b, const Pw &P, const void *tensor) {
     const int lane = threadIdx.x & 31, x = lane & (P.lpin - 1), seg = P.lin ? 0 : x / (P.lpin / 4), o = (P.lin ? x : x % (P.lpin / 4)) * V;
     const int step = 32 / P.lpin, pit = V == 8 ? 136 : 132;
     const char *src = b.p + (lane / P.lpin) * b.ds + seg * b.hs;
     const int64_t add = step * b.ds;
+    const char *nothing = pw_nothing(tensor);
     dst += seg * 32 + o;
 #pragma unroll 8
     for (int ch = lane / P.lpin; ch < PW_CH; ch += step) {
         const int od = EL ? (int)(reinterpret_cast<uintptr_t>(src) & 3) : 0;
         const bool on = ch < b.nch && seg < b.nseg && o + V > b.lo + od && o < b.hi + od;
         const char *s = src - od + o;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst + (ch & 1) * PW_HALF + (ch >> 1) * pit), "l"(on ? s : reinterpret_cast<const char *>(safe)), "n"(V), "r"(on ? V : 0) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst + (ch & 1) * PW_HALF + (ch >> 1) * pit), "l"(on ? s : nothing), "n"(V), "r"(on ? V : 0) : "memory");
         src += add;
     }
 }
@@ -194,16 +197,17 @@ __device__ __forceinline__ void pw_store(uint32_t from, const PwBlock &b, const 
 __device__ __forceinline__ uint32_t pw_place(const Pw &P, int ch, int seg, uint32_t x) {
     return (ch & 1) * PW_HALF + (ch >> 1) * 128 + ((P.lin ? x : seg * 32 + (x & 31)) ^ (((ch >> 1) & 7) << 4));
 }
-__device__ __forceinline__ void pw_fetch_ck(uint32_t dst, const PwBlock &b, const Pw &P, const void *safe) {
+__device__ __forceinline__ void pw_fetch_ck(uint32_t dst, const PwBlock &b, const Pw &P, const void *tensor) {
     const int lane = threadIdx.x & 31, x = lane & 7, seg = P.lin ? 0 : x >> 1, o = P.lin ? x * 16 : (x & 1) * 16;
     const char *src = b.p + (lane >> 3) * b.ds + seg * b.hs;
     const int64_t add = 4 * b.ds;
+    const char *nothing = pw_nothing(tensor);
 #pragma unroll 4
     for (int ch = lane >> 3; ch < PW_CH; ch += 4) {
         const int od = (int)(reinterpret_cast<uintptr_t>(src) & 15);
         const char *s = src + (o - od);
         const bool on = ch < b.nch && seg < b.nseg && o + 16 > b.lo + od && o < b.hi + od;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + pw_place(P, ch, seg, P.lin ? o : (uint32_t)reinterpret_cast<uintptr_t>(s))), "l"(on ? s : reinterpret_cast<const char *>(safe)), "r"(on ? 16 : 0) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + pw_place(P, ch, seg, P.lin ? o : (uint32_t)reinterpret_cast<uintptr_t>(s))), "l"(on ? s : nothing), "r"(on ? 16 : 0) : "memory");
         src += add;
     }
 }

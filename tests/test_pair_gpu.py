@@ -195,3 +195,18 @@ def test_results_at_any_address(shape, dtype, flip, at, pad, row_pad):
     inp = make_inputs(*shape, dtype=dtype, seed=at + 2)
     out, g = _c_abi(_dev(inp), dtype, flip, at, pad, row_pad)
     _check_flipped(out, g, inp, dtype, flip)
+
+
+@pytest.mark.parametrize("at", [(2, 0, 0), (0, 4, 4), (6, 2, 1), (1, 3, 2)], ids=str)
+@pytest.mark.parametrize("flip", [(False, False), (True, False), (False, True)], ids=["", "rows", "columns"])
+@pytest.mark.parametrize("shape,dtype", [((150, 1, 65, 1, 14, 14), torch.bfloat16), ((150, 2, 33, 1, 7, 14), torch.float16), ((150, 1, 66, 1, 8, 8), torch.bfloat16),
+                                         ((75, 1, 65, 1, 7, 8), torch.float16), ((75, 1, 66, 1, 7, 6), torch.float32)], ids=str)
+def test_inputs_at_any_address(shape, dtype, flip, at):
+    """u, delta and dout start elements into their buffers, as a view's do: the 16-byte chunks that a linear block touches begin before it, and
+    what the copies without a source name (channels that a warp has too many, rows below the image) is a multiple of 16 all the same."""
+    inp = make_inputs(*shape, dtype=dtype, seed=sum(at))
+    d = _dev(inp)
+    for name, n in zip(("u", "delta", "dout"), at):
+        d[name] = _placed(d[name].shape, dtype, n, fill=d[name])[0]
+    out, g = _c_abi(d, dtype, flip)
+    _check_flipped(out, g, inp, dtype, flip)
