@@ -329,6 +329,7 @@ __global__ void __launch_bounds__(BkBwd<NG>::WARPS * 32, 1) blk_bwd_kernel(const
             dA = bc(0.f);
             dwa = dec = bc(0.f);
             if (EXTRA) mwv = P.mw ? f2(__ldg(P.mw + cg + k0), __ldg(P.mw + cg + k1)) : bc(1.f);
+            __syncwarp();   // the item before has left its parameters: two lanes read them last, for its sums
             if (lane < SPW) {
                 const int k = 2 * lane;
                 const bool o0 = k < nch, o1 = k + 1 < nch;

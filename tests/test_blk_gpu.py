@@ -121,6 +121,25 @@ def test_four_corner_merge(shape, dtype):
     assert cs2d.device_status() == 0
 
 
+@pytest.mark.parametrize("n,batch", [(16, 250), (4, 200)])
+def test_parameters_change_with_the_item(n, batch):
+    """A warp goes through several items (a group's slots of channels) whose D and merge weights differ, the last of a group with a single
+    channel: dw and dD are sums with the item's own.  (u, B, C and dy positive: no sum cancels.)"""
+    K, dd, h, w = 4, 17, 3, 3
+    inp = make_inputs(batch, K, dd, n, h, w, dtype=torch.float32, seed=n)
+    gen = torch.Generator().manual_seed(n)
+    host = dict(u=torch.rand(batch, dd, h, w, generator=gen) + 0.1, delta=inp["delta"], A=inp["A"], B=inp["B"].abs(), C=inp["C"].abs(),
+                w=torch.rand(K, dd, generator=gen) + 0.1, D=torch.rand(K * dd, generator=gen) + 0.1, delta_bias=inp["delta_bias"])
+    dy = torch.rand(batch, dd, h, w, generator=gen) + 0.1
+    dev = {k: v.cuda().requires_grad_(True) for k, v in host.items()}
+    cs2d.cross_scan_2d(*dev.values(), True).backward(dy.cuda())
+    ref = {k: v.double().requires_grad_(True) for k, v in host.items()}
+    O.cross_fwd_torch(*ref.values(), True).backward(dy.double())
+    for k in ("w", "D"):
+        check_close("d" + k, dev[k].grad.cpu().numpy(), ref[k].grad.numpy(), *TOL["float32"])
+    assert cs2d.device_status() == 0
+
+
 def _places(t, how, n):
     """The same values `n` elements into a buffer, or in rows that are `n` elements longer than the image is wide."""
     if how == "offset":
