@@ -431,6 +431,7 @@ __global__ void __launch_bounds__(BkBwd<NG>::WARPS * 32, 1) blk_bwd_kernel(const
             float *dbc = ((lane >> 4) ? P.dC : P.dB) + ((int64_t)pos.bg * P.N + n) * HW + (int64_t)(fh ? P.H - 1 - frow : frow) * P.W;
             float2 dAt = bc(0.f);   // of this block: sums of sums
             load2(S::UC * ngrp - 1, 3);
+            tm_wait_ld(hq[1]);
 #pragma unroll 1
             for (int k = ngrp - 1; k >= 0; --k) {
                 float4 dn[PR], mb[PR], up;
@@ -450,12 +451,12 @@ __global__ void __launch_bounds__(BkBwd<NG>::WARPS * 32, 1) blk_bwd_kernel(const
 #pragma unroll
                     for (int r = BK_R - 1; r >= 0; --r) {
                         if (r == 3) {   // of the column two columns on: its terms have been asked for a column ago (at first: nothing, not used)
-                            tm_wait_ld(hq[1], x, y);
+                            if (cc < S::UC - 1) tm_wait_ld(hq[1], x, y);
                             load2(c, 1);
                             sum_states(c + 2);
                         } else if (r == 1) {
                             tm_wait_ld(hq[0]);
-                            if (cc || k) load2(c - 1, 3);
+                            load2(cc ? c - 1 : max(c - 1, 0), 3);   // (column 0 once more: not used)
                             ask_states(min(c + 1, 7));
                         }
                         const float4 in = rin[r];
@@ -495,6 +496,7 @@ __global__ void __launch_bounds__(BkBwd<NG>::WARPS * 32, 1) blk_bwd_kernel(const
                         d[0] = fold1(b3, dv[0], dv[1], 8); d[32] = fold1(b3, dv[2], dv[3], 8);
                     }
                 }
+                tm_wait_ld(hq[1], x, y);   // nothing that has been asked for crosses a branch: its registers may be copied there
                 if (blk > 0) {   // m of the block's first row
 #pragma unroll
                     for (int i = 0; i < PR; ++i) arow[(k * PR + i) * 32] = mb[i];
@@ -531,7 +533,6 @@ __global__ void __launch_bounds__(BkBwd<NG>::WARPS * 32, 1) blk_bwd_kernel(const
             }
             dA = add2(dA, dAt);
             if (non) load_col(nxt);
-            tm_wait_ld(x, y);
             sum_states(1);
             ask_states(0);
             tm_wait_ld(x, y);
