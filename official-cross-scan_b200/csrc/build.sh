@@ -19,7 +19,7 @@ if [ -z "${CS2D_OUT:-}" ]; then   # host code only: compiled while nvcc runs, li
     -c "$here/cs2d_torch.cpp" -o "$tmp/cs2d_torch.o" & native=$!
 fi
 "$NVCC" -gencode arch=compute_100a,code=sm_100a -lineinfo -O3 -std=c++17 \
-  -Xcompiler -fPIC -shared -cudart static --threads 0 "$@" -Xlinker -soname=libcs2d.so \
+  -Xcompiler -fPIC,-Wformat,-Werror=format,-Werror=format-extra-args -shared -cudart static --threads 0 "$@" -Xlinker -soname=libcs2d.so \
   -o "$out" "$here/cs2d_api.cu" "$here/cs2d_fwd.cu" "$here/cs2d_bwd.cu" "$here/cs2d_fwd_serial.cu" "$here/cs2d_bwd_serial.cu" "$here/cs2d_stream_fwd.cu" "$here/cs2d_stream_bwd.cu" "$here/cs2d_walk_fwd.cu" "$here/cs2d_blk_fwd.cu" "$here/cs2d_blk_bwd.cu" "$here/cs2d_pair_fwd.cu" "$here/cs2d_pair_bwd.cu"
 echo "built $out"
 if [ -n "$native" ]; then

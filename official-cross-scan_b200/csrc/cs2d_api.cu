@@ -29,7 +29,7 @@ int walk_channels_per_cta(int lr);
 size_t walk_bc_bytes(int batch, int groups, int nrows, int ncols);
 size_t fwd_smem_bytes(int L, int CG, int NPp, int W, int es, bool bulk, int CT, bool tiled, bool ws);
 size_t bwd_smem_bytes(int L, int CG, int NPp, int CT, bool acc, int W, int es, int eso, bool bulk, bool tiled, bool ws);
-static __device__ int g_cs2d_status = 0;  // see ERR_* in cs2d_common.cuh
+static __device__ int g_cs2d_status = 0;  // see ERR_* in cs2d_status.h
 
 // Device address of the status word on the current device (looked up once per device).
 static int *status_ptr() {
@@ -44,7 +44,7 @@ static int *status_ptr() {
 static thread_local char g_err[512] = "";
 static std::atomic<int64_t> g_launches{0};
 
-static int fail(int code, const char *fmt, ...) {
+__attribute__((format(printf, 2, 3))) static int fail(int code, const char *fmt, ...) {
     va_list ap;
     va_start(ap, fmt);
     vsnprintf(g_err, sizeof(g_err), fmt, ap);
@@ -1080,8 +1080,7 @@ int cs2d_device_status(void) {
     if (cudaMemcpyFromSymbol(&v, g_cs2d_status, sizeof(int)) != cudaSuccess) return CS2D_ERR_CUDA;
     if (v != 0) {
         cudaMemcpyToSymbol(g_cs2d_status, &zero, sizeof(int));
-        fail(CS2D_ERR_CUDA, "a kernel gave up on a bounded wait (status %d: %s%s); its outputs are invalid", v,
-             (v & ERR_BULK_COPY_TIMEOUT) ? "bulk copy " : "", (v & ERR_STAGE_TIMEOUT) ? "staging warps " : "", (v & ERR_WORKER_TIMEOUT) ? "row workers" : "");
+        status_text(g_err, sizeof(g_err), v);
     }
     return v;
 }

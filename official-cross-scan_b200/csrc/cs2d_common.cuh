@@ -30,6 +30,7 @@
 #include <stdint.h>
 
 #include "../../include/cs2d.h"
+#include "cs2d_status.h"
 
 namespace cs2d {
 
@@ -117,11 +118,6 @@ struct Dev {
 };
 enum { VEC_U = 1, VEC_DELTA = 2, VEC_B = 4, VEC_C = 8, VEC_OUT = 16, VEC_DU = 32,
        VEC_MDU = 64 };   // VEC_MDU: the merged fp32 du image of a direction merge
-
-// Device-side status word of the library (0 = fine).  A kernel that gives up on a
-// bounded wait records why here instead of spinning; the host reads and clears it
-// through cs2d_device_status().
-enum { ERR_BULK_COPY_TIMEOUT = 1, ERR_STAGE_TIMEOUT = 2, ERR_WORKER_TIMEOUT = 4 };
 
 // ---- packed fp32x2 helpers -------------------------------------------------
 __device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }

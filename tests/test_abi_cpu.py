@@ -4,6 +4,7 @@ fail loudly instead of falling back."""
 import ctypes
 import os
 import re
+import subprocess
 
 import pytest
 import torch
@@ -102,6 +103,24 @@ def test_operators_reject_cpu_tensors_and_bad_arguments():
         cs2d.fwd(u, u, A.double(), B, B, None, None, True, False, None)
     with pytest.raises(RuntimeError, match="dtype of u"):
         cs2d.fwd(u, u.half(), A, B, B, None, None, True, False, None)
+
+
+def test_status_text_names_every_reason(tmp_path):
+    """What cs2d_device_status() leaves for cs2d_last_error(): a reason for each bit, alone and with the others."""
+    src, so = tmp_path / "text.cpp", tmp_path / "text.so"
+    src.write_text(f'#include "{ROOT}/official-cross-scan_b200/csrc/cs2d_status.h"\n'
+                   'extern "C" void text(char *t, size_t n, int v) { cs2d::status_text(t, n, v); }\n')
+    subprocess.run(["g++", "-shared", "-fPIC", "-Wall", "-Werror", "-o", so, src], check=True)
+    text = ctypes.CDLL(str(so)).text
+    text.argtypes = (ctypes.c_char_p, ctypes.c_size_t, ctypes.c_int)
+    reasons = {1: "bulk copy", 2: "staging warps", 4: "row workers"}
+    for status in range(1, 8):
+        buf = ctypes.create_string_buffer(512)
+        text(buf, len(buf), status)
+        said = buf.value.decode()
+        assert f"status {status}:" in said and "outputs are invalid" in said
+        for bit, reason in reasons.items():
+            assert (reason in said) == bool(status & bit), said
 
 
 def test_missing_library_is_an_error_not_a_fallback(monkeypatch):
