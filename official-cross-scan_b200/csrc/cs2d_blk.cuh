@@ -115,11 +115,12 @@ struct RowSeq {
         __syncwarp();
         if ((threadIdx.x & 31) == 0) asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(mine), "r"(seq + 1) : "memory");
     }
-    // until the block above (in walking order) block `seq` is done.  Bounded: 2^22 polls of 20 ns or more, then false.
-    __device__ __forceinline__ bool wait(int seq) const {
+    // until the block above (in walking order) block `seq` is done.  Bounded by the number of polls
+    // (between two of them a thread sleeps 0 to 40 ns; a block takes some 10 us), then false.
+    __device__ __forceinline__ bool wait(int seq, int polls = 1 << 22) const {
         const int need = seq + 1 - nstrip;   // (of the first row of a sequence: 0 or less)
 #pragma unroll 1
-        for (int i = 0; i < (1 << 22); ++i) {
+        for (int i = 0; i < polls; ++i) {
             int have;
             asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(have) : "r"(before) : "memory");
             if (__all_sync(0xffffffffu, have >= need)) return true;

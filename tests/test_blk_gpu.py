@@ -3,10 +3,14 @@ one block and less, ragged in both directions, one to eight row workers per CTA,
 half), every number of state slots, delta shared by channels (the addresses of neighbouring channels coincide), fp32
 results of 16-bit inputs, rows that do and do not allow groups of four, state decay, and the deterministic
 backward, which makes the tile kernels' checkpoints again."""
+import ctypes
+import os
+import subprocess
+
 import pytest
 import torch
 
-from conftest import TOL, check_close
+from conftest import ROOT, TOL, check_close
 import cs2d
 from cs2d.synthetic import make_inputs
 from oracle import cs2d_oracle as O
@@ -138,6 +142,41 @@ def test_parameters_change_with_the_item(n, batch):
     for k in ("w", "D"):
         check_close("d" + k, dev[k].grad.cpu().numpy(), ref[k].grad.numpy(), *TOL["float32"])
     assert cs2d.device_status() == 0
+
+
+ROW_WAIT = r"""
+#include "cs2d_blk.cuh"
+using namespace cs2d;
+// Two row workers, three blocks per row.  Worker 1 waits for a block of worker 0 that is never counted, worker 0 for one of worker 1's.
+__global__ void row_wait_kernel(int *status, int *got) {
+    __shared__ int count[BK_MAXRW];
+    const int warp = threadIdx.x >> 5;
+    RowSeq rs;
+    rs.init(count, warp, 2, 3);
+    __syncthreads();
+    const bool ok = warp ? rs.wait(3, 1000) : rs.wait(6);
+    if (!ok) rs.abandon(status);
+    if ((threadIdx.x & 31) == 0) got[warp] = ok;
+}
+extern "C" int row_wait(int *status, int *got, void *stream) {
+    row_wait_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(status, got);
+    return cudaGetLastError();
+}
+"""
+
+
+def test_a_wait_that_runs_out_ends_with_a_status(tmp_path):
+    """The wait of a row worker, with a small number of polls: it gives up, says so, and lets the worker behind it go on."""
+    src, so = tmp_path / "row_wait.cu", tmp_path / "row_wait.so"
+    src.write_text(ROW_WAIT)
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-I",
+                    os.path.join(ROOT, "official-cross-scan_b200", "csrc"), "-o", so, src], check=True)
+    status, got = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((2,), -1, dtype=torch.int32, device="cuda")
+    f = ctypes.CDLL(str(so)).row_wait
+    assert f(ctypes.c_void_p(status.data_ptr()), ctypes.c_void_p(got.data_ptr()), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    assert got.tolist() == [1, 0]
+    assert status.item() == 4
 
 
 def _places(t, how, n):
