@@ -262,9 +262,7 @@ __global__ void __launch_bounds__(BK_MAXRW * 32, 2) blk_fwd_kernel(const __grid_
                     if (r == BK_R - 1) hb[c] = h;
                 }
                 bk_st16(trow + qt * RL(), make_float4(hb[0].x, hb[0].y, hb[1].x, hb[1].y), mine && blk + 1 < P.nblk);   // the block's last row of h
-            } else if (KEEP && pos.strip * BK_S + 4 * (qt >> 1) < P.W) {   // (the backward recomputes whole halves)
-                bk_st16(trow + qt * RL(), make_float4(0.f, 0.f, 0.f, 0.f), mine && blk + 1 < P.nblk);
-            }
+            }   // (a pair that the image does not have leaves no row of h: the backward copies its place, whatever it holds, and does not use it)
             if (!(qt & 1)) continue;
             const int k = qt >> 1, c0 = pos.strip * BK_S + k * 4;
             if (c0 >= P.W) continue;

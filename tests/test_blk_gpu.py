@@ -71,7 +71,7 @@ def test_block_walk_against_oracle(shape, dtype, kw, det):
 @pytest.mark.parametrize("w", [1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 13, 15, 17])
 @pytest.mark.parametrize("n", [3, 16])
 def test_every_number_of_columns_in_the_last_block(n, w):
-    """The forward leaves out the pairs of columns that a row's last block does not have, the backward its right half."""
+    """Forward and backward leave out the pairs of columns that a row's last block does not have."""
     inp = make_inputs(2, 1, 9, n, 9, w, dtype=torch.float32, seed=w)
     d = _dev(inp)
     args = (d["u"], d["delta"], d["A"], d["B"], d["C"], d["D"], d["delta_bias"])

@@ -18,7 +18,7 @@ def _poison():
     del held
 
 
-@pytest.mark.parametrize("shape", [(2, 4, 9, 16, 13, 56), (1, 2, 11, 3, 18, 21), (2, 1, 8, 7, 9, 4), (1, 2, 13, 2, 22, 100), (2, 2, 65, 1, 14, 7),
+@pytest.mark.parametrize("shape", [(2, 4, 9, 16, 13, 56), (1, 2, 11, 3, 18, 21), (2, 1, 8, 7, 9, 4), (1, 2, 10, 16, 9, 10), (1, 2, 13, 2, 22, 100), (2, 2, 65, 1, 14, 7),
                                    (1, 2, 9, 1, 13, 200), (2, 2, 5, 1, 14, 30), (2, 2, 5, 12, 9, 30), (1, 1, 3, 4, 9, 300)], ids=str)
 @pytest.mark.parametrize("cross", [False, True], ids=["scan", "corners"])
 def test_memory_full_of_nan(shape, cross):
