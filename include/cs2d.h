@@ -47,6 +47,11 @@ typedef enum { CS2D_F32 = 0, CS2D_F16 = 1, CS2D_BF16 = 2 } cs2d_dtype;
  * Strides are in ELEMENTS (64-bit, the reference uses 32-bit); the innermost
  * (ncols) stride of u, delta, B, C, out/dout must be 1 as the reference
  * requires (selective_scan_oflex.cpp:203-204,227,229,318).
+ *
+ * A kernel may read the whole aligned 16 bytes around any element of u, delta and
+ * dout: up to 14 bytes before and after a tensor, row or plane, whose values are
+ * not used.  What lies there may be written by others at the same time.  Nothing
+ * outside a result is written.
  */
 typedef struct {
     int32_t batch, dim, nrows, ncols, dstate, n_groups, delta_dim;

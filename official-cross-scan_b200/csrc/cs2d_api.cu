@@ -481,11 +481,12 @@ static void blk_fill(Blk &k, int &NG, const cs2d_problem *p, const cs2d_dirs *o,
     const int spw = 32 / NG, ctas = blk_ctas(backward, NG);   // slots per warp, CTAs per SM
     k.ntile = (k.nsl + spw - 1) / spw; k.items = p->batch * k.G * k.ntile;
     // Row workers: the number for which the longest chain of blocks that a worker walks takes the least time.  A block's time grows
-    // with the warps that share a scheduler (measured, 56x56 maps, 1 / full: forward 2.6 / 4.8 us at 4, backward 6.4 / 11.2 us at 3), the
+    // with the warps that share a scheduler (measured on 56x56 maps, and used for all sizes; 1 / full: forward 2.6 / 4.8 us at 4, backward 6.4 / 11.2 us at 3), the
     // last round of CTAs is seldom full, a worker is 1.3 (forward) or 1 blocks behind the one before it, which makes it wait where rows
     // are short, and waiting for each other costs a little (us with 1, 2, 4, 8 workers; stage-1 backward, 3.46 rounds: 3880, 3854, 3870,
-    // 4040; forward, 2.59: 1240, 1258, 1208, 1595; 16x4x192x16x28x28 forward: 200, 179, 220, 220; 2x4x192x16x200x336 backward: 14100,
-    // 8750, 6190, 6580; one 56x56 image: 632, 311, 236, 224; 3x4x51x7x45x61: 733, 371, 197, 156).
+    // 4040; forward, 2.59: 1240, 1258, 1208, 1595; 16x4x192x16x28x28 forward, 7 rows, with 1, 2, 4: 200, 179, 220; 2x4x192x16x200x336 backward: 14100,
+    // 8750, 6190, 6580; one 56x56 image: 632, 311, 236, 224; 3x4x51x7x45x61: 733, 371, 197, 156).  It is not always the fastest number: for
+    // the image the rule takes four workers, 5 % behind eight.
     const double slope = backward ? 0.375 : 0.28, lag = backward ? 1 : 1.3;
     double best = 1e300;
     for (int rwl = 0; (1 << rwl) <= std::min(k.nblk, BK_MAXRW); ++rwl) {

@@ -8,10 +8,11 @@
 // row of blocks (down: written as float4, 512 consecutive bytes per warp, read back by the block below).
 //
 // A warp is self-contained: its lanes are the NG states of 32/NG slots (a slot is a channel pair), it loads, transforms
-// (softplus) and stages delta and u of its own slots in shared memory, sums over the states through shared memory and
-// writes the results.  Neighbouring lanes share delta and u (measured on B200: a 128-bit shared load takes 2 cycles of
-// the SM's load unit when neighbouring lanes share their address, 4 otherwise, whatever else is broadcast - and that unit,
-// not arithmetic, bounds these kernels).  No barriers; sixteen warps per SM hide each other's latencies.
+// (softplus) and stages delta and u of its own slots in shared memory, sums over the states (forward: through shared memory,
+// backward: through tensor memory) and writes the results.  Neighbouring lanes share delta and u (measured on B200: a
+// 128-bit shared load takes 2 cycles of the SM's load unit when neighbouring lanes share their address, 4 otherwise, whatever
+// else is broadcast).  That unit bounds the forward, with 16 warps per SM; the backward, with 8 to 12, is bound by the issue
+// and fetch of instructions.  The walks have no CTA barriers.
 //
 // Images with few recurrences run with 2, 4 or 8 row WORKERS (warps of one CTA): the rows of blocks of a team's items are one
 // sequence, and worker w takes every RW-th of them.  A block needs the row of h (backward: of m) that the row before it in the
