@@ -25,8 +25,8 @@
 // that can be is a loop over slots, and addresses that the compiler would make again for every use are held (bk_keep: 3790 -> 3640).
 // With two states per thread in place of one the instructions fall to 99 but the body takes 16 KB (5400 us; a column per iteration: 4080).
 // Before (sums through shared memory, inputs loaded into registers at the end of a block, 4 columns per iteration, a CTA barrier per
-// block): 3770; 128x4x384x16x28x28 bf16 8530 -> 7530, 2x4x192x16x200x336 bf16 6150 -> 5790, 32x4x192x4x56x56 bf16 2760 -> 2190,
-// 3x4x51x7x45x61 fp16 228 -> 156.
+// block) and now: 3770 -> 3660; 128x4x384x16x28x28 bf16 8530 -> 7540, 2x4x192x16x200x336 bf16 6150 -> 5820, 32x4x192x4x56x56 bf16 2760 -> 2200,
+// 3x4x51x7x45x61 fp16 228 -> 156.  What is asked of tensor memory is waited for in the same iteration, not across its end (no difference in time).
 #include "cs2d_blk.cuh"
 
 namespace cs2d {
